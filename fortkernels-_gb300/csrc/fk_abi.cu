@@ -105,11 +105,23 @@ uint64_t fnv(const uint64_t* w, size_t n) {
     return h;
 }
 
+// Whether the workspace holds `need` bytes or can grow to them now.
+bool workspace_can_hold(Ctx& c, size_t need) {
+    if (c.ws.cap >= need) return true;
+    if (capturing(c.stream)) return false;
+    size_t avail = 0, total = 0;
+    if (cudaMemGetInfo(&avail, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return avail + c.ws.cap >= need + need / 4 + (2u << 20);
+}
+
 fk_status ensure_workspace(Ctx& c, size_t need) {
     if (c.ws.cap >= need) return FK_OK;
-    drop_graphs(c);  // captured graphs refer to the old workspace
     if (capturing(c.stream))
         return fail(c, FK_ENOMEM, "workspace must grow, which is not allowed during stream capture: call fk_reserve first");
+    drop_graphs(c);  // captured graphs refer to the old workspace
     cudaError_t e = cudaStreamSynchronize(c.stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "workspace: synchronize");
     if (c.ws.base) cudaFree(c.ws.base);
@@ -665,7 +677,14 @@ fk_status gpp_call(fk_ctx_t c, int nb, int nv, int nc, int ng, const fk_c128* aq
         }
     }
     const size_t outn = 7 + (size_t)nb;
-    const size_t need = fk::staged_bytes(ins) + fk::gpp_workspace(x, r) + outn * sizeof(double2) + 4096;
+    // FP64 contracts on the tensor cores when the workspace can hold its operand
+    // images (28 bytes per aqsntemp element, 42 per D element), else on DMMA
+    size_t need = 0;
+    for (int tc = precision == FK_FP64 ? 1 : 0; tc >= 0; --tc) {
+        r.tc64 = tc != 0;
+        need = fk::staged_bytes(ins) + fk::gpp_workspace(x, r) + outn * sizeof(double2) + 4096;
+        if (!tc || fk::workspace_can_hold(x, need)) break;
+    }
     fk_status s = fk::ensure_workspace(x, need);
     if (s != FK_OK) return s;
 
@@ -679,7 +698,7 @@ fk_status gpp_call(fk_ctx_t c, int nb, int nv, int nc, int ng, const fk_c128* aq
     fk::Ctx::GraphEntry* ge = nullptr;
     if (all_dev) {
         uint64_t w[24] = {(uint64_t)nb, (uint64_t)nv, (uint64_t)nc, (uint64_t)ng, (uint64_t)precision, flags,
-                          (uint64_t)(uintptr_t)x.stream, (uint64_t)(uintptr_t)x.ws.base, (uint64_t)x.est_on};
+                          (uint64_t)(uintptr_t)x.stream, (uint64_t)(uintptr_t)x.ws.base, (uint64_t)x.est_on | (uint64_t)r.tc64 << 1};
         int n = 9;
         for (auto* i : ins) w[n++] = (uint64_t)(uintptr_t)i->user;
         for (auto* o : outs) w[n++] = (uint64_t)(uintptr_t)o;
@@ -831,7 +850,12 @@ fk_status fk_gpp_real(fk_ctx_t c, int nb, int nv, int nc, int ng, const double* 
     r.nb = nb; r.nv = nv; r.nc = nc; r.ng = ng; r.prec = precision; r.flags = flags;
     r.lda = aqn_in_place ? nc : lda;
     const size_t outn = 6 + (size_t)nb;
-    const size_t need = fk::staged_bytes(ins) + aqn_bytes + fk::gpp_real_workspace(x, r) + outn * sizeof(double) + 4096;
+    size_t need = 0;
+    for (int tc = precision == FK_FP64 ? 1 : 0; tc >= 0; --tc) {  // as in fk_gpp
+        r.tc64 = tc != 0;
+        need = fk::staged_bytes(ins) + aqn_bytes + fk::gpp_real_workspace(x, r) + outn * sizeof(double) + 4096;
+        if (!tc || fk::workspace_can_hold(x, need)) break;
+    }
     fk_status s = fk::ensure_workspace(x, need);
     if (s != FK_OK) return s;
     x.ws.reset();
@@ -916,16 +940,21 @@ fk_status fk_ff(fk_ctx_t c, int nb, int nv, int nc, int ng, int nf, int ne, cons
     // host I_epsR / I_epsA of a large request: streamed in plane groups while
     // the groups already copied are being computed (fk::FfPipe)
     const bool pipelined = !er.dev && !ea.dev && planes >= ((size_t)64 << 20) && !fk::capturing(x.stream);
-    const size_t wsb = fk::ff_workspace(x, r, pipelined);
-    if (wsb == (size_t)-1) return fk::fail(x, FK_ECUDA, "ff: reading ekq/dFreqGrid");
     const size_t outn = 1 + 4 * (size_t)ne + (size_t)nb * nf;
     auto r256 = [](size_t b) { return (b + 255) & ~(size_t)255; };
     std::vector<fk::In*> small{&vc, &inv, &ind, &ek, &gr, &br, &pr}, bands{&aqm, &aqn};
     size_t packed = 0;
     for (auto* i : small)
         if (!fk::in_place(i)) packed += r256(i->bytes);
-    const size_t need = (pipelined ? fk::staged_bytes(bands) + 2 * r256(planes) + r256(packed) : fk::staged_bytes(ins)) +
-                        wsb + outn * sizeof(double2) + 4096;
+    size_t need = 0;
+    for (int tc = precision == FK_FP64 ? 1 : 0; tc >= 0; --tc) {  // as in fk_gpp
+        r.tc64 = tc != 0;
+        const size_t wsb = fk::ff_workspace(x, r, pipelined);
+        if (wsb == (size_t)-1) return fk::fail(x, FK_ECUDA, "ff: reading ekq/dFreqGrid");
+        need = (pipelined ? fk::staged_bytes(bands) + 2 * r256(planes) + r256(packed) : fk::staged_bytes(ins)) + wsb +
+               outn * sizeof(double2) + 4096;
+        if (!tc || fk::workspace_can_hold(x, need)) break;
+    }
     fk_status s = fk::ensure_workspace(x, need);
     if (s != FK_OK) return s;
     x.ws.reset();

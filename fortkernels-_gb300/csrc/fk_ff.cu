@@ -19,6 +19,7 @@
 
 #include "fk_gemm.cuh"
 #include "fk_internal.h"
+#include "fk_tc64.cuh"
 #include "fk_tc_contract.cuh"
 #include <cstdlib>
 
@@ -299,7 +300,16 @@ struct FfPlan {
     bool mixed;
     size_t bytes, bytesImgR, bytesImgA, bytesW, bytesAimg;
     size_t bytesScale;  // mixed: 2^-k of every A image row and of every row of the converted planes
+    // FP64 on the tensor cores (fk_tc64.cuh): the planes are converted and contracted zgroup at a time
+    bool tc64 = false;
+    tc64::Plan z{};
+    int zgroup = 0;
 };
+
+// The converted planes of an FP64 request held at once: 2 GB of images (the
+// planes of 512 x 4096 x 512 x 15 in one launch), at most the 64 planes of one
+// launch's table.
+constexpr size_t FF_ZGROUP_BYTES = (size_t)2 << 30;
 
 // k-slices for the persistent tensor-core kernel (see fk_gpp.cu)
 void ff_pick_split_tc(long tiles, int K, int sms, int& KS, int& kchunk) {
@@ -405,8 +415,19 @@ FfPlan make_plan(const Ctx& c, const FfDev& r, const double* ekq_h, const double
         p.KS = std::max(1, std::min((c.sms * 2 + tiles - 1) / tiles, std::max(1, r.nc / 256)));
         p.kchunk = ((r.nc + p.KS - 1) / p.KS + 15) / 16 * 16;
         p.KS = (r.nc + p.kchunk - 1) / p.kchunk;
+        if (r.tc64) {
+            const tc64::Plan one = tc64::make_plan(r.nb, r.ng, r.nc, 1, c.sms / 2);
+            p.zgroup = (int)std::min<size_t>(std::min(nplanes, (int)tc64::MAXPL), std::max<size_t>(1, FF_ZGROUP_BYTES / one.bytesB));
+            p.zgroup = ceil_div(nplanes, ceil_div(nplanes, p.zgroup));  // even groups
+            p.z = tc64::make_plan(r.nb, r.ng, r.nc, p.zgroup, c.sms / 2);
+            p.tc64 = p.z.KS > 0;
+        }
+        if (p.tc64) {
+            p.NT = 2 * p.z.NT;  // its partial slots: the re and im half of each 64-wide n-tile
+            p.KS = p.z.KS;
+        }
     }
-    if (p.mixed) {
+    if (p.mixed || p.tc64) {
         // the correction term of band n1 reads the A planes ifq_c and ifq_c + 1 only
         // (achDtemp_cor_Kernel, FFKer_cori/ffKernel.cpp:212-246): sort the bands by that
         // bracket so that each A plane is contracted over the row tiles of its bands only
@@ -432,7 +453,7 @@ FfPlan make_plan(const Ctx& c, const FfDev& r, const double* ekq_h, const double
             tiles += hi > lo ? (hi - 1) / tcx::BM - lo / tcx::BM + 1 : 0;
         }
         // k-slices for the one launch over all A planes' (row tile, n-tile) pairs
-        ff_pick_split_tc(std::max(1L, tiles) * p.NT, r.nc, c.sms, p.KSa, p.kchunka);
+        if (p.mixed) ff_pick_split_tc(std::max(1L, tiles) * p.NT, r.nc, c.sms, p.KSa, p.kchunka);
     }
     const size_t slots = (size_t)p.KS * p.NT * (p.mixed ? tcx::FF_EPI_WARPS : 1);  // partial slots per plane
     const size_t slotsA = p.mixed ? (size_t)p.KSa * p.NT * tcx::FF_EPI_WARPS : slots;
@@ -442,6 +463,9 @@ FfPlan make_plan(const Ctx& c, const FfDev& r, const double* ekq_h, const double
               r.nb * sizeof(FactRow) + (p.planesR.size() + p.planesA.size()) * sizeof(int) + r.ng * sizeof(int) +
               r.nb * sizeof(int) +
               p.bytesImgR + p.bytesImgA + p.bytesW + p.bytesAimg + p.bytesScale + 20 * 256;
+    if (p.tc64)
+        p.bytes += p.z.bytesA + p.z.bytesEa + p.zgroup * (p.z.bytesB + p.z.bytesEb) +
+                   2 * (size_t)r.nb * r.ng * sizeof(double2) + 6 * 256;
     return p;
 }
 
@@ -474,7 +498,7 @@ fk_status ff_run(Ctx& c, const FfDev& r, const FfPipe* pipe) {
     const size_t slots = (size_t)p.KS * p.NT * (p.mixed ? tcx::FF_EPI_WARPS : 1);  // partial slots per plane
     const size_t slotsA = p.mixed ? (size_t)p.KSa * p.NT * tcx::FF_EPI_WARPS : slots;
     int* igp = (int*)c.ws.take(r.ng * sizeof(int));
-    int* order = p.mixed ? (int*)c.ws.take(r.nb * sizeof(int)) : nullptr;
+    int* order = p.mixed || p.tc64 ? (int*)c.ws.take(r.nb * sizeof(int)) : nullptr;
     int* planes = (int*)c.ws.take((nR + nA) * sizeof(int));
     FactRow* fact = (FactRow*)c.ws.take(r.nb * sizeof(FactRow));
     double2* PR = (double2*)c.ws.take(slots * std::max(nR, 1) * r.nb * 2 * sizeof(double2));
@@ -496,7 +520,18 @@ fk_status ff_run(Ctx& c, const FfDev& r, const FfPipe* pipe) {
     float* ascale = scales;                                              // [nb], image row order
     float* bscaleR = scales ? scales + r.nb : nullptr;                   // [nR][ng]
     float* bscaleA = scales ? bscaleR + (size_t)nR * r.ng : nullptr;     // [nA][ng]
-    if (!igp || (p.mixed && !order) || !planes || !fact || !PR || (nA && !PA) || !tabs || !SD || (p.bytesImgR && !imgR) ||
+    tc64::Bufs zb{};
+    if (p.tc64) {
+        zb.A = (uint8_t*)c.ws.take(p.z.bytesA);
+        zb.B = (uint8_t*)c.ws.take(p.zgroup * p.z.bytesB);
+        zb.ea = (int*)c.ws.take(p.z.bytesEa);
+        zb.eb = (int*)c.ws.take(p.zgroup * p.z.bytesEb);
+        zb.W1 = (double2*)c.ws.take((size_t)r.nb * r.ng * sizeof(double2));
+        zb.W2 = (double2*)c.ws.take((size_t)r.nb * r.ng * sizeof(double2));
+        if (!zb.A || !zb.B || !zb.ea || !zb.eb || !zb.W1 || !zb.W2)
+            return fail(c, FK_ENOMEM, "workspace too small for FF request");
+    }
+    if (!igp || ((p.mixed || p.tc64) && !order) || !planes || !fact || !PR || (nA && !PA) || !tabs || !SD || (p.bytesImgR && !imgR) ||
         (p.bytesImgA && !imgA) || (p.bytesW && !W) || (p.bytesAimg && !Aimg) || (p.bytesScale && !scales))
         return fail(c, FK_ENOMEM, "workspace too small for FF request");
     double2 *RW = tabs, *RS = tabs + (size_t)r.nb * r.nf, *AW = tabs + 2 * (size_t)r.nb * r.nf;
@@ -557,6 +592,14 @@ fk_status ff_run(Ctx& c, const FfDev& r, const FfPipe* pipe) {
         tcx::aimg_convert_kernel<<<r.nb, 256, 0, st>>>(r.aqsn, r.nb, r.nc, p.kstages, Aimg, order, ascale);
         c.launches += 2;
         cudaMemsetAsync(c.errword, 0, sizeof(int), st);
+    }
+    if (p.tc64) {
+        cudaMemsetAsync(c.errword, 0, sizeof(int), st);
+        ContractArgs a{};
+        a.A = r.aqsn; a.lda = r.nc; a.M = r.nb; a.K = r.nc; a.rowmap = order;
+        a.aqsm = r.aqsm; a.ldm = r.nc; a.vcoul = r.vcoul; a.igp = igp; a.acol = igp; a.wscale = 1.0;
+        tc64::enqueue_weights(c, a, r.ng, zb, true);
+        tc64::enqueue_a(c, a, p.z, zb);
     }
     // a0 < 0: R planes, all bands on CTA pairs; a0 >= 0: the A planes a0 .. a0+nb_-1
     // of planesA, each over the row tiles of the bands that read it
@@ -649,6 +692,31 @@ fk_status ff_run(Ctx& c, const FfDev& r, const FfPipe* pipe) {
             k<<<grid1, tcx::THREADS_FF, smem, st>>>(t);
             kernel_end(c);
             c.launches += 2;
+        } else if (p.tc64) {
+            a.rowmap = order;
+            const size_t pslab = slots * r.nb * 2;
+            for (int g0 = 0; g0 < nb_; g0 += p.zgroup) {
+                ContractArgs ag = a;
+                ag.batches = std::min(p.zgroup, nb_ - g0);
+                ag.batch_plane = pls + g0;
+                ag.P = P + g0 * pslab;
+                // R planes: all bands; A planes: the 256-row tiles of the bands that read each one
+                tc64::PlaneTab tab{};
+                tab.n = ag.batches;
+                for (int j = 0; j < tab.n; ++j) {
+                    const int lo = a0 < 0 ? 0 : p.aLo[a0 + g0 + j], hi = a0 < 0 ? r.nb : p.aHi[a0 + g0 + j];
+                    tab.mt0[j] = hi > lo ? lo / tc64::BM : 0;
+                    tab.MT[j] = hi > lo ? (hi - 1) / tc64::BM - tab.mt0[j] + 1 : 0;
+                    tab.u0[j + 1] = tab.u0[j] + tab.MT[j] * p.z.NT * p.z.KS;
+                }
+                if (tab.u0[tab.n] == 0) continue;
+                // the timed kernel is the R planes' contraction
+                const bool prof = c.profiling;
+                if (a0 >= 0) c.profiling = false;
+                tc64::enqueue<EPI_FF>(c, ag, p.z, zb, tab, a0 < 0);
+                if (a0 >= 0) --c.nk;
+                c.profiling = prof;
+            }
         } else {
             dim3 grid(p.MT, p.NT * p.KS * nb_);
             auto k = d64::contract_kernel<EPI_FF>;

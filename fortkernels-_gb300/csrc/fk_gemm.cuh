@@ -48,7 +48,13 @@ struct ContractArgs {
     double wscale;
     int G;                  // groups per row in P
     double2* P;             // [slots][M][G]
+    // FP64 engine behind the tensor-core one (fk_tc64.cuh)
+    int nt_tiles = 0;               // n-tiles of the slot layout (0: ceil(N / BN))
+    const int* only_if = nullptr;   // the launch does nothing while this is 0
+    const int* rowmap = nullptr;    // row m of A and aqsm (nullptr: m0 + m)
 };
+
+FK_DEV long contract_row(const ContractArgs& a, int m) { return a.rowmap ? a.rowmap[m] : a.m0 + m; }
 
 __host__ __device__ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
@@ -56,7 +62,7 @@ __host__ __device__ inline int ceil_div(int a, int b) { return (a + b - 1) / b; 
 FK_DEV double2 epi_weight(const ContractArgs& a, int m, int h) {
     int g = a.igp[h];
     if (g < 0) return make_double2(0.0, 0.0);
-    double2 am = a.aqsm[(long)(a.m0 + m) * a.ldm + a.acol[h]];
+    double2 am = a.aqsm[contract_row(a, m) * a.ldm + a.acol[h]];
     double s = a.wscale * a.vcoul[g];
     return make_double2(am.x * s, -am.y * s);
 }
@@ -71,7 +77,7 @@ FK_DEV void epi_accum(const ContractArgs& a, int m, int n, double2 c, double2* g
     } else if (EPI == EPI_FF) {
         int ig = a.igp[n];
         if (ig < 0) return;
-        double2 am = a.aqsm[(long)(a.m0 + m) * a.ldm + a.acol[n]];
+        double2 am = a.aqsm[contract_row(a, m) * a.ldm + a.acol[n]];
         double2 t = cmul(cconj(am), c);
         gs[0] = cadd(gs[0], cscale(t, a.vcoul[ig]));
         gs[1] = cadd(gs[1], t);
@@ -123,7 +129,8 @@ __global__ void __launch_bounds__(THREADS) contract_kernel(ContractArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2* As = reinterpret_cast<double2*>(smem_raw);
     double2* Bs = As + STAGES * BM * LDS;
-    const int NT = ceil_div(a.N, BN);
+    if (a.only_if && !*a.only_if) return;
+    const int NT = a.nt_tiles ? a.nt_tiles : ceil_div(a.N, BN);
     const int mt = blockIdx.x, nt = blockIdx.y % NT;
     const int ks = (blockIdx.y / NT) % a.KS, batch = blockIdx.y / (NT * a.KS);
     const int plane = a.batch_plane ? a.batch_plane[batch] : batch;
@@ -142,7 +149,7 @@ __global__ void __launch_bounds__(THREADS) contract_kernel(ContractArgs a) {
             int r = i / BK, c = i % BK;
             int m = mt * BM + r, k = kb + c;
             bool ok = m < a.M && k < k1;
-            const double2* src = ok ? a.A + (long)(a.m0 + m) * a.lda + k : a.A;
+            const double2* src = ok ? a.A + contract_row(a, m) * a.lda + k : a.A;
             cp_async16(&as[r * LDS + c], src, ok);
         }
         for (int i = tid; i < BN * BK; i += THREADS) {

@@ -30,6 +30,7 @@
 
 #include "fk_gemm.cuh"
 #include "fk_internal.h"
+#include "fk_tc64.cuh"
 #include "fk_tc_contract.cuh"
 
 namespace fk {
@@ -1235,6 +1236,11 @@ struct Plan {
     // image) instead of by the converter warps of every n-tile's units
     bool apre;
     size_t bytesD, bytesF, bytesP, bytesS, bytesRows, bytesIgp, bytesW, bytesAimg;
+    // FP64 on the tensor cores (fk_tc64.cuh): the main and the static remainder contraction, and their workspace
+    bool tc64;
+    tc64::Plan z, zs;
+    size_t zA, zB, zEa, zEb, zW;
+    size_t bytesZ() const { return tc64 ? zA + zB + zEa + zEb + zW + 5 * 256 : 0; }
 };
 
 // fk_gpp's mixed path (not the half sum, not the root file's flag-band I_eps
@@ -1333,12 +1339,35 @@ Plan make_plan(const Ctx& c, const GppDev& r, int ks_override = 0, bool pipeline
         p.MT = ceil_div(std::max(M, 1), d64::BM);
         p.NT = ceil_div(N, d64::BN);
         pick_split(p.MT * p.NT, r.nc, c.sms * 2, p.KS, p.kchunk);
+        if (r.tc64 && M > 0) {
+            p.z = tc64::make_plan(M, N, r.nc, 1, c.sms / 2);
+            if (r.flags & FK_GPP_ACHSTEMP) p.zs = tc64::make_plan(r.nb, r.ng, r.nc, 1, c.sms / 2);
+            p.tc64 = p.z.KS && (p.zs.KS || !(r.flags & FK_GPP_ACHSTEMP));
+        }
+        if (p.tc64) {
+            p.NT = 2 * p.z.NT;  // its partial slots: the re and im half of each 64-wide n-tile
+            p.KS = p.z.KS;
+            p.zA = p.z.bytesA;
+            p.zB = p.z.bytesB;
+            p.zEa = p.z.bytesEa;
+            p.zEb = p.z.bytesEb;
+            p.zW = (size_t)r.ng * M * sizeof(double2);
+        }
     }
     const int per_sm = p.mixed ? 4 : 2;
     const int BM = p.mixed ? f32::BM : d64::BM, BN = p.mixed ? f32::BN : d64::BN;
     p.MTs = ceil_div(r.nb, BM);
     p.NTs = ceil_div(r.ng, BN);
     pick_split(p.MTs * p.NTs, r.nc, c.sms * per_sm, p.KSs, p.kchunks);
+    if (p.tc64 && (r.flags & FK_GPP_ACHSTEMP)) {
+        p.NTs = 2 * p.zs.NT;
+        p.KSs = p.zs.KS;
+        p.zA = std::max(p.zA, p.zs.bytesA);
+        p.zB = std::max(p.zB, p.zs.bytesB);
+        p.zEa = std::max(p.zEa, p.zs.bytesEa);
+        p.zEb = std::max(p.zEb, p.zs.bytesEb);
+        p.zW = (size_t)r.ng * r.nb * sizeof(double2);
+    }
     p.bytesD = M <= 0 ? 0
                : p.mixed ? (size_t)p.NT * p.kstages * tcx::Cfg<64>::B_BYTES
                          : (size_t)N * r.nc * sizeof(double2);
@@ -1349,6 +1378,24 @@ Plan make_plan(const Ctx& c, const GppDev& r, int ks_override = 0, bool pipeline
     p.bytesRows = rows_bytes(r.nb);
     p.bytesIgp = 2 * (size_t)r.ng * sizeof(int);  // igp, acol
     return p;
+}
+
+// FP64 on the tensor cores: takes its workspace / runs one contraction.
+bool take_tc64(Ctx& c, const Plan& p, tc64::Bufs& b) {
+    if (!p.tc64) return true;
+    b.A = (uint8_t*)c.ws.take(p.zA);
+    b.B = (uint8_t*)c.ws.take(p.zB);
+    b.ea = (int*)c.ws.take(p.zEa);
+    b.eb = (int*)c.ws.take(p.zEb);
+    b.W1 = (double2*)c.ws.take(p.zW);
+    b.W2 = nullptr;
+    return b.A && b.B && b.ea && b.eb && b.W1;
+}
+template <int EPI>
+void run_tc64(Ctx& c, const ContractArgs& a, const tc64::Plan& z, const tc64::Bufs& b) {
+    tc64::enqueue_weights(c, a, EPI == EPI_GPP ? a.N / 3 : a.N, b, false);
+    tc64::enqueue_a(c, a, z, b);
+    tc64::enqueue<EPI>(c, a, z, b, tc64::one_plane(z), false);
 }
 
 template <class K>
@@ -1667,7 +1714,7 @@ size_t gpp_workspace(const Ctx& c, const GppDev& r, bool pipelined) {
                            ? (size_t)p.nch * r.ng * 18 * sizeof(float) + (size_t)r.nb * (sizeof(float2) + 6 * sizeof(double)) + 768
                            : 0;
     return p.bytesD + p.bytesF + p.bytesP + p.bytesS + p.bytesRows + p.bytesIgp + p.bytesW + p.bytesAimg + half + wf + est +
-           16 * 256;
+           p.bytesZ() + 16 * 256;
 }
 
 int gpp_pipe_chunks(const Ctx& c, const GppDev& r) { return make_plan(c, r, 0, true, false, gpp_fsch(r)).pipe_chunks; }
@@ -1717,12 +1764,14 @@ fk_status gpp_run_half(Ctx& c, const GppDev& r) {
     int* brk = (int*)c.ws.take((size_t)r.ng * sizeof(int));
     double2* schd = (double2*)c.ws.take((size_t)r.ng * 3 * sizeof(double2));
     int* counter = (int*)c.ws.take(sizeof(int));
+    tc64::Bufs zb{};
+    if (!take_tc64(c, p, zb)) return fail(c, FK_ENOMEM, "workspace too small for GPP request");
     if (!igp || !F || !rows || !brk || !schd || !counter || (p.bytesD && !D) || (p.bytesP && (!P || !P2)) || (p.bytesW && !W))
         return fail(c, FK_ENOMEM, "workspace too small for GPP request");
     if (r.aqsm_compact || r.ldm != r.nc) return fail(c, FK_EINVAL, "gpp: the half sum needs all of aqsmtemp");
     c.launches = 0;
-    if (p.mixed && D) {
-        if (tcx::img_needs_pad(64, r.ng, GPP_COLS, r.nc))
+    if ((p.mixed || p.tc64) && D) {
+        if (p.mixed && tcx::img_needs_pad(64, r.ng, GPP_COLS, r.nc))
             tcx::img_pad_kernel<64><<<dim3(p.kstages, p.NT, 1), 256, 0, st>>>((uint8_t*)D, p.NT, p.kstages, r.ng,
                                                                             GPP_COLS, r.nc);
         if (cudaMemsetAsync(c.errword, 0, sizeof(int), st) != cudaSuccess)
@@ -1771,6 +1820,9 @@ fk_status gpp_run_half(Ctx& c, const GppDev& r) {
             kernel_begin(c);
             k<<<std::min(p.units, c.sms), tcx::THREADS, tcx::Cfg<64>::SMEM, st>>>(t);
             kernel_end(c);
+        } else if (p.tc64) {
+            run_tc64<EPI_GPP>(c, a, p.z, zb);
+            continue;
         } else {
             auto k = d64::contract_kernel<EPI_GPP>;
             set_smem(k, d64::SMEM);
@@ -1819,7 +1871,9 @@ fk_status gpp_run(Ctx& c, const GppDev& r, const GppPipe* pipe) {
     if (!igp || !F || !rows || !counter || (p.bytesD && !D) || (p.bytesP && !P) || (p.bytesS && !S) ||
         (p.bytesW && !W) || (r.nv > 0 && !wf) || (est && (!estE || !estA || !estB)) || (p.bytesAimg && !Aimg))
         return fail(c, FK_ENOMEM, "workspace too small for GPP request");
-    if (p.mixed && D) {
+    tc64::Bufs zb{};
+    if (!take_tc64(c, p, zb)) return fail(c, FK_ENOMEM, "workspace too small for GPP request");
+    if ((p.mixed || p.tc64) && D) {
         cudaError_t e = cudaMemsetAsync(c.errword, 0, sizeof(int), st);  // bounded-wait status
         if (e != cudaSuccess) return cuda_fail(c, e, "gpp: error word");
     }
@@ -1966,6 +2020,9 @@ fk_status gpp_run(Ctx& c, const GppDev& r, const GppPipe* pipe) {
                 k<<<std::min(p.units, c.sms), tcx::THREADS, tcx::Cfg<64>::SMEM, st>>>(t);
                 kernel_end(c);
             }
+        } else if (p.tc64) {
+            run_tc64<EPI_GPP>(c, a, p.z, zb);
+            --c.launches;
         } else {
             auto k = d64::contract_kernel<EPI_GPP>;
             set_smem(k, d64::SMEM);
@@ -1986,6 +2043,15 @@ fk_status gpp_run(Ctx& c, const GppDev& r, const GppPipe* pipe) {
             auto k = f32::contract_kernel<EPI_STAT, double2>;
             set_smem(k, f32::SMEM);
             k<<<grid, f32::THREADS, f32::SMEM, st>>>(a);
+        } else if (p.tc64) {
+            // not the dominant kernel of the call: outside the kernel timer
+            const bool prof = c.profiling;
+            const int nk = c.nk;
+            c.profiling = false;
+            run_tc64<EPI_STAT>(c, a, p.zs, zb);
+            c.profiling = prof;
+            c.nk = nk;
+            --c.launches;
         } else {
             auto k = d64::contract_kernel<EPI_STAT>;
             set_smem(k, d64::SMEM);
@@ -2420,7 +2486,7 @@ RealPlan make_real_plan(const Ctx& c, const GppRealDev& r) {
     RealPlan q{};
     q.K2 = (r.nc + 1) / 2;
     q.cd = GppDev{};
-    q.cd.nb = r.nb; q.cd.nv = r.nv; q.cd.nc = (int)q.K2; q.cd.ng = r.ng; q.cd.prec = r.prec; q.cd.flags = 0;
+    q.cd.nb = r.nb; q.cd.nv = r.nv; q.cd.nc = (int)q.K2; q.cd.ng = r.ng; q.cd.prec = r.prec; q.cd.flags = 0; q.cd.tc64 = r.tc64;
     q.c = make_plan(c, q.cd);
     // FP64: tiles of the FP64 prep; mixed: chunks of one resident wave
     q.tile = r.prec == FK_MIXED ? ceil_div(ceil_div(r.nc, std::max(1, 4 * c.sms / r.ng)), PREP_THREADS) * PREP_THREADS
@@ -2438,7 +2504,7 @@ RealPlan make_real_plan(const Ctx& c, const GppRealDev& r) {
 size_t gpp_real_workspace(const Ctx& c, const GppRealDev& r) {
     const RealPlan q = make_real_plan(c, r);
     return q.c.bytesD + q.c.bytesW + q.c.bytesP + q.c.bytesRows + q.c.bytesIgp + q.bytesDv + q.bytesMask + q.bytesF +
-           q.bytesAC + q.bytesOutc + 13 * 256;
+           q.bytesAC + q.bytesOutc + q.c.bytesZ() + 13 * 256;
 }
 
 fk_status gpp_real_run(Ctx& c, const GppRealDev& r) {
@@ -2462,9 +2528,11 @@ fk_status gpp_real_run(Ctx& c, const GppRealDev& r) {
     if (!igp || !rows || !Dv || !mask || !F || !AC || !outc || !counter || (p.bytesD && !D) || (p.bytesP && !P) ||
         (p.bytesW && !W))
         return fail(c, FK_ENOMEM, "workspace too small for the real-valued GPP request");
+    tc64::Bufs zb{};
+    if (!take_tc64(c, p, zb)) return fail(c, FK_ENOMEM, "workspace too small for the real-valued GPP request");
     c.launches = 0;
-    if (p.mixed && D) {
-        if (tcx::img_needs_pad(64, r.ng, GPP_COLS, (int)q.K2))
+    if ((p.mixed || p.tc64) && D) {
+        if (p.mixed && tcx::img_needs_pad(64, r.ng, GPP_COLS, (int)q.K2))
             tcx::img_pad_kernel<64><<<dim3(p.kstages, p.NT, 1), 256, 0, st>>>((uint8_t*)D, p.NT, p.kstages, r.ng,
                                                                             GPP_COLS, (int)q.K2);
         if (cudaMemsetAsync(c.errword, 0, sizeof(int), st) != cudaSuccess)
@@ -2519,6 +2587,9 @@ fk_status gpp_real_run(Ctx& c, const GppRealDev& r) {
             kernel_begin(c);
             k<<<std::min(p.units, c.sms), tcx::THREADS, tcx::Cfg<64>::SMEM, st>>>(t);
             kernel_end(c);
+        } else if (p.tc64) {
+            run_tc64<EPI_GPP>(c, a, p.z, zb);
+            --c.launches;
         } else {
             auto k = d64::contract_kernel<EPI_GPP>;
             set_smem(k, d64::SMEM);

@@ -82,6 +82,7 @@ struct GppDev {
     fk_precision prec;
     unsigned flags;
     double2* out;      // device [3 achtemp | 3 asxtemp | 1 achstemp | nb acht_n1_loc]
+    bool tc64 = false; // FP64: the contraction on the tensor cores (fk_tc64.cuh; needs workspace for its images)
 };
 // Host arrays of a mixed-precision request streamed to the device in row
 // blocks while the blocks already copied are being computed (the host link is
@@ -115,6 +116,7 @@ struct GppRealDev {
     fk_precision prec;
     unsigned flags;
     double* out;       // device [3 achtemp | 3 asxtemp | nb acht_n1_loc]
+    bool tc64 = false; // FP64: the contraction on the tensor cores
 };
 size_t gpp_real_workspace(const Ctx& c, const GppRealDev& r);
 fk_status gpp_real_run(Ctx& c, const GppRealDev& r);
@@ -161,6 +163,7 @@ struct FfDev {
     unsigned flags;
     // outputs (device): [achsDtemp | asx[ne] | achD[ne] | cor[ne] | a2[ne] | schDt[nb*nf]]
     double2* out;
+    bool tc64 = false; // FP64: the contraction on the tensor cores
 };
 // Host I_epsR / I_epsA arrays of an FF request streamed to the device in plane
 // groups on c.copy_stream, each group followed by its event (pipe_ev[0..7]);

@@ -60,6 +60,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long l
 // behind at a collective.
 __device__ __forceinline__ bool warp_all(bool v) { return __all_sync(0xffffffffu, v); }
 
+// One lane of a converged warp.  The warp that issues MMAs runs its loops with
+// all lanes (every value warp-uniform, so that descriptors are formed in uniform
+// registers) and issues under this predicate: 64 cycles per M=256 N=128 MMA
+// whatever the other warps do.  The same loops inside a `lane == 0` branch were
+// measured at 70 cycles alone and 92-102 beside busy epilogue warps.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+    return p != 0;
+}
+
 // Make generic-proxy writes to shared memory visible to the async proxy
 // (tensor-core operand reads, bulk copies).
 __device__ __forceinline__ void fence_proxy_async_smem() {
