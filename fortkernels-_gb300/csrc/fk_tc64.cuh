@@ -36,12 +36,10 @@
 // and half of B 8 KB per CTA) into nine slots and a stage's digit pairs run in
 // an order that spreads the classes' drains and the slots' reuse over the stage
 // (PAIRS, below).
-// Measured (GB300): the contraction of GPP 512 x 2 x 32768 x 20 takes 0.18 ms
-// (DMMA 7.85 ms), FF's planes at 512 x 4096 x 512 x 15 take 3.6 ms (DMMA 222 ms;
+// Measured (GB300): the contraction of GPP 512 x 2 x 32768 x 20 takes 0.17 ms
+// (DMMA 7.85 ms), FF's planes at 512 x 4096 x 512 x 15 take 3.28 ms (DMMA 222 ms;
 // the A planes over the bands that read them only); errors against 64-bit
 // references are those of the DMMA path or lower (FF 1.9e-15 against 4.8e-15).
-// What bounds it now: 9.9 thousand cycles per stage in FF, 10.9 in GPP (operand
-// supply), and ~50 (GPP) to 100 (FF) thousand per unit for the weighted sums.
 #pragma once
 #include <algorithm>
 
@@ -382,7 +380,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) contract
                             ok = false;
                             break;
                         }
-                        tc::mbar_arrive_remote(&full[s], 0);
+                        tc::mbar_arrive_peer(&full[s], 0);
                     }
             }
         } else if (rank == 0) {

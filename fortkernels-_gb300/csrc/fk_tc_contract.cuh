@@ -16,7 +16,7 @@
 // FP64 epilogue every CHUNK_STAGES*32 k-values.
 //
 // CTA organisation (one persistent CTA per SM):
-//   warp 0      TMEM allocation, MMA issue (one lane)
+//   warp 0      TMEM allocation, MMA issue (the warp walks the loops, one elected lane issues)
 //   warp 1      copies: pre-split B tiles (and FF's pre-split A tiles) by bulk
 //               copy, GPP's FP64 A rows by tensor-map TMA (one lane issues)
 //   GPP, 448 threads: warps 4..7 epilogue (TMEM lanes 0..127 = tile rows,
@@ -25,7 +25,12 @@
 //   FF, 576 threads: warps 2..17 epilogue, one per (lane quarter, 16-column
 //               group), weights in registers; three operand stages
 // Work units are (m-tile, n-tile, k-slice, batch); CTA i takes units
-// i, i + gridDim.x, ...  Every wait is bounded; on timeout the CTA records
+// i, i + gridDim.x, ...  What set the pace before: MMAs issued from a lane == 0
+// branch (92-102 cycles each beside busy warps instead of 64; now a converged
+// warp with one elected lane) and, on CTA pairs, the odd CTA's relay, whose
+// cluster-scope release took 1000-2000 cycles per stage.  The GPP contraction over
+// 26 n-tiles went from 3.09 to 2.10 ms (1610 cycles per stage of 24 MMAs = 1536),
+// FF's R planes from 0.448 to 0.326 ms.  Every wait is bounded; on timeout the CTA records
 // an error code and unwinds without further waits of unbounded length.
 #pragma once
 #include <cuda.h>
@@ -377,11 +382,13 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
                         ok = false;
                         break;
                     }
-                    tc::mbar_arrive_remote(&peerFull[s], 0);
+                    tc::mbar_arrive_peer(&peerFull[s], 0);
                 }
             }
-        } else if (lane == 0 && (!PAIR || rank == 0)) {
+        } else if (!PAIR || rank == 0) {
             // ------------------------------------------------------------ MMA
+            // all lanes walk the loops (values stay warp-uniform), one issues
+            const bool issue = tc::elect_one();
             int g = 0, grp = 0;
             bool ok = true;
             const uint32_t idp = C::F16 ? tc::idesc_f16(PAIR ? 2 * BM : BM, 2 * BN)
@@ -402,7 +409,7 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
                     const uint32_t bpar = ((grp / C::NSLOT) & 1) ^ 1;
                     const bool freed = PAIR ? tc::mbar_wait_cluster(&accEmpty[slot], bpar, wait_limit)
                                             : tc::mbar_wait(&accEmpty[slot], bpar, wait_limit);
-                    if (!freed) { fail(1); ok = false; break; }
+                    if (!tc::warp_all(freed)) { fail(1); ok = false; break; }
                     tc::tc_fence_after();
                     const int sg1 = min(nst, sg0 + C::GRP * CH);
                     for (int st0 = sg0, b = slot * C::GRP; st0 < sg1 && ok; st0 += CH, ++b) {
@@ -414,9 +421,9 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
                             const uint32_t par = (g / C::STAGES) & 1;
                             // pre-split A: the A image lands on fullB too (one barrier per stage);
                             // FF: negFull follows fullB once the -B_im warp has written -B_im
-                            if ((!ua && !tc::mbar_wait(&fullA[s], par, wait_limit)) ||
-                                !tc::mbar_wait(C::IMGN ? &negFull[s] : &fullB[s], par, wait_limit) ||
-                                (PAIR && !tc::mbar_wait_cluster(&peerFull[s], par, wait_limit))) {
+                            if (!tc::warp_all((ua || tc::mbar_wait(&fullA[s], par, wait_limit)) &&
+                                              tc::mbar_wait(C::IMGN ? &negFull[s] : &fullB[s], par, wait_limit) &&
+                                              (!PAIR || tc::mbar_wait_cluster(&peerFull[s], par, wait_limit)))) {
                                 fail(2);
                                 ok = false;
                                 break;
@@ -459,28 +466,34 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
                             // below of the sum; FP16: lh, hl, 2^-11) of both k-steps go in first,
                             // while the accumulator is small, and the two hh products last: two
                             // full-scale roundings per stage.
-                            constexpr int NQ = C::F16 ? 2 : 5;
-                            constexpr int PA[5] = {1, C::F16 ? 0 : 2, 0, 1, 0};
-                            constexpr int PB[5] = {C::F16 ? 0 : 1, C::F16 ? 1 : 0, 2, 0, 1};
+                            if (issue) {
+                                constexpr int NQ = C::F16 ? 2 : 5;
+                                constexpr int PA[5] = {1, C::F16 ? 0 : 2, 0, 1, 0};
+                                constexpr int PB[5] = {C::F16 ? 0 : 1, C::F16 ? 1 : 0, 2, 0, 1};
 #pragma unroll
-                            for (int kk = 0; kk < 2; ++kk)
+                                for (int kk = 0; kk < 2; ++kk)
 #pragma unroll
-                                for (int q = 0; q < NQ; ++q) mma2(PA[q], PB[q], kk, (st > st0 || kk > 0 || q > 0) ? 1u : 0u);
-                            mma2(0, 0, 0, 1u);
-                            mma2(0, 0, 1, 1u);
-                            if constexpr (PAIR) tc::mma_commit_pair(&empty[s], 3);  // frees the stage in both CTAs
-                            else tc::mma_commit(&empty[s]);
+                                    for (int q = 0; q < NQ; ++q) mma2(PA[q], PB[q], kk, (st > st0 || kk > 0 || q > 0) ? 1u : 0u);
+                                mma2(0, 0, 0, 1u);
+                                mma2(0, 0, 1, 1u);
+                                if constexpr (PAIR) tc::mma_commit_pair(&empty[s], 3);  // frees the stage in both CTAs
+                                else tc::mma_commit(&empty[s]);
+                            }
                         }
                     }
                     if (!ok) break;
                     // one commit tracks every earlier MMA of this thread: the whole group
-                    if constexpr (PAIR) tc::mma_commit_pair(&accFull[slot], 3);  // both CTAs' epilogues
-                    else tc::mma_commit(&accFull[slot]);
+                    if (issue) {
+                        if constexpr (PAIR) tc::mma_commit_pair(&accFull[slot], 3);  // both CTAs' epilogues
+                        else tc::mma_commit(&accFull[slot]);
+                    }
                 }
             }
             // drain: every issued MMA has completed before TMEM is released
-            if constexpr (PAIR) tc::mma_commit_pair(done, 1);
-            else tc::mma_commit(done);
+            if (issue) {
+                if constexpr (PAIR) tc::mma_commit_pair(done, 1);
+                else tc::mma_commit(done);
+            }
             if (!tc::mbar_wait(done, 0, DRAIN_LIMIT)) fail(4);
         }
     } else if (warp == 1) {
@@ -625,14 +638,15 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
                     for (int pc = 0; pc < C::NPIECE; ++pc) {
                         const uint4* from = (const uint4*)(bsm + (PAIR ? 2 * pc + 1 : 3 * pc + 2) * BN * 64);
                         uint4* to = (uint4*)(bsm + (PAIR ? 2 * pc + 1 : 3 * pc) * BN * 64);
-                        for (int i = lane; i < BN * 64 / 16; i += 32) {
-                            uint4 v = from[i];
-                            v.x ^= 0x80008000u;
-                            v.y ^= 0x80008000u;
-                            v.z ^= 0x80008000u;
-                            v.w ^= 0x80008000u;
-                            to[i] = v;
-                        }
+                        // all eight chunks of a lane are read before the first is written: one round
+                        // trip to shared memory per piece instead of eight
+                        uint4 v[BN * 64 / 16 / 32];
+#pragma unroll
+                        for (int i = 0; i < BN * 64 / 16 / 32; ++i) v[i] = from[i * 32 + lane];
+#pragma unroll
+                        for (int i = 0; i < BN * 64 / 16 / 32; ++i)
+                            to[i * 32 + lane] = make_uint4(v[i].x ^ 0x80008000u, v[i].y ^ 0x80008000u,
+                                                           v[i].z ^ 0x80008000u, v[i].w ^ 0x80008000u);
                     }
                     tc::fence_proxy_async_smem();
                     __syncwarp();
