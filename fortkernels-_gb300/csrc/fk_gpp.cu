@@ -2229,6 +2229,13 @@ struct GppStep {
     bool launched = false;
 };
 
+// k-stages of a served request's unit at most.  A step hands out whole units
+// within its budget (96 stages per SM by default), so the units of a large
+// request, 340 stages long under the plan of a call of its own, left most SMs
+// without one: 32 requests of 128-1024 bands took 40.2 ms, with units of at most
+// 64, 32 and 16 stages 22.2, 19.8 and 20.1 ms.
+constexpr int SERVED_UNIT = 32;
+
 // A served request over four or more n-tiles gets an A image: without it the
 // converter warps of every n-tile's units would split the same A rows again.
 inline size_t job_aimg_bytes(const Plan& p) {
@@ -2470,6 +2477,11 @@ fk_status gpp_time_plan(Ctx& c, GppStep* s, const GppDev& r, int ks, long step_b
 }
 
 int gpp_default_ks(const Ctx& c, const GppDev& r) { return make_plan(c, r).KS; }
+
+int gpp_served_ks(const Ctx& c, const GppDev& r) {
+    const Plan p = make_plan(c, r);
+    return std::max(p.KS, ceil_div(p.kstages, SERVED_UNIT));
+}
 
 
 // ------------------------------------------------------------ real-valued run

@@ -150,6 +150,8 @@ fk_status gpp_step_launch(Ctx& c, GppStep* s, const GppStepItem* items, int n);
 // request run alone through served steps of step_budget k-stages with ks
 // k-slices per tile (r: device inputs; [ws, ws+bytes) its workspace).
 int gpp_default_ks(const Ctx& c, const GppDev& r);
+// The k-slice count of a served request that was not autotuned.
+int gpp_served_ks(const Ctx& c, const GppDev& r);
 fk_status gpp_time_plan(Ctx& c, GppStep* s, const GppDev& r, int ks, long step_budget, void* ws, size_t bytes,
                         float* ms, int* units);
 

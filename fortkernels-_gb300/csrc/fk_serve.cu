@@ -142,10 +142,9 @@ struct fk_server {
     size_t pinned_n = 0;
     // autotuned k-slice counts by request shape (nb, nvband, ncouls, ngpown, flags)
     std::map<std::vector<long>, int> tuned;
-    int ks_for(const fk_gpp_request& q) const {
-        auto it = tuned.find({q.number_bands, q.nvband, q.ncouls, q.ngpown, (long)q.flags});
-        return it == tuned.end() ? 0 : it->second;
-    }
+    // k-slices of a request: its shape's tuned count, else the served default
+    // where its partial sums fit the budget too (0: the plan of a call of its own)
+    int ks_for(const fk_gpp_request& q) const;
 
     void run();
     bool admit(fk::Request* r);
@@ -186,6 +185,15 @@ GppDev request_dev(const fk_gpp_request& q) {
 
 }  // namespace
 }  // namespace fk
+
+int fk_server::ks_for(const fk_gpp_request& q) const {
+    auto it = tuned.find({q.number_bands, q.nvband, q.ncouls, q.ngpown, (long)q.flags});
+    if (it != tuned.end()) return it->second;
+    const fk::GppDev d = fk::request_dev(q);
+    const int ks = fk::gpp_served_ks(*ctx, d);
+    const size_t need = fk::staged_bytes(*this, q) + fk::gpp_job_bytes(*ctx, d, ks) + 4096;
+    return fk::round256(need) <= arena.capacity() ? ks : 0;
+}
 
 bool fk_server::admit(fk::Request* r) {
     using namespace fk;
