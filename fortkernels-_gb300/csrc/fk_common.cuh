@@ -60,6 +60,12 @@ FK_DEV double f32_to_f64_bits(float f) {
         (long long)(s | ((unsigned long long)(e + 896u) << 52) | ((unsigned long long)(u & 0x7FFFFFu) << 29)));
 }
 
+// The same for any value (subnormals, infinities and NaN by the conversion instruction).
+FK_DEV double f32_to_f64(float f) {
+    const unsigned e = (__float_as_uint(f) >> 23) & 0xFFu;
+    return e - 1u < 254u ? f32_to_f64_bits(f) : (double)f;
+}
+
 // x[0] + x[stride] + ... + x[(n-1)*stride], added left to right.  The loads
 // of a group are issued together ahead of the adds, so a long sum waits for
 // memory once per group.  Every load reads a valid address (the index is

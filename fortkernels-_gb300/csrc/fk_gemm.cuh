@@ -235,19 +235,20 @@ __global__ void __launch_bounds__(THREADS) contract_kernel(ContractArgs a) {
 // CTA tile 64 x 64 complex, 256 threads, 4 x 4 complex per thread, k-step
 // 16.  FP64 inputs are rounded to FP32 with the integer conversion; products
 // accumulate in FP32 for one 16-value k-step, then into a float-float (hi, lo)
-// accumulator (TwoSum), so the FP32 rounding error does not grow with K.
+// accumulator (TwoSum), so the FP32 rounding error does not grow with K.  Runs
+// the static remainder of mixed calls.  Bound at small sizes by the latency of
+// the k-steps' loads and by the FP64 pipe in the weighted sums; 130 x 4099 x 70:
+// 98 us with one k-step in flight (registers), ~20 FP64 instructions per element
+// and 96 blocks, 46 us now (four in flight, 8, 144 blocks of one wave).
 namespace f32 {
 constexpr int BM = 64, BN = 64, BK = 16, THREADS = 256, FLUSH_TILES = 1;
 constexpr int LDA = BM + 1, LDB = BN + 1;
 constexpr size_t SMEM_PIPE = (size_t)2 * BK * (LDA + LDB) * sizeof(float2);
-constexpr size_t SMEM_RED = (size_t)BM * 16 * GMAX * sizeof(double2);
-constexpr size_t SMEM = SMEM_PIPE > SMEM_RED ? SMEM_PIPE : SMEM_RED;
+constexpr int RAW = 4;  // k-steps in flight
+constexpr size_t SMEM = SMEM_PIPE + (size_t)RAW * 8 * THREADS * sizeof(double2);
+static_assert(SMEM >= (size_t)BM * 16 * sizeof(double2), "the row sums' partials fit");
 
-template <class TB> FK_DEV float2 to_f2(TB v);
-template <> FK_DEV float2 to_f2<double2>(double2 v) { return c64_to_f32(v); }
-template <> FK_DEV float2 to_f2<float2>(float2 v) { return v; }
-
-template <int EPI, class TB>
+template <int EPI>
 __global__ void __launch_bounds__(THREADS) contract_kernel(ContractArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2* As = reinterpret_cast<float2*>(smem_raw);  // [2][BK][LDA]
@@ -256,33 +257,37 @@ __global__ void __launch_bounds__(THREADS) contract_kernel(ContractArgs a) {
     const int mt = blockIdx.x, nt = blockIdx.y % NT;
     const int ks = (blockIdx.y / NT) % a.KS, batch = blockIdx.y / (NT * a.KS);
     const int plane = a.batch_plane ? a.batch_plane[batch] : batch;
-    const TB* B = reinterpret_cast<const TB*>(a.B) + (long)plane * a.bstride;
+    const double2* B = reinterpret_cast<const double2*>(a.B) + (long)plane * a.bstride;
     const int k0 = ks * a.kchunk;
     const int k1 = min(a.K, k0 + a.kchunk);
     const int nk = k1 > k0 ? ceil_div(k1 - k0, BK) : 0;
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
 
-    // register staging: 4 A and 4 B complex values per thread per k-step
-    float2 ra[4], rb[4];
+    // k-steps arrive by cp.async as FP64, RAW of them in flight; a thread rounds the
+    // 4 A and 4 B values it copied itself into the FP32 buffers one k-step ahead
+    double2* raw = reinterpret_cast<double2*>(smem_raw + SMEM_PIPE);  // [RAW][8][THREADS]
     auto gload = [&](int kt) {
         const int kb = k0 + kt * BK;
+        double2* dst = raw + (kt % RAW) * 8 * THREADS + tid;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            int idx = tid + i * THREADS;
-            int r = idx / BK, c = idx % BK;
-            int m = mt * BM + r, k = kb + c;
-            ra[i] = (m < a.M && k < k1) ? c64_to_f32(a.A[(long)(a.m0 + m) * a.lda + k]) : make_float2(0.f, 0.f);
-            int n = nt * BN + r;
-            rb[i] = (n < a.N && k < k1) ? to_f2<TB>(B[(long)n * a.ldb + k]) : make_float2(0.f, 0.f);
+            const int idx = tid + i * THREADS;
+            const int r = idx / BK, k = kb + idx % BK;
+            const int m = mt * BM + r, n = nt * BN + r;
+            const bool oka = m < a.M && k < k1, okb = n < a.N && k < k1;
+            d64::cp_async16(dst + i * THREADS, oka ? a.A + (long)(a.m0 + m) * a.lda + k : a.A, oka);
+            d64::cp_async16(dst + (4 + i) * THREADS, okb ? B + (long)n * a.ldb + k : B, okb);
         }
     };
-    auto sstore = [&](int buf) {
+    auto sstore = [&](int kt) {
+        const double2* src = raw + (kt % RAW) * 8 * THREADS + tid;
+        const int buf = kt & 1;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            int idx = tid + i * THREADS;
-            int r = idx / BK, c = idx % BK;
-            As[(buf * BK + c) * LDA + r] = ra[i];
-            Bs[(buf * BK + c) * LDB + r] = rb[i];
+            const int idx = tid + i * THREADS;
+            const int r = idx / BK, c = idx % BK;
+            As[(buf * BK + c) * LDA + r] = c64_to_f32(src[i * THREADS]);
+            Bs[(buf * BK + c) * LDB + r] = c64_to_f32(src[(4 + i) * THREADS]);
         }
     };
 
@@ -297,11 +302,16 @@ __global__ void __launch_bounds__(THREADS) contract_kernel(ContractArgs a) {
             hi_[i][j] = {0.f, 0.f};
         }
 
-    if (nk > 0) { gload(0); sstore(0); }
+#pragma unroll
+    for (int s = 0; s < RAW; ++s) {
+        if (s < nk) gload(s);
+        d64::cp_commit();
+    }
+    d64::cp_wait<RAW - 1>();
+    if (nk > 0) sstore(0);
     __syncthreads();
     for (int kt = 0; kt < nk; ++kt) {
         const int buf = kt & 1;
-        if (kt + 1 < nk) gload(kt + 1);
         const float2* as = As + buf * BK * LDA;
         const float2* bs = Bs + buf * BK * LDB;
 #pragma unroll
@@ -326,24 +336,43 @@ __global__ void __launch_bounds__(THREADS) contract_kernel(ContractArgs a) {
                     acc[i][j] = make_float2(0.f, 0.f);
                 }
         }
-        if (kt + 1 < nk) sstore(buf ^ 1);
+        // the raw slot of this k-step was read an iteration ago, by this thread alone
+        if (kt + RAW < nk) gload(kt + RAW);
+        d64::cp_commit();
+        d64::cp_wait<RAW - 1>();
+        if (kt + 1 < nk) sstore(kt + 1);
         __syncthreads();
     }
 
-    double2* part = reinterpret_cast<double2*>(smem_raw);  // [BM][16 slots][G]
+    // Weighted sums per thread -> smem -> fixed-order row sums.  The FP64 pipe (64
+    // cycles per warp instruction) bounds this part, so a column's scale goes into S
+    // once (2 multiplications) and conj(aqsm) into 4 FMAs, and FP32 is widened with
+    // integer instructions: 8 FP64 instructions per element instead of ~20.
+    static_assert(EPI == EPI_STAT, "one group, columns h = n");
+    double2* part = reinterpret_cast<double2*>(smem_raw);  // [BM][16 slots]
+    double2 gs[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int ml = ty + 16 * i;
-        double2 gs[GMAX] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+    for (int i = 0; i < 4; ++i) gs[i] = make_double2(0.0, 0.0);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            int nl = tx + 16 * j;
-            double2 c = make_double2((double)hr[i][j].hi + (double)hr[i][j].lo,
-                                     (double)hi_[i][j].hi + (double)hi_[i][j].lo);
-            epi_accum<EPI>(a, mt * BM + ml, nt * BN + nl, c, gs);
+    for (int j = 0; j < 4; ++j) {
+        const int n = nt * BN + tx + 16 * j;
+        const int g = n < a.N ? a.igp[n] : -1;
+        if (g < 0) continue;
+        const double s = a.wscale * a.vcoul[g];
+        const long col = a.acol[n];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int m = mt * BM + ty + 16 * i;
+            if (m >= a.M) continue;
+            const double2 am = a.aqsm[contract_row(a, m) * a.ldm + col];
+            const double cx = s * (f32_to_f64(hr[i][j].hi) + f32_to_f64(hr[i][j].lo));
+            const double cy = s * (f32_to_f64(hi_[i][j].hi) + f32_to_f64(hi_[i][j].lo));
+            gs[i].x = fma(am.x, cx, fma(am.y, cy, gs[i].x));
+            gs[i].y = fma(am.x, cy, fma(-am.y, cx, gs[i].y));
         }
-        for (int g = 0; g < a.G; ++g) part[(ml * 16 + tx) * a.G + g] = gs[g];
     }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) part[(ty + 16 * i) * 16 + tx] = gs[i];
     __syncthreads();
     epi_reduce_store<BM, 16>(a, part, mt, (batch * a.KS + ks) * NT + nt);
 }

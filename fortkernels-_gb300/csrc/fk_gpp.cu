@@ -1050,7 +1050,7 @@ FK_DEV void rows_warp(const RowsArgs& ra, int n1, int c, int lane) {
 // instruction-level parallelism, so the sums are laid out to need few FP64
 // warp instructions per warp: lane 5p + s (p < 6: component p/2, real or
 // imaginary part p%2; s < 5) adds slots s, s+5, s+10, .. of its part, and
-// four shuffles add the five splits; lanes 30 and 31 add the static
+// four shuffles add the five splits; lanes 30 and 31 hold the static
 // remainder's parts.  Blocks are four warps (four bands, one per
 // sub-partition); warp 0 then writes the block's partial totals (eight
 // parts: components 0..2 and 6), so the totals read one value per four bands.
@@ -1096,9 +1096,16 @@ FK_DEV void rows_band_warp(const RowsArgs& ra, int n1, int lane, double* parts) 
                 d = __dadd_rn(d, part_of(cscale(cmul(am, ra.schd[h * 3 + c]), 0.5 * ra.vcoul[g]), im));
             }
         }
-    } else if (ra.S) {
-        // static remainder: lane 30 the real, lane 31 the imaginary part
-        for (int k = 0; k < ra.nslots_s; ++k) a = __dadd_rn(a, part_of(ra.S[(long)k * ra.nb + n1], lane - 30));
+    }
+    if (ra.S) {
+        // static remainder: the lanes take slots, a fixed tree adds them; lane 30 keeps
+        // the real, lane 31 the imaginary part
+        double2 v = make_double2(0.0, 0.0);
+        if (lane < ra.nslots_s) v = ordered_sum(ra.S + (long)lane * ra.nb + n1, 32L * ra.nb, (ra.nslots_s - lane + 31) / 32);
+        v = warp_tree(v);
+        v.x = __shfl_sync(0xffffffffu, v.x, 0);
+        v.y = __shfl_sync(0xffffffffu, v.y, 0);
+        if (lane >= 30) a = part_of(v, lane - 30);
     }
     // lane 5p adds the other four splits of part p, in split order (the
     // shuffles read the unmodified split sums a0, b0, d0)
@@ -1354,11 +1361,18 @@ Plan make_plan(const Ctx& c, const GppDev& r, int ks_override = 0, bool pipeline
             p.zW = (size_t)r.ng * M * sizeof(double2);
         }
     }
-    const int per_sm = p.mixed ? 4 : 2;
     const int BM = p.mixed ? f32::BM : d64::BM, BN = p.mixed ? f32::BN : d64::BN;
     p.MTs = ceil_div(r.nb, BM);
     p.NTs = ceil_div(r.ng, BN);
-    pick_split(p.MTs * p.NTs, r.nc, c.sms * per_sm, p.KSs, p.kchunks);
+    if (p.mixed) {
+        // one block per SM (its registers): the k-slices that fill one wave, of at least
+        // 64 k-values; the FP32 sums run over 16-wide k-steps whatever the slice
+        const int ks = std::max(1, std::min(c.sms / std::max(1, p.MTs * p.NTs), std::max(1, r.nc / 64)));
+        p.kchunks = ceil_div(ceil_div(r.nc, ks), 16) * 16;
+        p.KSs = ceil_div(r.nc, p.kchunks);
+    } else {
+        pick_split(p.MTs * p.NTs, r.nc, c.sms * 2, p.KSs, p.kchunks);
+    }
     if (p.tc64 && (r.flags & FK_GPP_ACHSTEMP)) {
         p.NTs = 2 * p.zs.NT;
         p.KSs = p.zs.KS;
@@ -2040,7 +2054,7 @@ fk_status gpp_run(Ctx& c, const GppDev& r, const GppPipe* pipe) {
         a.aqsm = r.aqsm; a.ldm = r.ldm; a.vcoul = r.vcoul; a.igp = igp; a.acol = acol; a.wscale = -0.5; a.G = 1; a.P = S;
         dim3 grid(p.MTs, p.NTs * p.KSs);
         if (p.mixed) {
-            auto k = f32::contract_kernel<EPI_STAT, double2>;
+            auto k = f32::contract_kernel<EPI_STAT>;
             set_smem(k, f32::SMEM);
             k<<<grid, f32::THREADS, f32::SMEM, st>>>(a);
         } else if (p.tc64) {
