@@ -37,8 +37,7 @@ namespace fk {
 namespace {
 
 constexpr int PREP_THREADS = 256;
-constexpr int PREP_EPT = 2;  // elements per thread, FP64 prep
-constexpr int PREP_TILE = PREP_THREADS * PREP_EPT;
+constexpr int PREP_TILE = 2 * PREP_THREADS;  // plane waves per chunk of the FP64 half-sum and real preps
 constexpr int NVC = 2;  // flag bands contracted per prep pass
 constexpr double TO1 = 1e-6;
 constexpr float GUARD = 1e-5f;  // relative guard band of the FP32 branch tests
@@ -249,57 +248,178 @@ FK_DEV void block_sum_ff(float2 (&v)[NV], double2* sm /* [8][NV] */, double2 (&o
     }
 }
 
-// Q = 0: BGW-Kernels/gppKer.cpp; 1: root gppKer.cpp semantics; 2: the Fortran
-// source's (physics mode)
+// Sums of N <= 16 values over a block of 256 threads, in a fixed order: in each
+// step a lane hands half of its values to its partner and adds the partner's
+// half of the others (8 + 4 + 2 + 1 + 1 additions instead of a five-level tree
+// per value), then the warps are added in order.  Thread v < N receives value v.
+template <int N>
+FK_DEV double block_sum_scatter(double (&v)[16], double* sm /* [8][16] */) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int w = 8; w >= 1; w >>= 1) {
+        const bool up = (lane & w) != 0;  // this lane keeps the upper half of its 2w values
+#pragma unroll
+        for (int i = 0; i < w; ++i) {
+            const double give = up ? v[i] : v[i + w], keep = up ? v[i + w] : v[i];
+            v[i] = __dadd_rn(keep, __shfl_xor_sync(0xffffffffu, give, w));
+        }
+    }
+    // lane l (of 16) holds value l; the two halves of the warp
+    v[0] = __dadd_rn(v[0], __shfl_xor_sync(0xffffffffu, v[0], 16));
+    if (lane < 16) sm[warp * 16 + lane] = v[0];
+    __syncthreads();
+    double s = 0.0;
+    if (threadIdx.x < N)
+        for (int w = 0; w < PREP_THREADS / 32; ++w) s = __dadd_rn(s, sm[w * 16 + threadIdx.x]);
+    return s;
+}
+
+// One (igp, ig, iw) element by the reference's FP64 sequence: the value delw*I_eps,
+// sch and ssx, and the noflag mask.  Out of line: the common path keeps its registers.
+struct Element64 {
+    double2 dv, sch, ssx;
+    int A;
+};
 template <int Q>
-__global__ void __launch_bounds__(PREP_THREADS) prep64_kernel(PrepArgs p) {
-    __shared__ double2 sm[8 * NVC * 6];
+__device__ __noinline__ Element64 element64(double wxt, double2 wt, double2 ep, double2 eq, int flags) {
+    const Branch64 b = branch64(wxt, wt);
+    Element64 r;
+    r.A = b.A;
+    r.dv = cmul(b.delw, ep);
+    r.sch = r.ssx = make_double2(0.0, 0.0);
+    if (flags) {
+        const double2 wt2 = cmul(wt, wt);
+        if (b.A) r.sch = cmul(b.delw, eq);
+        r.ssx = ssx64(b, wxt, wt2, cmul(wt2, ep), Q == 2);
+        if (Q == 2) r.ssx = sexcut64(r.ssx, wxt, ep);
+    }
+    return r;
+}
+
+// FP64 prep of chunk ch (tile plane waves) of column my_igp.  Q = 0:
+// BGW-Kernels/gppKer.cpp; 1: root gppKer.cpp semantics; 2: the Fortran source's
+// (physics mode).  SCH = false: the flag bands' sch sums go through the contraction
+// (rows from band 0), only the ssx sums are kept here.
+// Bound by the FP64 pipe (64 cycles per warp instruction on each sub-partition),
+// so the common path spends few FP64 instructions: the branch tests run in FP32
+// on |wdiff|^2 (from its FP64 value) and |wt|^2/|wdiff|^2, any element within a
+// relative 1e-5 of a threshold, out of FP32's comfortable range or not finite
+// takes the reference's sequence (element64), as do the rare branches of ssx; the
+// value wt*I_eps*conj(wdiff)/|wdiff|^2 needs ten (the reciprocal: an FP32 one and
+// two Newton steps, r += r(1 - n r), relative error 2^-23 -> 2^-46 -> 2^-53), and
+// ssx = Omega2/wx^2 six per element and band plus two per frequency.  512 x 2 x
+// 32768 x 20: 339 us with the reference's sequence for every element.
+template <int Q, bool SCH>
+__global__ void __launch_bounds__(PREP_THREADS, 2) prep64_kernel(PrepArgs p) {
+    __shared__ double sm[8 * 16];
     const int my_igp = blockIdx.y, ch = blockIdx.x, tid = threadIdx.x;
     const int igp = prep_setup(p, ch, my_igp);
     const int nflag = min(NVC, p.nv - p.n1base);
-    double2 acc[NVC * 6];
+    const bool flags = nflag > 0 && igp >= 0;
+    const bool all_exact = Q != 0 && flags;
+    const float limitone = 250000.0f, limittwo = 0.25f, to1 = 1e-6f;
+    double2 sx[NVC * 3], sc[SCH ? NVC * 3 : 1];
 #pragma unroll
-    for (int i = 0; i < NVC * 6; ++i) acc[i] = make_double2(0.0, 0.0);
+    for (int i = 0; i < NVC * 3; ++i) {
+        sx[i] = make_double2(0.0, 0.0);
+        if (SCH) sc[i] = make_double2(0.0, 0.0);
+    }
+    double wx[3], iw2[3];
+    bool wok[3];
+#pragma unroll
+    for (int iw = 0; iw < 3; ++iw) {
+        wx[iw] = p.wx[iw];
+        const double w2 = wx[iw] * wx[iw];
+        iw2[iw] = 1.0 / w2;
+        wok[iw] = w2 > 1e-200 && w2 < 1e200;
+    }
     const double2* wrow = p.wt + (long)my_igp * p.nc;
     const double2* erow = p.eps + (long)my_igp * p.nc;
     double2* D = reinterpret_cast<double2*>(p.D);
-    for (int e = 0; e < PREP_EPT; ++e) {
-        const int ig = ch * PREP_TILE + e * PREP_THREADS + tid;
-        if (ig >= p.nc) continue;
+    const int ig_end = min(p.nc, (ch + 1) * p.tile);
+    auto large = [](double v) { return (((unsigned)__double2hiint(v) >> 20) & 0x7ffu) >= 1023u + 60u; };
+    for (int ig = ch * p.tile + tid; ig < ig_end; ig += PREP_THREADS) {
         const double2 wt = wrow[ig], ep = erow[ig];
-        double2 wt2 = make_double2(0, 0), Om = make_double2(0, 0), eq = ep;
-        if (nflag > 0) {
-            wt2 = cmul(wt, wt);
-            Om = cmul(wt2, ep);
-            if (Q == 1) eq = p.eps[(long)my_igp * p.ng + ig];  // gppKer.cpp:139
+        double2 eq = ep, an[NVC], pn[NVC];
+        if (Q == 1 && flags) eq = p.eps[(long)my_igp * p.ng + ig];  // gppKer.cpp:139
+        if (flags) {
+            // aqsntemp*Omega2 of the pass's bands
+            const double2 w2 = make_double2(fma(wt.x, wt.x, -(wt.y * wt.y)), (wt.x + wt.x) * wt.y);
+            const double2 om = make_double2(fma(w2.x, ep.x, -(w2.y * ep.y)), fma(w2.x, ep.y, w2.y * ep.x));
+#pragma unroll
+            for (int j = 0; j < NVC; ++j) {
+                an[j] = j < nflag ? p.aqsn[(long)(p.n1base + j) * p.nc + ig] : make_double2(0.0, 0.0);
+                pn[j] = make_double2(fma(an[j].x, om.x, -(an[j].y * om.y)), fma(an[j].x, om.y, an[j].y * om.x));
+            }
         }
+        const bool weird = all_exact || large(wt.x) || large(wt.y) || large(ep.x) || large(ep.y);
+        const float2 wf = c64_to_f32(wt);
+        const float wsq = wf.x * wf.x + wf.y * wf.y;
+        const double y2 = wt.y * wt.y;
+        const double2 a = make_double2(fma(wt.x, ep.x, -(wt.y * ep.y)), fma(wt.x, ep.y, wt.y * ep.x));
+        const double cx = -(a.y * wt.y), cy = a.x * wt.y;
 #pragma unroll
         for (int iw = 0; iw < 3; ++iw) {
-            const double wxt = p.wx[iw];
-            Branch64 b = branch64(wxt, wt);
-            if (D) {
-                double2 dv = (igp >= 0 && (Q == 1 || b.A)) ? cmul(b.delw, ep) : make_double2(0.0, 0.0);
-                D[((long)my_igp * 3 + iw) * p.nc + ig] = dv;
-            }
-            if (nflag > 0 && igp >= 0) {
-                double2 sch = b.A ? cmul(b.delw, eq) : make_double2(0.0, 0.0);
-                double2 ssx = ssx64(b, wxt, wt2, Om, Q == 2);
-                if (Q == 2) ssx = sexcut64(ssx, wxt, ep);
+            const double wd = __dsub_rn(wx[iw], wt.x);
+            const double n = fma(wd, wd, y2);
+            const float nf = f64_to_f32_bits(n), rf = __frcp_rn(nf), dr = wsq * rf;
+            const bool amb = weird || !wok[iw] || !(nf > 1e-30f) || !(nf < 1e30f) || !(dr < 1e30f) ||
+                             fabsf(nf - limittwo) <= limittwo * GUARD || fabsf(dr - limitone) <= limitone * GUARD ||
+                             (flags && fabsf(dr - to1) <= to1 * GUARD);
+            bool A = nf > limittwo && dr < limitone;
+            // the sequence itself: near a threshold, or ssx of the branches but the common one
+            const bool seq = amb || (flags && !A && dr > to1);
+            double2 dv;
+            if (seq) {
+                const Element64 x = element64<Q>(wx[iw], wt, ep, eq, flags);
+                A = x.A != 0;
+                dv = x.dv;
+                if (flags)
 #pragma unroll
-                for (int j = 0; j < NVC; ++j)
-                    if (j < nflag) {
-                        double2 an = p.aqsn[(long)(p.n1base + j) * p.nc + ig];
-                        cfma(acc[(j * 3 + iw) * 2 + 0], an, sch);
-                        cfma(acc[(j * 3 + iw) * 2 + 1], an, ssx);
+                    for (int j = 0; j < NVC; ++j) {
+                        cfma(sx[j * 3 + iw], an[j], x.ssx);
+                        if (SCH) cfma(sc[SCH ? j * 3 + iw : 0], an[j], x.sch);
                     }
+            } else {
+                double r = f32_to_f64_bits(rf);
+                r = fma(r, fma(-n, r, 1.0), r);
+                r = fma(r, fma(-n, r, 1.0), r);
+                dv = make_double2(fma(a.x, wd, cx) * r, fma(a.y, wd, cy) * r);
+                if (flags && A)
+#pragma unroll
+                    for (int j = 0; j < NVC; ++j) {
+                        sx[j * 3 + iw].x = fma(pn[j].x, iw2[iw], sx[j * 3 + iw].x);
+                        sx[j * 3 + iw].y = fma(pn[j].y, iw2[iw], sx[j * 3 + iw].y);
+                        if (SCH) cfma(sc[SCH ? j * 3 + iw : 0], an[j], dv);
+                    }
+            }
+            if (D) {
+                const bool keep = igp >= 0 && (Q == 1 || A);
+                D[((long)my_igp * 3 + iw) * p.nc + ig] = keep ? dv : make_double2(0.0, 0.0);
             }
         }
     }
     if (nflag <= 0) return;
-    block_sum<NVC * 6>(acc, sm);
-    if (tid < nflag * 6) {
-        int j = tid / 6, r = tid % 6;
-        p.F[(((long)ch * p.nv + p.n1base + j) * p.ng + my_igp) * 6 + r] = acc[tid];
+    // F[..][iw * 2 + kind], kind 0 sch, 1 ssx
+    double* F = (double*)(p.F + ((long)ch * p.nv * p.ng) * 6);
+    auto put = [&](double2(&s)[NVC * 3], int kind) {
+        double v[16];
+#pragma unroll
+        for (int i = 0; i < NVC * 3; ++i) {
+            v[2 * i] = s[i].x;
+            v[2 * i + 1] = s[i].y;
+        }
+#pragma unroll
+        for (int i = NVC * 6; i < 16; ++i) v[i] = 0.0;
+        const double x = block_sum_scatter<NVC * 6>(v, sm);
+        const int j = tid / 6, q = tid % 6;  // band, (frequency, re or im)
+        if (tid < nflag * 6)
+            F[(((long)(p.n1base + j) * p.ng + my_igp) * 6 + (q >> 1) * 2 + kind) * 2 + (q & 1)] = x;
+    };
+    put(sx, 1);
+    if constexpr (SCH) {
+        __syncthreads();  // sm is reused
+        put(sc, 0);
     }
 }
 
@@ -1250,11 +1370,11 @@ struct Plan {
     size_t bytesZ() const { return tc64 ? zA + zB + zEa + zEb + zW + 5 * 256 : 0; }
 };
 
-// fk_gpp's mixed path (not the half sum, not the root file's flag-band I_eps
-// indexing, whose sch differs from the image's values) contracts the occupied
+// fk_gpp's mixed path and its FP64 path on the tensor cores (not the half sum, not
+// the root file's flag-band I_eps indexing, whose sch differs from the image's values) contracts the occupied
 // bands too: their sch terms are the image's products.
 inline bool gpp_fsch(const GppDev& r) {
-    return r.prec == FK_MIXED && !(r.flags & (FK_GPP_HALF_SUM | FK_GPP_ROOT_QUIRKS));
+    return (r.prec == FK_MIXED || r.tc64) && !(r.flags & (FK_GPP_HALF_SUM | FK_GPP_ROOT_QUIRKS));
 }
 
 // k-slice count for the persistent tensor-core kernel: the fewest slices
@@ -1290,7 +1410,16 @@ Plan make_plan(const Ctx& c, const GppDev& r, int ks_override = 0, bool pipeline
                bool fsch = false) {
     Plan p{};
     p.mixed = r.prec == FK_MIXED;
-    p.fsch = fsch && p.mixed;
+    if (!p.mixed && r.tc64) {
+        // FP64 on the tensor cores, where a split of both contractions exists
+        const int M = r.nb - (fsch ? 0 : r.nv);
+        if (M > 0) {
+            p.z = tc64::make_plan(M, 3 * r.ng, r.nc, 1, c.sms / 2);
+            if (r.flags & FK_GPP_ACHSTEMP) p.zs = tc64::make_plan(r.nb, r.ng, r.nc, 1, c.sms / 2);
+            p.tc64 = p.z.KS && (p.zs.KS || !(r.flags & FK_GPP_ACHSTEMP));
+        }
+    }
+    p.fsch = fsch && (p.mixed || p.tc64);
     p.m0 = p.fsch ? 0 : r.nv;
     p.pipe_sub = p.pipe_chunks = 0;
     if (r.prec == FK_MIXED) {
@@ -1305,8 +1434,11 @@ Plan make_plan(const Ctx& c, const GppDev& r, int ks_override = 0, bool pipeline
         p.tile = ceil_div(ceil_div(r.nc, nch), tcx::BK) * tcx::BK;
         p.nch = ceil_div(r.nc, p.tile);
     } else {
-        p.tile = PREP_TILE;
-        p.nch = ceil_div(r.nc, PREP_TILE);
+        // one wave of two resident blocks per SM; each chunk is one partial per flag band
+        // and column for the band reduction
+        const int nch = std::max(1, 2 * c.sms / r.ng);
+        p.tile = ceil_div(ceil_div(r.nc, nch), PREP_THREADS) * PREP_THREADS;
+        p.nch = ceil_div(r.nc, p.tile);
     }
     const bool half = (r.flags & FK_GPP_HALF_SUM) != 0;
     if (half) {
@@ -1346,11 +1478,6 @@ Plan make_plan(const Ctx& c, const GppDev& r, int ks_override = 0, bool pipeline
         p.MT = ceil_div(std::max(M, 1), d64::BM);
         p.NT = ceil_div(N, d64::BN);
         pick_split(p.MT * p.NT, r.nc, c.sms * 2, p.KS, p.kchunk);
-        if (r.tc64 && M > 0) {
-            p.z = tc64::make_plan(M, N, r.nc, 1, c.sms / 2);
-            if (r.flags & FK_GPP_ACHSTEMP) p.zs = tc64::make_plan(r.nb, r.ng, r.nc, 1, c.sms / 2);
-            p.tc64 = p.z.KS && (p.zs.KS || !(r.flags & FK_GPP_ACHSTEMP));
-        }
         if (p.tc64) {
             p.NT = 2 * p.z.NT;  // its partial slots: the re and im half of each 64-wide n-tile
             p.KS = p.z.KS;
@@ -1936,9 +2063,9 @@ fk_status gpp_run(Ctx& c, const GppDev& r, const GppPipe* pipe) {
             else if (Q == 2) prep_mixed_kernel<2, 64><<<grid, PREP_THREADS, 0, st>>>(a);
             else prep_mixed_kernel<0, 64><<<grid, PREP_THREADS, 0, st>>>(a);
         } else {
-            if (Q == 1) prep64_kernel<1><<<grid, PREP_THREADS, 0, st>>>(a);
-            else if (Q == 2) prep64_kernel<2><<<grid, PREP_THREADS, 0, st>>>(a);
-            else prep64_kernel<0><<<grid, PREP_THREADS, 0, st>>>(a);
+            auto k = p.fsch ? (Q == 2 ? prep64_kernel<2, false> : prep64_kernel<0, false>)
+                            : (Q == 1 ? prep64_kernel<1, true> : Q == 2 ? prep64_kernel<2, true> : prep64_kernel<0, true>);
+            k<<<grid, PREP_THREADS, 0, st>>>(a);
         }
         ++c.launches;
     };
