@@ -48,6 +48,7 @@
 #include "fk_gemm.cuh"
 #include "fk_internal.h"
 #include "fk_tc.cuh"
+#include "fk_tc_contract.cuh"
 
 namespace fk {
 namespace tc64 {
@@ -98,6 +99,8 @@ struct SplitArgs {
     uint8_t* img;
     int* exps;           // [plane][slice][rows]
     int* flag;
+    int* err;
+    long long wait_limit;
 };
 
 __device__ __forceinline__ unsigned long long abs_bits(double v) {
@@ -124,22 +127,82 @@ __device__ __forceinline__ uint32_t digit_pair(unsigned long long u0, unsigned l
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// One block per (k-slice, row, plane): the slice's largest magnitude, then its
-// digits, 16-byte swizzle chunks of 8 k-values.  Memory-bound: reads 16 and
-// writes 28 (A) or 42 (B, with -im) bytes per complex value.  The second read
-// of the slice hits the caches.
+// The digits of 8 values k .. k+7 of image row `row`: one 16-byte swizzle chunk per
+// digit and part (tile: the row tile's image).
 template <bool BSIDE>
-__global__ void __launch_bounds__(128) split_kernel(SplitArgs s) {
+__device__ __forceinline__ void store_digits(uint8_t* tile, int row, int k, const double2 (&v)[8], int emax) {
+    constexpr int R = BSIDE ? BN : 128;
+    unsigned long long ur[8], ui[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        ur[j] = biased_fixed(v[j].x, emax);
+        ui[j] = biased_fixed(v[j].y, emax);
+    }
+    uint8_t* st = tile + (long)(k / BK) * (ND * (BSIDE ? B_IMG : A_DIG)) + tc::sw64_offset(row % R, k % BK);
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+        uint4 re, im;
+        re.x = digit_pair(ur[0], ur[1], d); re.y = digit_pair(ur[2], ur[3], d);
+        re.z = digit_pair(ur[4], ur[5], d); re.w = digit_pair(ur[6], ur[7], d);
+        im.x = digit_pair(ui[0], ui[1], d); im.y = digit_pair(ui[2], ui[3], d);
+        im.z = digit_pair(ui[4], ui[5], d); im.w = digit_pair(ui[6], ui[7], d);
+        if (BSIDE) {
+            uint8_t* q = st + (long)d * B_IMG;
+            *(uint4*)q = im;
+            *(uint4*)(q + 4096) = re;
+            *(uint4*)(q + 8192) = make_uint4(im.x ^ 0x80008000u, im.y ^ 0x80008000u, im.z ^ 0x80008000u, im.w ^ 0x80008000u);
+        } else {
+            uint8_t* q = st + (long)d * A_DIG;
+            *(uint4*)q = re;
+            *(uint4*)(q + 8192) = im;
+        }
+    }
+}
+
+// One block per (k-slice, row, plane): the slice's largest magnitude, then its
+// digits.  Memory-bound: reads 16 and writes 28 (A) or 42 (B, with -im) bytes per
+// complex value.  SMEM: the slice (at most SMEM_K k-values) comes to shared memory
+// by bulk copies, several blocks per SM overlapping theirs with the others' digits,
+// and a thread reads its 8 values in an order rotated by its lane
+// (tcx::smem_chunk8); longer slices are read twice from global memory.
+constexpr int SMEM_K = 4096;
+template <bool BSIDE, bool SMEM_ROW>
+__global__ void __launch_bounds__(256) split_kernel(SplitArgs s) {
+    extern __shared__ __align__(16) uint8_t smem_row[];
+    const double2* rowbuf = (const double2*)smem_row;
     const int ks = blockIdx.x, batch = blockIdx.z;
     const int plane = s.planes ? s.planes[batch] : batch;
     const int kst0 = ks * s.kst_unit, kst1 = min(s.kstages, kst0 + s.kst_unit);
-    const int k0 = kst0 * BK, k1 = min(s.K, kst1 * BK);
-    __shared__ unsigned long long wm[4];
-    for (int row = blockIdx.y; row < s.rows; row += gridDim.y) {
-        const double2* src = s.src + (long)plane * s.plane_stride + (long)(s.rowmap ? s.rowmap[row] : row) * s.ld;
+    const int k0 = kst0 * BK, k1 = min(s.K, kst1 * BK), nk = k1 - k0;
+    __shared__ unsigned long long wm[8];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ int ok;
+    if (SMEM_ROW && threadIdx.x == 0) {
+        tc::mbar_init(&bar, 1);
+        tc::fence_barrier_init();
+    }
+    uint32_t ph = 0;
+    for (int row = blockIdx.y; row < s.rows; row += gridDim.y, ph ^= 1) {
+        const double2* src = s.src + (long)plane * s.plane_stride + (long)(s.rowmap ? s.rowmap[row] : row) * s.ld + k0;
+        if (SMEM_ROW) {
+            __syncthreads();  // the previous row was read
+            if (threadIdx.x == 0) {
+                const uint32_t bytes = (uint32_t)nk * 16u;
+                tc::mbar_arrive_expect_tx(&bar, bytes);
+                for (uint32_t o = 0; o < bytes; o += 16384u)
+                    tc::bulk_g2s(smem_row + o, (const uint8_t*)src + o, min(16384u, bytes - o), &bar);
+                ok = tc::mbar_wait(&bar, ph, s.wait_limit) ? 1 : 0;
+                if (!ok) {  // the block exits only after its copy has landed
+                    atomicOr(s.err, 0x200);
+                    tc::mbar_wait(&bar, ph, DRAIN_LIMIT);
+                }
+            }
+            __syncthreads();
+            if (!ok) return;
+        }
         unsigned long long mx = 0;
-        for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
-            const double2 v = src[k];
+        for (int k = threadIdx.x; k < nk; k += blockDim.x) {
+            const double2 v = SMEM_ROW ? rowbuf[k] : src[k];
             mx = max(mx, max(abs_bits(v.x), abs_bits(v.y)));
         }
 #pragma unroll
@@ -155,39 +218,17 @@ __global__ void __launch_bounds__(128) split_kernel(SplitArgs s) {
             s.exps[((long)batch * s.KS + ks) * s.rows + row] = mx ? emax - 1023 : 0;
             if (bad) atomicOr(s.flag, 1);
         }
-        const int R = BSIDE ? BN : 128;
-        uint8_t* tile = s.img + ((long)batch * s.tiles + row / R) * s.kstages * (long)(ND * (BSIDE ? B_IMG : A_DIG));
-        for (int c = kst0 * 4 + threadIdx.x; c < kst1 * 4; c += blockDim.x) {
-            const int k = 8 * c;
+        uint8_t* tile = s.img + ((long)batch * s.tiles + row / (BSIDE ? BN : 128)) * s.kstages *
+                                    (long)(ND * (BSIDE ? B_IMG : A_DIG));
+        for (int c = 8 * threadIdx.x; c < (kst1 - kst0) * BK; c += 8 * blockDim.x) {
             double2 v[8];
+            if (SMEM_ROW) {
+                tcx::smem_chunk8(rowbuf, c, nk, v);
+            } else {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = k + j < k1 ? src[k + j] : make_double2(0.0, 0.0);
-            unsigned long long ur[8], ui[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                ur[j] = biased_fixed(v[j].x, emax);
-                ui[j] = biased_fixed(v[j].y, emax);
+                for (int j = 0; j < 8; ++j) v[j] = c + j < nk ? src[c + j] : make_double2(0.0, 0.0);
             }
-            uint8_t* st = tile + (long)(c >> 2) * (ND * (BSIDE ? B_IMG : A_DIG)) + tc::sw64_offset(row % R, k % BK);
-#pragma unroll
-            for (int d = 0; d < ND; ++d) {
-                uint4 re, im;
-                re.x = digit_pair(ur[0], ur[1], d); re.y = digit_pair(ur[2], ur[3], d);
-                re.z = digit_pair(ur[4], ur[5], d); re.w = digit_pair(ur[6], ur[7], d);
-                im.x = digit_pair(ui[0], ui[1], d); im.y = digit_pair(ui[2], ui[3], d);
-                im.z = digit_pair(ui[4], ui[5], d); im.w = digit_pair(ui[6], ui[7], d);
-                if (BSIDE) {
-                    uint8_t* q = st + (long)d * B_IMG;
-                    *(uint4*)q = im;
-                    *(uint4*)(q + 4096) = re;
-                    *(uint4*)(q + 8192) = make_uint4(im.x ^ 0x80008000u, im.y ^ 0x80008000u, im.z ^ 0x80008000u,
-                                                     im.w ^ 0x80008000u);
-                } else {
-                    uint8_t* q = st + (long)d * A_DIG;
-                    *(uint4*)q = re;
-                    *(uint4*)(q + 8192) = im;
-                }
-            }
+            store_digits<BSIDE>(tile, row, k0 + c, v, emax);
         }
     }
 }
@@ -653,13 +694,27 @@ struct Bufs {
 // Set when a row cannot be represented (a word beside the error word).
 inline int* flag_word(const Ctx& c) { return c.errword + 16; }
 
+template <bool BSIDE>
+inline void launch_split(Ctx& c, const SplitArgs& s, int batches) {
+    const int nk = s.kst_unit * BK;
+    const dim3 grid(s.KS, std::min(s.rows, 65535), batches);
+    const int threads = nk > 1024 ? 256 : 128;
+    if (nk <= SMEM_K) {
+        auto k = split_kernel<BSIDE, true>;
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_K * 16);
+        k<<<grid, threads, nk * 16, c.stream>>>(s);
+    } else {
+        split_kernel<BSIDE, false><<<grid, threads, 0, c.stream>>>(s);
+    }
+    ++c.launches;
+}
+
 // The digits of a.A's rows m0 .. m0+M-1 (or rowmap[0 .. M)) and the flag's reset.
 inline void enqueue_a(Ctx& c, const ContractArgs& a, const Plan& p, const Bufs& b) {
     cudaMemsetAsync(flag_word(c), 0, sizeof(int), c.stream);
     SplitArgs s{a.rowmap ? a.A : a.A + (long)a.m0 * a.lda, a.lda, 0, nullptr, a.rowmap, a.M, a.K, p.KS, p.kst_unit,
-                p.kstages, 2 * p.MT, b.A, b.ea, flag_word(c)};
-    split_kernel<false><<<dim3(p.KS, std::min(a.M, 65535), 1), 128, 0, c.stream>>>(s);
-    ++c.launches;
+                p.kstages, 2 * p.MT, b.A, b.ea, flag_word(c), c.errword, c.wait_limit};
+    launch_split<false>(c, s, 1);
 }
 
 // The digits of a.batches planes (at most MAXPL) of a.B, the contraction over the row tiles of `tab` and the
@@ -667,8 +722,8 @@ inline void enqueue_a(Ctx& c, const ContractArgs& a, const Plan& p, const Bufs& 
 template <int EPI>
 inline void enqueue(Ctx& c, ContractArgs a, const Plan& p, const Bufs& b, const PlaneTab& tab, bool second) {
     SplitArgs s{(const double2*)a.B, a.ldb, a.bstride, a.batch_plane, nullptr, a.N, a.K, p.KS, p.kst_unit, p.kstages,
-                p.NT, b.B, b.eb, flag_word(c)};
-    split_kernel<true><<<dim3(p.KS, std::min(a.N, 65535), a.batches), 128, 0, c.stream>>>(s);
+                p.NT, b.B, b.eb, flag_word(c), c.errword, c.wait_limit};
+    launch_split<true>(c, s, a.batches);
     Args t{b.A, b.B, b.ea, b.eb, b.W1, second ? b.W2 : nullptr, a.P, a.M, a.N, p.NT, p.KS, p.kst_unit, p.kstages, a.G,
            flag_word(c), c.errword, c.wait_limit, tab};
     auto k = contract_kernel<EPI>;
@@ -683,7 +738,7 @@ inline void enqueue(Ctx& c, ContractArgs a, const Plan& p, const Bufs& b, const 
     auto f = d64::contract_kernel<EPI>;
     cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d64::SMEM);
     f<<<dim3(ceil_div(a.M, d64::BM), a.nt_tiles * a.KS * a.batches), d64::THREADS, d64::SMEM, c.stream>>>(a);
-    c.launches += 3;
+    c.launches += 2;
 }
 
 inline void enqueue_weights(Ctx& c, const ContractArgs& a, int ncols, const Bufs& b, bool second) {
