@@ -936,23 +936,35 @@ fk_status fk_ff(fk_ctx_t c, int nb, int nv, int nc, int ng, int nf, int ne, cons
     r.nb = nb; r.nv = nv; r.nc = nc; r.ng = ng; r.nf = nf; r.ne = ne;
     r.pref_zb = pref_zb; r.fmin = freqevalmin; r.fstep = freqevalstep; r.occ = occ;
     r.prec = precision; r.flags = flags;
-    r.ekq = ekq; r.grid = dFreqGrid;  // host or device; only read by the planner
+    if (fk::capturing(x.stream)) return fk::fail(x, FK_ECUDA, "ff: not supported during stream capture");
+    // the planner reads ekq and dFreqGrid on the host: host arrays where they lie,
+    // device arrays behind the work queued so far
+    fk::FfHost hf{ekq, dFreqGrid, nullptr};
+    std::vector<double> ekq_h, grid_h;
+    if (ek.dev || gr.dev) {
+        ekq_h.resize(nb);
+        grid_h.resize(nf);
+        cudaError_t e = cudaMemcpyAsync(ekq_h.data(), ekq, nb * sizeof(double), cudaMemcpyDefault, x.stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(grid_h.data(), dFreqGrid, nf * sizeof(double), cudaMemcpyDefault, x.stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(x.stream);
+        if (e != cudaSuccess) return fk::cuda_fail(x, e, "ff: reading ekq/dFreqGrid");
+        hf.ekq = ekq_h.data();
+        hf.grid = grid_h.data();
+    }
     // host I_epsR / I_epsA of a large request: streamed in plane groups while
     // the groups already copied are being computed (fk::FfPipe)
-    const bool pipelined = !er.dev && !ea.dev && planes >= ((size_t)64 << 20) && !fk::capturing(x.stream);
+    const bool pipelined = !er.dev && !ea.dev && planes >= ((size_t)64 << 20);
     const size_t outn = 1 + 4 * (size_t)ne + (size_t)nb * nf;
     auto r256 = [](size_t b) { return (b + 255) & ~(size_t)255; };
-    std::vector<fk::In*> small{&vc, &inv, &ind, &ek, &gr, &br, &pr}, bands{&aqm, &aqn};
-    size_t packed = 0;
+    std::vector<fk::In*> small{&vc, &inv, &ind, &ek, &gr, &br, &pr}, bands{&aqm, &aqn}, large{&aqm, &aqn, &er, &ea};
+    size_t packed = 0, packed_host = 0;
     for (auto* i : small)
         if (!fk::in_place(i)) packed += r256(i->bytes);
     size_t need = 0;
     for (int tc = precision == FK_FP64 ? 1 : 0; tc >= 0; --tc) {  // as in fk_gpp
         r.tc64 = tc != 0;
-        const size_t wsb = fk::ff_workspace(x, r, pipelined);
-        if (wsb == (size_t)-1) return fk::fail(x, FK_ECUDA, "ff: reading ekq/dFreqGrid");
-        need = (pipelined ? fk::staged_bytes(bands) + 2 * r256(planes) + r256(packed) : fk::staged_bytes(ins)) + wsb +
-               outn * sizeof(double2) + 4096;
+        need = fk::staged_bytes(pipelined ? bands : large) + (pipelined ? 2 * r256(planes) : 0) + r256(packed) +
+               fk::ff_workspace(x, r, hf, pipelined) + outn * sizeof(double2) + 4096;
         if (!tc || fk::workspace_can_hold(x, need)) break;
     }
     fk_status s = fk::ensure_workspace(x, need);
@@ -961,49 +973,48 @@ fk_status fk_ff(fk_ctx_t c, int nb, int nv, int nc, int ng, int nf, int ne, cons
     double2* out = (double2*)x.ws.take(outn * sizeof(double2));
     fk::phase_mark(x, 0);
     fk::FfPipe pipe{};
-    std::vector<double> ekq_h, grid_h;
-    if (!pipelined) {
-        if ((s = fk::stage(x, ins)) != FK_OK) return s;
-    } else {
-        // small inputs packed into pinned memory, then aqsmtemp and aqsntemp, on
-        // the copy stream ahead of the planes; the planner reads ekq and dFreqGrid on the host
-        pipe.ekq_h = ekq;
-        pipe.grid_h = dFreqGrid;
-        if (ek.dev || gr.dev) {
-            ekq_h.resize(nb);
-            grid_h.resize(nf);
-            if (cudaMemcpy(ekq_h.data(), ekq, nb * sizeof(double), cudaMemcpyDefault) != cudaSuccess ||
-                cudaMemcpy(grid_h.data(), dFreqGrid, nf * sizeof(double), cudaMemcpyDefault) != cudaSuccess)
-                return fk::cuda_fail(x, cudaGetLastError(), "ff: reading ekq/dFreqGrid");
-            pipe.ekq_h = ekq_h.data();
-            pipe.grid_h = grid_h.data();
+    // small inputs (and the planner's tables) through the pinned buffer: one copy
+    // each, and the call does not wait for the stream; it holds the previous call's
+    // until their copies are done
+    uint8_t* small_d = packed ? (uint8_t*)x.ws.take(packed) : nullptr;
+    uint8_t* pb = (uint8_t*)fk::pinned_buffer(x, packed + fk::ff_table_bytes(r));
+    if (!out || (packed && !small_d)) return fk::fail(x, FK_ENOMEM, "workspace: staging");
+    if (!pb) return fk::fail(x, FK_ENOMEM, "ff: pinned staging");
+    hf.tab = pb + packed;
+    size_t off = 0;
+    for (int dev = 0; dev < 2; ++dev)  // the host arrays first: one copy; then device ones off a 16-byte boundary
+        for (auto* i : small) {
+            if (fk::in_place(i)) i->d = i->user;
+            if (fk::in_place(i) || (int)i->dev != dev) continue;
+            i->d = small_d + off;
+            if (!dev) {
+                std::memcpy(pb + off, i->user, i->bytes);
+                x.h2d_bytes += i->bytes;
+            } else if (cudaMemcpyAsync(small_d + off, i->user, i->bytes, cudaMemcpyDeviceToDevice, x.stream) != cudaSuccess) {
+                return fk::cuda_fail(x, cudaGetLastError(), "staging copy");
+            }
+            off += r256(i->bytes);
+            if (!dev) packed_host = off;
         }
+    cudaStream_t cs = x.stream;
+    if (pipelined) {  // the small inputs, then aqsmtemp and aqsntemp, on the copy stream ahead of the planes
+        if ((s = fk::pipe_begin(x)) != FK_OK) return s;
+        cs = x.copy_stream;
+    }
+    if (packed_host) {
+        cudaError_t e = cudaMemcpyAsync(small_d, pb, packed_host, cudaMemcpyHostToDevice, cs);
+        if (e == cudaSuccess) e = cudaEventRecord(x.pinned_ev, cs);
+        if (e != cudaSuccess) return fk::cuda_fail(x, e, "ff: small inputs");
+    }
+    if (!pipelined) {
+        if ((s = fk::stage(x, large)) != FK_OK) return s;
+    } else {
         pipe.epsR = (const double2*)I_epsR_array;
         pipe.epsA = (const double2*)I_epsA_array;
         pipe.epsR_d = (double2*)x.ws.take(planes);
         pipe.epsA_d = (double2*)x.ws.take(planes);
-        uint8_t* small_d = packed ? (uint8_t*)x.ws.take(packed) : nullptr;
-        if (!out || !pipe.epsR_d || !pipe.epsA_d || (packed && !small_d)) return fk::fail(x, FK_ENOMEM, "workspace: pipeline");
-        uint8_t* pb = packed ? (uint8_t*)fk::pinned_buffer(x, packed) : nullptr;  // free once its last copy is done
-        if (packed && !pb) return fk::fail(x, FK_ENOMEM, "ff: pinned staging");
-        if ((s = fk::pipe_begin(x)) != FK_OK) return s;
-        cudaStream_t cs = x.copy_stream;
-        size_t off = 0;
-        for (auto* i : small) {
-            if (fk::in_place(i)) {
-                i->d = i->user;
-                continue;
-            }
-            std::memcpy(pb + off, i->user, i->bytes);
-            x.h2d_bytes += i->bytes;
-            i->d = small_d + off;
-            off += r256(i->bytes);
-        }
+        if (!pipe.epsR_d || !pipe.epsA_d) return fk::fail(x, FK_ENOMEM, "workspace: pipeline");
         cudaError_t e = cudaSuccess;
-        if (packed) {
-            e = cudaMemcpyAsync(small_d, pb, packed, cudaMemcpyHostToDevice, cs);
-            if (e == cudaSuccess) e = cudaEventRecord(x.pinned_ev, cs);
-        }
         for (auto* i : bands) {
             if (e != cudaSuccess) break;
             if (fk::in_place(i)) {
@@ -1025,7 +1036,7 @@ fk_status fk_ff(fk_ctx_t c, int nb, int nv, int nc, int ng, int nf, int ne, cons
     r.epsR = (const double2*)er.d; r.epsA = (const double2*)ea.d; r.brd = (const double2*)br.d;
     r.vcoul = (const double*)vc.d; r.ekq = (const double*)ek.d; r.grid = (const double*)gr.d;
     r.pref = (const double*)pr.d; r.inv = (const int*)inv.d; r.indinv = (const int*)ind.d; r.out = out;
-    if ((s = fk::ff_run(x, r, pipelined ? &pipe : nullptr)) != FK_OK) return s;
+    if ((s = fk::ff_run(x, r, hf, pipelined ? &pipe : nullptr)) != FK_OK) return s;
     bool host_out = false;
     if ((s = fk::deliver(x, achsDtemp, out, 0, 1, host_out)) != FK_OK) return s;
     if ((s = fk::deliver(x, asxDtemp, out, 1, ne, host_out)) != FK_OK) return s;

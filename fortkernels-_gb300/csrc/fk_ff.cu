@@ -15,6 +15,7 @@
 // calculate_schDt_lin3, achDtemp_Kernel's frequency sums) in FP64.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "fk_gemm.cuh"
@@ -471,36 +472,35 @@ FfPlan make_plan(const Ctx& c, const FfDev& r, const double* ekq_h, const double
 
 }  // namespace
 
-size_t ff_workspace(const Ctx& c, const FfDev& r, bool pipelined) {
-    std::vector<double> ekq(r.nb), grid(r.nf);
-    if (cudaMemcpy(ekq.data(), r.ekq, r.nb * sizeof(double), cudaMemcpyDefault) != cudaSuccess ||
-        cudaMemcpy(grid.data(), r.grid, r.nf * sizeof(double), cudaMemcpyDefault) != cudaSuccess)
-        return (size_t)-1;
-    return make_plan(c, r, ekq.data(), grid.data(), pipelined).bytes;
+// The planner's tables on the device: one block, copied at once.
+struct FfTables {
+    size_t order, planes, bytes;  // offsets behind the FactRow of each band
+    explicit FfTables(const FfDev& r) {
+        auto r256 = [](size_t b) { return (b + 255) & ~(size_t)255; };
+        order = r256(r.nb * sizeof(FactRow));
+        planes = order + r256(r.nb * sizeof(int));
+        bytes = planes + r256(2 * (size_t)r.nf * sizeof(int));
+    }
+};
+size_t ff_table_bytes(const FfDev& r) { return FfTables(r).bytes; }
+
+size_t ff_workspace(const Ctx& c, const FfDev& r, const FfHost& h, bool pipelined) {
+    return make_plan(c, r, h.ekq, h.grid, pipelined).bytes + FfTables(r).bytes;
 }
 
-fk_status ff_run(Ctx& c, const FfDev& r, const FfPipe* pipe) {
-    std::vector<double> ekq, grid;
+fk_status ff_run(Ctx& c, const FfDev& r, const FfHost& h, const FfPipe* pipe) {
     cudaError_t e = cudaSuccess;
-    if (!pipe) {
-        ekq.resize(r.nb);
-        grid.resize(r.nf);
-        e = cudaMemcpyAsync(ekq.data(), r.ekq, r.nb * sizeof(double), cudaMemcpyDefault, c.stream);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(grid.data(), r.grid, r.nf * sizeof(double), cudaMemcpyDefault, c.stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);
-        if (e != cudaSuccess) return cuda_fail(c, e, "ff: reading ekq/dFreqGrid");
-    }
-    const FfPlan p = pipe ? make_plan(c, r, pipe->ekq_h, pipe->grid_h, true)
-                          : make_plan(c, r, ekq.data(), grid.data(), false);
+    const FfPlan p = make_plan(c, r, h.ekq, h.grid, pipe != nullptr);
     cudaStream_t st = c.stream;
     const int nR = (int)p.planesR.size(), nA = (int)p.planesA.size();
     const size_t slots = (size_t)p.KS * p.NT * (p.mixed ? tcx::FF_EPI_WARPS : 1);  // partial slots per plane
     const size_t slotsA = p.mixed ? (size_t)p.KSa * p.NT * tcx::FF_EPI_WARPS : slots;
     int* igp = (int*)c.ws.take(r.ng * sizeof(int));
-    int* order = p.mixed || p.tc64 ? (int*)c.ws.take(r.nb * sizeof(int)) : nullptr;
-    int* planes = (int*)c.ws.take((nR + nA) * sizeof(int));
-    FactRow* fact = (FactRow*)c.ws.take(r.nb * sizeof(FactRow));
+    const FfTables ft(r);
+    uint8_t* tab = (uint8_t*)c.ws.take(ft.bytes);
+    FactRow* fact = (FactRow*)tab;
+    int* order = p.mixed || p.tc64 ? (int*)(tab + ft.order) : nullptr;
+    int* planes = (int*)(tab + ft.planes);
     double2* PR = (double2*)c.ws.take(slots * std::max(nR, 1) * r.nb * 2 * sizeof(double2));
     double2* PA = nA ? (double2*)c.ws.take(slotsA * nA * r.nb * 2 * sizeof(double2)) : nullptr;
     double2* tabs = (double2*)c.ws.take(3 * (size_t)r.nb * r.nf * sizeof(double2));
@@ -531,17 +531,18 @@ fk_status ff_run(Ctx& c, const FfDev& r, const FfPipe* pipe) {
         if (!zb.A || !zb.B || !zb.ea || !zb.eb || !zb.W1 || !zb.W2)
             return fail(c, FK_ENOMEM, "workspace too small for FF request");
     }
-    if (!igp || ((p.mixed || p.tc64) && !order) || !planes || !fact || !PR || (nA && !PA) || !tabs || !SD || (p.bytesImgR && !imgR) ||
+    if (!igp || !tab || !PR || (nA && !PA) || !tabs || !SD || (p.bytesImgR && !imgR) ||
         (p.bytesImgA && !imgA) || (p.bytesW && !W) || (p.bytesAimg && !Aimg) || (p.bytesScale && !scales))
         return fail(c, FK_ENOMEM, "workspace too small for FF request");
     double2 *RW = tabs, *RS = tabs + (size_t)r.nb * r.nf, *AW = tabs + 2 * (size_t)r.nb * r.nf;
-    // host tables -> device (pageable source; the copy completes before return of the call's sync)
-    std::vector<int> pl(p.planesR);
-    pl.insert(pl.end(), p.planesA.begin(), p.planesA.end());
-    e = cudaMemcpyAsync(planes, pl.data(), pl.size() * sizeof(int), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(fact, p.fact.data(), r.nb * sizeof(FactRow), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && order)
-        e = cudaMemcpyAsync(order, p.order.data(), r.nb * sizeof(int), cudaMemcpyHostToDevice, st);
+    // the tables -> device, through pinned memory: the call neither waits for the
+    // stream nor issues a copy per table
+    std::memcpy(h.tab, p.fact.data(), r.nb * sizeof(FactRow));
+    if (order) std::memcpy(h.tab + ft.order, p.order.data(), r.nb * sizeof(int));
+    std::memcpy(h.tab + ft.planes, p.planesR.data(), nR * sizeof(int));
+    std::memcpy(h.tab + ft.planes + nR * sizeof(int), p.planesA.data(), nA * sizeof(int));
+    e = cudaMemcpyAsync(tab, h.tab, ft.bytes, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess && !pipe) e = cudaEventRecord(c.pinned_ev, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(tabs, 0, 3 * (size_t)r.nb * r.nf * sizeof(double2), st);
     if (e != cudaSuccess) return cuda_fail(c, e, "ff: tables");
     c.launches = 0;
@@ -571,6 +572,7 @@ fk_status ff_run(Ctx& c, const FfDev& r, const FfPipe* pipe) {
                            isR ? pipe->epsR : pipe->epsA, isR ? pipe->epsR_d : pipe->epsA_d, q);
         }
         if (e == cudaSuccess) e = cudaStreamWaitEvent(st, c.pipe_ev[PIPE_READY], 0);
+        if (e == cudaSuccess) e = cudaEventRecord(c.pinned_ev, st);  // behind both copies out of the pinned buffer
         if (e != cudaSuccess) return cuda_fail(c, e, "ff: plane copies");
     }
 

@@ -176,10 +176,18 @@ struct FfDev {
 struct FfPipe {
     const double2 *epsR, *epsA;      // host sources [nFreq][ngpown][ncouls]
     double2 *epsR_d, *epsA_d;        // device destinations (r.epsR, r.epsA point at them)
-    const double *ekq_h, *grid_h;    // host copies of ekq and dFreqGrid (the planner reads them)
 };
-size_t ff_workspace(const Ctx& c, const FfDev& r, bool pipelined = false);
-fk_status ff_run(Ctx& c, const FfDev& r, const FfPipe* pipe = nullptr);
+// What an FF request needs on the host: ekq and dFreqGrid, which the planner
+// reads, and room in the context's pinned buffer for the planner's tables
+// (ff_table_bytes), which one copy takes to the device.
+struct FfHost {
+    const double *ekq, *grid;
+    uint8_t* tab;
+};
+size_t ff_table_bytes(const FfDev& r);
+size_t ff_workspace(const Ctx& c, const FfDev& r, const FfHost& h, bool pipelined = false);
+// Records c.pinned_ev behind its copy out of h.tab.
+fk_status ff_run(Ctx& c, const FfDev& r, const FfHost& h, const FfPipe* pipe = nullptr);
 
 // Phase timing helpers (no-ops unless profiling is on).
 void phase_mark(Ctx& c, int i);

@@ -105,3 +105,32 @@ def test_capture_without_room_for_the_images(fk, orc):
     ref = orc.gpp(p)
     check({k: v.cpu().numpy() for k, v in out.items()}, ref)
     c.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_ff_small_arrays_wherever_they_are(ctx, fk, prec):
+    """The small arrays as numpy, as GPU tensors and as GPU tensors off a
+    16-byte boundary (copied), and calls queued behind one another without a
+    wait: the same bits every time."""
+    import torch
+    p = fk.inputs.ff_synthetic(40, 2, 640, 48, 6, 5, seed=8)
+    want = ctx.ff(p, prec, 5)
+    small = ("vcoul", "inv_igp_index", "indinv", "ekq", "dFreqGrid", "dFreqBrd", "pref")
+    d = {k: torch.from_numpy(v).cuda() if isinstance(v, np.ndarray) and k not in small else v for k, v in p.items()}
+    dev, off = dict(d), dict(d)
+    for k in small:
+        dev[k] = torch.from_numpy(p[k]).cuda()
+        if k != "dFreqBrd":  # torch's complex loads want 16 bytes themselves
+            raw = torch.zeros(8 + p[k].nbytes, dtype=torch.uint8, device="cuda")
+            raw[8:] = torch.from_numpy(p[k].view(np.uint8)).cuda()
+            off[k] = raw[8:].view(dev[k].dtype)
+    torch.cuda.synchronize()
+    outs = []
+    for q in (d, dev, off, d, d, d):
+        o = {k: torch.zeros(v.shape, dtype=torch.complex128, device="cuda") for k, v in want.items()}
+        ctx.ff(q, prec, 5, out=o)
+        outs.append(o)
+    ctx.synchronize()
+    for o in outs:
+        for k in FFKEYS:
+            np.testing.assert_array_equal(o[k].cpu().numpy(), want[k])
