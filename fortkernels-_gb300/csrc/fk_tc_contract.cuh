@@ -180,6 +180,20 @@ __device__ __forceinline__ void bimg_store(uint8_t* img_nt, int kstage_total_unu
     img_store<BN, true>(img_nt, n_in_tile, k, re, im);
 }
 
+// A paired B element at its place in a stage (`at`: the stage + tc::sw64_offset).
+template <int BN>
+__device__ __forceinline__ void bimg_store_at(uint8_t* at, float re, float im) {
+    uint16_t h, m, l;
+    split3(re, h, m, l);
+    *(uint16_t*)(at + 0 * BN * 64) = h;
+    *(uint16_t*)(at + 2 * BN * 64) = m;
+    *(uint16_t*)(at + 4 * BN * 64) = l;
+    split3(im, h, m, l);
+    *(uint16_t*)(at + 1 * BN * 64) = h;
+    *(uint16_t*)(at + 3 * BN * 64) = m;
+    *(uint16_t*)(at + 5 * BN * 64) = l;
+}
+
 // One half of a paired B element: the three pieces of its real (part 0) or
 // imaginary (part 1) component, for writers that produce the two halves
 // separately.
