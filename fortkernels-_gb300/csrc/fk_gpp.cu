@@ -1454,9 +1454,10 @@ Plan make_plan(const Ctx& c, const GppDev& r, int ks_override = 0, bool pipeline
         p.tile = ceil_div(ceil_div(r.nc, nch), tcx::BK) * tcx::BK;
         p.nch = ceil_div(r.nc, p.tile);
     } else {
-        // one wave of two resident blocks per SM; each chunk is one partial per flag band
-        // and column for the band reduction
-        const int nch = std::max(1, 2 * c.sms / r.ng);
+        // one wave of resident blocks (two per SM; one beside the digit conversion of
+        // aqsntemp, which takes the rest of the registers); each chunk is one partial per
+        // flag band and column for the band reduction
+        const int nch = std::max(1, (p.tc64 ? 1 : 2) * c.sms / r.ng);
         p.tile = ceil_div(ceil_div(r.nc, nch), PREP_THREADS) * PREP_THREADS;
         p.nch = ceil_div(r.nc, p.tile);
     }
@@ -1553,11 +1554,35 @@ bool take_tc64(Ctx& c, const Plan& p, tc64::Bufs& b) {
     return b.A && b.B && b.ea && b.eb && b.W1;
 }
 template <int EPI>
-void run_tc64(Ctx& c, const ContractArgs& a, const tc64::Plan& z, const tc64::Bufs& b) {
+void run_tc64(Ctx& c, const ContractArgs& a, const tc64::Plan& z, const tc64::Bufs& b, bool have_a = false) {
     tc64::enqueue_weights(c, a, EPI == EPI_GPP ? a.N / 3 : a.N, b, false);
-    tc64::enqueue_a(c, a, z, b);
+    if (!have_a) tc64::enqueue_a(c, a, z, b);
     tc64::enqueue<EPI>(c, a, z, b, tc64::one_plane(z), false);
 }
+
+// A side branch of the context's stream: work queued between fork and join on
+// `side` runs beside the stream's own; join makes the stream wait for it.
+struct Branch {
+    Ctx& c;
+    cudaStream_t main, side = nullptr;
+    explicit Branch(Ctx& c_) : c(c_), main(c_.stream) {
+        if (side_ready(c) != FK_OK) return;  // no side stream (none yet, and the caller captures): the work stays in line
+        if (cudaEventRecord(c.pipe_ev[0], main) == cudaSuccess && cudaStreamWaitEvent(c.copy_stream, c.pipe_ev[0], 0) == cudaSuccess)
+            side = c.copy_stream;
+        else cudaGetLastError();
+    }
+    // queues f's launches (which go to c.stream) on the side stream
+    template <class F>
+    void run(F f) {
+        if (side) c.stream = side;
+        f();
+        c.stream = main;
+        if (side && cudaEventRecord(c.pipe_ev[1], side) != cudaSuccess) cudaStreamSynchronize(side);
+    }
+    void join() {
+        if (side) cudaStreamWaitEvent(main, c.pipe_ev[1], 0);
+    }
+};
 
 template <class K>
 cudaError_t set_smem(K kernel, size_t bytes) {
@@ -1880,12 +1905,26 @@ size_t gpp_workspace(const Ctx& c, const GppDev& r, bool pipelined) {
 
 int gpp_pipe_chunks(const Ctx& c, const GppDev& r) { return make_plan(c, r, 0, true, false, gpp_fsch(r)).pipe_chunks; }
 
-fk_status pipe_begin(Ctx& c) {
-    if (!c.copy_stream && cudaStreamCreateWithFlags(&c.copy_stream, cudaStreamNonBlocking) != cudaSuccess)
-        return cuda_fail(c, cudaGetLastError(), "pipeline: copy stream");
+fk_status side_ready(Ctx& c) {
+    if (!c.copy_stream) {
+        // not created while the caller captures the stream
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(c.stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+            cudaGetLastError();
+            return FK_ENOTSUP;
+        }
+        if (cudaStreamCreateWithFlags(&c.copy_stream, cudaStreamNonBlocking) != cudaSuccess)
+            return cuda_fail(c, cudaGetLastError(), "pipeline: copy stream");
+    }
     for (auto& e : c.pipe_ev)
         if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
             return cuda_fail(c, cudaGetLastError(), "pipeline: events");
+    return FK_OK;
+}
+
+fk_status pipe_begin(Ctx& c) {
+    const fk_status s = side_ready(c);
+    if (s != FK_OK) return s;
     // the destinations are free once the work queued before this call is done
     cudaError_t e = cudaEventRecord(c.pipe_ev[PIPE_FREE], c.stream);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(c.copy_stream, c.pipe_ev[PIPE_FREE], 0);
@@ -2085,6 +2124,9 @@ fk_status gpp_run(Ctx& c, const GppDev& r, const GppPipe* pipe) {
         } else {
             auto k = p.fsch ? (Q == 2 ? prep64_kernel<2, false> : prep64_kernel<0, false>)
                             : (Q == 1 ? prep64_kernel<1, true> : Q == 2 ? prep64_kernel<2, true> : prep64_kernel<0, true>);
+            // blocks of the digit conversion share the SM with it (p.tc64): the same split of
+            // the SM's memory between L1 and shared memory
+            if (p.tc64) cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
             k<<<grid, PREP_THREADS, 0, st>>>(a);
         }
         ++c.launches;
@@ -2131,7 +2173,18 @@ fk_status gpp_run(Ctx& c, const GppDev& r, const GppPipe* pipe) {
             }
         }
     }
-    for (int pass = 0; pass < p.passes && !pipe; ++pass) launch_prep(prep_args(pass), dim3(p.nch, r.ng));
+    // FP64: aqsntemp's digits (bound by memory) beside the prep (by the FP64 pipe).
+    // 512 x 32768 x 20: the prep takes 103 us at one block per SM instead of 98 at two, the
+    // digits hide behind it, the call goes from 435 to 406 us.
+    if (p.tc64) {
+        Branch br(c);
+        ContractArgs a{};
+        a.A = r.aqsn; a.lda = r.nc; a.m0 = p.m0; a.M = M; a.K = r.nc;
+        for (int pass = 0; pass < p.passes; ++pass) launch_prep(prep_args(pass), dim3(p.nch, r.ng));
+        br.run([&] { tc64::enqueue_a(c, a, p.z, zb); });
+        br.join();
+    }
+    for (int pass = 0; pass < p.passes && !pipe && !p.tc64; ++pass) launch_prep(prep_args(pass), dim3(p.nch, r.ng));
     phase_mark(c, 2);
     if (M > 0 && !pipe) {
         ContractArgs a{};
@@ -2182,7 +2235,7 @@ fk_status gpp_run(Ctx& c, const GppDev& r, const GppPipe* pipe) {
                 kernel_end(c);
             }
         } else if (p.tc64) {
-            run_tc64<EPI_GPP>(c, a, p.z, zb);
+            run_tc64<EPI_GPP>(c, a, p.z, zb, true);
             --c.launches;
         } else {
             auto k = d64::contract_kernel<EPI_GPP>;

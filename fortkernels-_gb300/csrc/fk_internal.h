@@ -101,6 +101,8 @@ size_t gpp_workspace(const Ctx& c, const GppDev& r, bool pipelined = false);
 // eps, wtilde and the small inputs first and records pipe_ev[PIPE_READY].
 constexpr int PIPE_FREE = 8, PIPE_READY = 9;
 int gpp_pipe_chunks(const Ctx& c, const GppDev& r);
+// The context's copy stream and events exist (created on first use, not during a capture).
+fk_status side_ready(Ctx& c);
 fk_status pipe_begin(Ctx& c);
 fk_status gpp_pipe_copy(Ctx& c, const GppDev& r, const GppPipe* pipe, int q0, int q1);
 fk_status gpp_run(Ctx& c, const GppDev& r, const GppPipe* pipe = nullptr);

@@ -702,6 +702,8 @@ inline void launch_split(Ctx& c, const SplitArgs& s, int batches) {
     if (nk <= SMEM_K) {
         auto k = split_kernel<BSIDE, true>;
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_K * 16);
+        // the SM's memory split as the GPP prep asks for it, so that blocks of both share an SM
+        cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         k<<<grid, threads, nk * 16, c.stream>>>(s);
     } else {
         split_kernel<BSIDE, false><<<grid, threads, 0, c.stream>>>(s);
