@@ -41,12 +41,14 @@ FK_DEV void cfmaf(float2& acc, float2 a, float2 b) {
 // flush to signed zero.  Inputs must satisfy |x| < 2^127 (the kernels' data
 // are O(1); larger values are rejected by the host-side checks where the
 // mixed path is used on user data).
-FK_DEV float f64_to_f32_bits(double d) {
+constexpr unsigned F32_TINY = 897u << 20;  // high word of the smallest magnitude that is not flushed
+// (tiny: another such bound; 0xFFFFFFFF makes every value a zero)
+FK_DEV float f64_to_f32_bits(double d, unsigned tiny = F32_TINY) {
     unsigned long long u = (unsigned long long)__double_as_longlong(d) + 0x10000000ull;
     unsigned hi = (unsigned)(u >> 32), lo = (unsigned)u;
     unsigned sign = hi & 0x80000000u;
     unsigned mag = hi & 0x7FFFFFFFu;
-    unsigned f = mag < (897u << 20) ? 0u : __funnelshift_l(lo, mag - (896u << 20), 3);
+    unsigned f = mag < tiny ? 0u : __funnelshift_l(lo, mag - (896u << 20), 3);
     return __uint_as_float(f | sign);
 }
 FK_DEV float2 c64_to_f32(double2 v) { return make_float2(f64_to_f32_bits(v.x), f64_to_f32_bits(v.y)); }

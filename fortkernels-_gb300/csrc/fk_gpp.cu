@@ -1364,8 +1364,8 @@ __global__ void __launch_bounds__(ROWS_THREADS) rows_kernel(RowsArgs ra) {
 // pipelined host path (one launch per row block), the half sum, the served
 // steps and the real-valued sum, which keep the single-CTA kernel.
 // A request with one n-tile of columns (ngpown <= 21) streams aqsntemp once at
-// the HBM rate, where the single-CTA kernel is the faster one (measured: 73 vs
-// 79 us at 512 x 2 x 32768 x 20); with more n-tiles the tensor work dominates.
+// the HBM rate, where the single-CTA kernel is the faster one (measured: the call takes
+// 96 us against 103 at 512 x 2 x 32768 x 20); with more n-tiles the tensor work dominates.
 inline bool gpp_pair(const GppDev& r, bool pipelined) {
     return r.prec == FK_MIXED && !pipelined && !(r.flags & FK_GPP_HALF_SUM) && r.ng > 21;
 }

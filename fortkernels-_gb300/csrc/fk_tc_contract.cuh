@@ -49,14 +49,17 @@ constexpr int BM = 128;
 constexpr int BK = 32;            // complex k-values per stage (64 B of bf16 per row)
 constexpr int NSPLIT = 3;         // bf16 pieces per real value
 constexpr int NSUB = 2 * NSPLIT;  // sub-tiles per operand: re h/m/l, im h/m/l
-constexpr int THREADS = 448;     // GPP: MMA, producer, 8 converter warps, 4 epilogue warps
+constexpr int THREADS = 704;     // GPP: MMA, producer, 8 converter warps, 4 epilogue warps
 constexpr int THREADS_FF = 608;  // FF: MMA, producer, 16 epilogue warps, the -B_im warp
 // FF (A operand pre-split, no converter work): the 16 warps 2..17 all drain
 // TMEM, four per lane quarter, each over one 16-column group with its own
 // weights in registers and its own partial-sum slot; GPP: warps 4..7, one per
 // quarter, all columns.
 constexpr int FF_EPI_WARPS = 4;
-constexpr int NCONV = 8;          // converter warps
+constexpr int NCONV = 16;          // converter warps
+constexpr int QK = 8;             // GPP: complex k-values per quarter of the FP64 staging ring
+constexpr int FQ = 5;             // its quarters
+constexpr uint32_t FQ_BYTES = BM * QK * 16;
 // Default bound of every wait on another role of the CTA (SM clock cycles,
 // ~2 s at 2 GHz); a launch may pass a different one (TcArgs::wait_limit).
 constexpr long long WAIT_LIMIT = 4000000000LL;
@@ -69,11 +72,12 @@ template <int BN, bool WSMEM = false, bool PAIR = false, bool APRE = WSMEM>
 struct Cfg {
     static_assert(BN == 64, "the accumulator buffers fill the 512 TMEM columns at BN = 64");
     // Operand stages: FF three (its epilogue keeps the per-unit weights in
-    // registers, so shared memory holds operands only), GPP two.  GPP: a 64 KB staging buffer receives
-    // FP64 A rows by TMA in two halves of BK/2 k-values, so that one half is in
-    // flight while the converters read the other.  (Two full stagings do not fit
-    // beside two operand stages; one operand stage with two stagings measured
-    // slower: the converters then wait for each stage's MMAs.)
+    // registers, so shared memory holds operands only), GPP two.  GPP: FP64 A rows arrive by
+    // TMA in a ring of 16 KB quarters (QK = 8 k-values of the tile's rows, one swizzled
+    // 128-byte line per row); a quarter is refilled as soon as the converters have read it.
+    // Five quarters are what fits beside two operand stages (four in flight while the
+    // fifth is read).  (One operand stage with more staging measured slower: the converters
+    // then wait for each stage's MMAs.)
     static constexpr int CHUNK_STAGES = 1;  // k-values per TMEM accumulation = 32
     // FF operands are FP16 hi/lo pieces (two per real value; every row scaled by
     // a power of two that brings its largest magnitude just below 2^15, three
@@ -113,12 +117,12 @@ struct Cfg {
     static constexpr uint32_t ACC_COLS = SL ? 2 * BN : 4 * BN;
     static constexpr uint32_t TMEM_COLS = NBUF * ACC_COLS;
     static constexpr uint32_t W_BYTES = 0u;
-    static constexpr uint32_t F64_BYTES = APRE ? 0u : (uint32_t)(BM * BK * sizeof(double2));
+    static constexpr uint32_t F64_BYTES = APRE ? 0u : FQ * FQ_BYTES;
     static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + W_BYTES + F64_BYTES + 1024 + 512;
 };
 
 struct TcArgs {
-    CUtensorMap amap;     // GPP: A (FP64 complex rows) as a 2-D FP64 tensor, box 32 x BM (half a stage), zero fill
+    CUtensorMap amap;     // GPP: A (FP64 complex rows) as a 2-D FP64 tensor, box 16 x BM (a quarter of a stage), 128-byte swizzle, zero fill
     ContractArgs c;       // shapes, partial buffer (same meaning as fk_gemm.cuh)
     const uint8_t* Bimg;  // pre-split B tiles: [plane][nt][kstage][NSUB][BN rows][64 B]
     const uint8_t* Aimg;  // pre-split A tiles [mt][kstage][ASUB][BM rows][64 B] (APRE kernels only)
@@ -149,6 +153,19 @@ __device__ __forceinline__ void split3(float f, uint16_t& h, uint16_t& m, uint16
     h = (uint16_t)(hb >> 16);
     m = (uint16_t)(mb >> 16);
     l = (uint16_t)(__float_as_uint(r2) >> 16);  // r2 has at most 8 significant bits: exact
+}
+
+// The pieces of two neighbouring k-values, as words of one row of three sub-tiles of
+// ROWS rows (at: the pair's place in the first).
+template <int ROWS>
+__device__ __forceinline__ void split3_store(uint8_t* at, float f0, float f1) {
+    const uint32_t a0 = __float_as_uint(f0), a1 = __float_as_uint(f1);
+    const float r0 = f0 - __uint_as_float(a0 & 0xFFFF0000u), r1 = f1 - __uint_as_float(a1 & 0xFFFF0000u);
+    const uint32_t b0 = __float_as_uint(r0), b1 = __float_as_uint(r1);
+    const float q0 = r0 - __uint_as_float(b0 & 0xFFFF0000u), q1 = r1 - __uint_as_float(b1 & 0xFFFF0000u);
+    *(uint32_t*)(at) = __byte_perm(a0, a1, 0x7632);
+    *(uint32_t*)(at + ROWS * 64) = __byte_perm(b0, b1, 0x7632);
+    *(uint32_t*)(at + 2 * ROWS * 64) = __byte_perm(__float_as_uint(q0), __float_as_uint(q1), 0x7632);
 }
 
 // Image element writer shared by the prep/conversion kernels: complex value
@@ -292,7 +309,7 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // 1024-aligned operand area
     uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    double2* sF = (double2*)(base + C::STAGES * C::STAGE_BYTES + C::W_BYTES);  // GPP: FP64 rows [BM][BK]
+    uint8_t* sF = base + C::STAGES * C::STAGE_BYTES + C::W_BYTES;  // GPP: FP64 staging ring [FQ][BM rows][128 B]
     uint64_t* bars = (uint64_t*)(base + C::STAGES * C::STAGE_BYTES + C::W_BYTES + C::F64_BYTES);
     uint64_t* fullA = bars;
     uint64_t* fullB = bars + C::STAGES;
@@ -300,11 +317,11 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
     uint64_t* accFull = bars + 3 * C::STAGES;  // [NBUF]
     uint64_t* accEmpty = accFull + C::NBUF;    // [NBUF]
     uint64_t* done = accEmpty + C::NBUF;
-    uint64_t* fFull = done + 1;    // [2] GPP: FP64 staging half filled (tx bytes)
-    uint64_t* fEmpty = done + 3;   // [2] GPP: FP64 staging half read by all converter warps
-    uint64_t* peerFull = done + 5; // [STAGES] PAIR, even CTA: the odd CTA's half of the stage has landed
-    uint64_t* negFull = done + 5 + C::STAGES;  // [STAGES] FF: the stage's -B_im is written
-    uint32_t* tslot = (uint32_t*)(done + 5 + 2 * C::STAGES);
+    uint64_t* fFull = done + 1;         // [FQ] GPP: FP64 staging quarter filled (tx bytes)
+    uint64_t* fEmpty = fFull + FQ;      // [FQ] GPP: FP64 staging quarter read by all converter warps
+    uint64_t* peerFull = fEmpty + FQ;   // [STAGES] PAIR, even CTA: the odd CTA's half of the stage has landed
+    uint64_t* negFull = peerFull + C::STAGES;  // [STAGES] FF: the stage's -B_im is written
+    uint32_t* tslot = (uint32_t*)(negFull + C::STAGES);
     __shared__ int s_abort_flag;
     volatile int& s_abort = s_abort_flag;
 
@@ -330,7 +347,7 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
             tc::mbar_init(&negFull[s], 1);
         }
         tc::mbar_init(done, 1);
-        for (int h = 0; h < 2; ++h) {
+        for (int h = 0; h < FQ; ++h) {
             tc::mbar_init(&fFull[h], 1);
             tc::mbar_init(&fEmpty[h], NCONV);
         }
@@ -514,13 +531,13 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
         // ------------------------------------------------ bulk copies
         // lane 0: pre-split B (and, for a pre-split A, A) tiles into the operand stage;
         // all lanes (GPP): the next stage's FP64 A rows into the staging buffer.
-        // g counts stage uses, gf the stage uses staged in FP64 (the staging
-        // halves' barriers complete once per such use)
-        int g = 0, gf = 0;
+        // g counts stage uses, fq the quarters staged in FP64 (quarter fq goes to
+        // ring slot fq % FQ)
+        int g = 0, fq = 0;
         bool ok = true;
-        // the last copy issued into each stage / staging half (-1: none), so
-        // that the CTA can wait for every copy it started before it exits
-        int last_st[C::STAGES], last_f[2] = {-1, -1};
+        // the last copy issued into each stage (-1: none; the ring's follow from
+        // fq), so that the CTA can wait for every copy it started before it exits
+        int last_st[C::STAGES];
 #pragma unroll
         for (int s = 0; s < C::STAGES; ++s) last_st[s] = -1;
         for (int u = pid; u < src.units() && ok; u += npairs) {
@@ -542,23 +559,23 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
                 const int s = g % C::STAGES;
                 const long kst = (long)(k0 / BK) + st;
                 if (!ua) {
-                    // FP64 rows in two halves of BK/2 k-values, each into its own half of the
-                    // staging buffer as soon as the converters have read that half of the last stage
-                    for (int h = 0; h < 2 && ok; ++h) {
-                        if (!tc::warp_all(tc::mbar_wait(&fEmpty[h], (gf & 1) ^ 1, wait_limit) && !s_abort)) {
+                    // FP64 rows in quarters of QK k-values, each into the ring as soon as the
+                    // converters have read the slot's last one
+                    for (int h = 0; h < BK / QK; ++h) {
+                        const int sl = fq % FQ;
+                        if (!tc::warp_all(tc::mbar_wait(&fEmpty[sl], ((fq / FQ) & 1) ^ 1, wait_limit) && !s_abort)) {
                             fail(64);
                             ok = false;
                             break;
                         }
                         if (lane == 0) {
-                            tc::mbar_arrive_expect_tx(&fFull[h], C::F64_BYTES / 2);
-                            tc::tma_load_2d(sF + h * (BM * BK / 2), &t.amap, 2 * (k0 + st * BK + h * (BK / 2)),
-                                            a.m0 + mt * BM, &fFull[h]);
-                            last_f[h] = gf;
+                            tc::mbar_arrive_expect_tx(&fFull[sl], FQ_BYTES);
+                            tc::tma_load_2d(sF + sl * FQ_BYTES, &t.amap, 2 * (k0 + st * BK + h * QK), a.m0 + mt * BM,
+                                            &fFull[sl]);
                         }
+                        ++fq;
                     }
                     if (!ok) break;
-                    ++gf;
                 }
                 if (lane == 0) {
                     if (!tc::mbar_wait(&empty[s], ((g / C::STAGES) & 1) ^ 1, wait_limit) || s_abort) {
@@ -619,8 +636,8 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
                     drained = tc::mbar_wait(&fullB[s], par, DRAIN_LIMIT) && drained;  // a pre-split A image too
                 }
             if (!APRE)
-                for (int h = 0; h < 2; ++h)
-                    if (last_f[h] >= 0) drained = tc::mbar_wait(&fFull[h], (uint32_t)last_f[h] & 1u, DRAIN_LIMIT) && drained;
+                for (int q = max(0, fq - FQ); q < fq; ++q)
+                    drained = tc::mbar_wait(&fFull[q % FQ], (uint32_t)(q / FQ) & 1u, DRAIN_LIMIT) && drained;
             if (!drained) fail(128);
         }
     } else if (C::IMGN && warp == THREADS_FF / 32 - 1) {
@@ -792,17 +809,17 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
                     }
                 }
 #pragma unroll
-                for (int c0 = 0; c0 < BN && EPI == EPI_GPP; c0 += 16) {
+                for (int c0 = 0; c0 < BN && EPI == EPI_GPP; c0 += 8) {
                     // X = [A_re B_re | A_re B_im], Y = [A_im B_re | A_im B_im]
-                    float xr[16], xi[16], yr[16], yi[16];
-                    tc::tmem_ld16(tl + c0, xr);
-                    tc::tmem_ld16(tl + BN + c0, xi);
-                    tc::tmem_ld16(tl + 2 * BN + c0, yr);
-                    tc::tmem_ld16(tl + 3 * BN + c0, yi);
+                    float xr[8], xi[8], yr[8], yi[8];
+                    tc::tmem_ld8(tl + c0, xr);
+                    tc::tmem_ld8(tl + BN + c0, xi);
+                    tc::tmem_ld8(tl + 2 * BN + c0, yr);
+                    tc::tmem_ld8(tl + 3 * BN + c0, yi);
                     tc::tmem_ld_wait();
-                    if (c0 + 16 >= BN) release();
+                    if (c0 + 8 >= BN) release();
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
+                    for (int j = 0; j < 8; ++j) {
                         const int c = c0 + j;
                         const float2 sv = make_float2(xr[j] - yi[j], xi[j] + yr[j]);
                         // tile column c = 3*(igp offset) + iw; column 63 is padding
@@ -827,16 +844,23 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
         }
     } else {
         // ----------------------------------------------------- converters
-        // warp cw converts rows cw*16 .. cw*16+15 of each stage.  The staging
-        // buffer holds the stage in two halves of BK/2 k-values, each filled by
-        // its own TMA box: read a half (lane = (row pair, k), one conflict-free
-        // 512-byte read per instruction), release it so that the next stage's
-        // half is copied while the other half is read, then split everything
-        // into BF16 pieces and store it into the operand stage.
+        // warp cw converts rows cw*16 .. cw*16+15 of each stage, quarter by quarter:
+        // lane = (row lane>>2 of eight, k-pair lane&3).  The quarter's 128-byte
+        // lines are swizzled, so a pair's two 16-byte reads and the two-element
+        // stores of its pieces touch every bank once.  The next quarter is read (and
+        // its slot released) before the current one is split, within a unit.
+        // With the stage's two halves read first and split together by element (2-byte
+        // stores) a stage took 4400 cycles, now 3950: 2300 of splitting, 1300 of waiting
+        // for HBM (the copies alone: 40 us for 268 MB).  512 x 32768 x 20: 65 -> 57 us.
+        // 16 converter warps (80 registers) took 4 us longer, CTA pairs 6 us; asking L2
+        // for the rows 8 to 28 quarters ahead 4 to 27 us: the copy unit's time per row
+        // is what the copies cost.
         if (!APRE) {
             const int cw = warp < 4 ? warp - 2 : warp - 6;  // 0..7
-            constexpr int RPW = BM / NCONV;                  // rows per converter warp
-            int g = 0, gf = 0;  // stage uses, FP64-staged stage uses (as the copy warp counts them)
+            constexpr int RPL = BM / NCONV / 8;             // rows per lane
+            constexpr int NQ = BK / QK;
+            const int kp = lane & 3, r8 = lane >> 2;
+            int g = 0, fq = 0;  // stage uses, quarters read (as the copy warp counts them)
             bool ok = true;
             for (int u = pid; u < src.units() && ok; u += npairs) {
                 int lu;
@@ -846,10 +870,9 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
                 unit_coords(t, lu, mt, nt, ks, batch);
                 krange(t, ks, k0, k1);
                 const int nst = k1 > k0 ? (k1 - k0 + BK - 1) / BK : 0;
-                const bool ua = Src::kTable && t.Aimg != nullptr;  // the request's A is pre-split
-                for (int st = 0; st < nst; ++st, ++g) {
-                    const int s = g % C::STAGES;
-                    if (ua) {
+                if (Src::kTable && t.Aimg != nullptr) {  // the request's A is pre-split
+                    for (int st = 0; st < nst; ++st, ++g) {
+                        const int s = g % C::STAGES;
                         // the stage's A arrives by bulk copy: only complete this use's phase of
                         // fullA (no data), after the stage is free, so that every use of a
                         // stage completes one phase whichever way its A arrives
@@ -860,60 +883,61 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
                         }
                         __syncwarp();
                         if (lane == 0) tc::mbar_arrive(&fullA[s]);
-                        continue;
                     }
-                    if (!tc::warp_all(tc::mbar_wait(&fFull[0], gf & 1, wait_limit) && !s_abort)) {
-                        fail(32);
-                        ok = false;
-                        break;
-                    }
-                    // lane -> (row pair offset lane>>4, k within the half lane&15)
-                    double2 v[RPW];
-                    const int kk = lane & 15, rr = lane >> 4;
+                    continue;
+                }
+                const uint32_t rowoff = (uint32_t)(cw * (BM / NCONV) + r8);  // the lane's first row, then + 8
+                // rows past the tile's last and k-values past the slice's end become zeros: the
+                // magnitude below which a value rounds to zero is raised above every magnitude
+                unsigned rowthr[RPL];
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        if (h == 1 && !tc::warp_all(tc::mbar_wait(&fFull[1], gf & 1, wait_limit) && !s_abort)) {
-                            fail(32);
-                            ok = false;
-                            break;
-                        }
-                        const double2* sh = sF + h * (BM * BK / 2);
-                        const int kh = k0 + st * BK + h * (BK / 2) + kk;
+                for (int i = 0; i < RPL; ++i) rowthr[i] = mt * BM + (int)rowoff + 8 * i < a.M ? F32_TINY : 0xFFFFFFFFu;
+                double2 v[2][RPL][2];
+                auto read = [&](int par) {
+                    const int sl = fq % FQ;
+                    if (!tc::warp_all(tc::mbar_wait(&fFull[sl], (fq / FQ) & 1, wait_limit) && !s_abort)) return false;
+                    const uint8_t* sh = sF + sl * FQ_BYTES + rowoff * 128u;
 #pragma unroll
-                        for (int i = 0; i < RPW / 2; ++i) {
-                            const int r = cw * RPW + 2 * i + rr;
-                            v[h * (RPW / 2) + i] = (mt * BM + r < a.M && kh < k1) ? sh[r * (BK / 2) + kk] : make_double2(0.0, 0.0);
+                    for (int i = 0; i < RPL; ++i)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e)
+                            v[par][i][e] = *(const double2*)(sh + i * 1024 + ((uint32_t)((2 * kp + e) ^ r8) << 4));
+                    __syncwarp();
+                    if (lane == 0) tc::mbar_arrive(&fEmpty[sl]);
+                    ++fq;
+                    return true;
+                };
+                if (nst > 0) ok = read(0);
+                for (int st = 0; st < nst && ok; ++st, ++g) {
+                    const int s = g % C::STAGES;
+                    uint8_t* sa = base + s * C::STAGE_BYTES + rowoff * 64u + kp * 4u;
+#pragma unroll
+                    for (int h = 0; h < NQ; ++h) {
+                        if (h + 1 < NQ || st + 1 < nst) {
+                            ok = read((h + 1) & 1);
+                            if (!ok) break;
                         }
-                        __syncwarp();
-                        if (lane == 0) tc::mbar_arrive(&fEmpty[h]);
+                        if (h == 0) {
+                            ok = tc::warp_all(tc::mbar_wait(&empty[s], ((g / C::STAGES) & 1) ^ 1, wait_limit) && !s_abort);
+                            if (!ok) break;
+                        }
+                        const int left = k1 - (k0 + st * BK + h * QK + 2 * kp);  // k-values of the pair inside the slice
+#pragma unroll
+                        for (int i = 0; i < RPL; ++i) {
+                            const unsigned t0 = left > 0 ? rowthr[i] : 0xFFFFFFFFu, t1 = left > 1 ? rowthr[i] : 0xFFFFFFFFu;
+                            const double2 *p = v[h & 1][i];
+                            // swizzled position: the quarter's 16-byte chunk is h
+                            uint8_t* at = sa + i * 512 + ((uint32_t)(h ^ ((r8 >> 1) & 3)) << 4);
+                            split3_store<BM>(at, f64_to_f32_bits(p[0].x, t0), f64_to_f32_bits(p[1].x, t1));
+                            split3_store<BM>(at + 3 * BM * 64, f64_to_f32_bits(p[0].y, t0), f64_to_f32_bits(p[1].y, t1));
+                        }
                     }
                     if (!ok) break;
-                    if (!tc::warp_all(tc::mbar_wait(&empty[s], ((g / C::STAGES) & 1) ^ 1, wait_limit) && !s_abort)) {
-                        fail(32);
-                        ok = false;
-                        break;
-                    }
-                    uint8_t* sa = base + s * C::STAGE_BYTES;
-#pragma unroll
-                    for (int i = 0; i < RPW; ++i) {
-                        // v[i]: half i / (RPW/2), row pair i % (RPW/2)
-                        const uint32_t off =
-                            tc::sw64_offset(cw * RPW + 2 * (i % (RPW / 2)) + rr, (i / (RPW / 2)) * (BK / 2) + kk);
-                        uint16_t hh, mm, ll;
-                        split3(f64_to_f32_bits(v[i].x), hh, mm, ll);
-                        *(uint16_t*)(sa + 0 * BM * 64 + off) = hh;
-                        *(uint16_t*)(sa + 1 * BM * 64 + off) = mm;
-                        *(uint16_t*)(sa + 2 * BM * 64 + off) = ll;
-                        split3(f64_to_f32_bits(v[i].y), hh, mm, ll);
-                        *(uint16_t*)(sa + 3 * BM * 64 + off) = hh;
-                        *(uint16_t*)(sa + 4 * BM * 64 + off) = mm;
-                        *(uint16_t*)(sa + 5 * BM * 64 + off) = ll;
-                    }
                     tc::fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) tc::mbar_arrive(&fullA[s]);
-                    ++gf;
                 }
+                if (!ok) fail(32);
             }
         }
     }
@@ -1395,10 +1419,10 @@ inline cudaError_t encode_rows_map(CUtensorMap* map, const double2* A, long lda,
     if (!fn) return cudaErrorNotSupported;
     const cuuint64_t dims[2] = {(cuuint64_t)2 * K, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)lda * sizeof(double2)};
-    const cuuint32_t box[2] = {BK, BM};  // half a stage: BK/2 complex values of BM rows
+    const cuuint32_t box[2] = {2 * QK, BM};  // a quarter of a stage: QK complex values of BM rows
     const cuuint32_t estr[2] = {1, 1};
     const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, (void*)A, dims, strides, box, estr,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
