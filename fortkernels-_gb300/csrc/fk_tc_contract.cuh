@@ -49,14 +49,14 @@ constexpr int BM = 128;
 constexpr int BK = 32;            // complex k-values per stage (64 B of bf16 per row)
 constexpr int NSPLIT = 3;         // bf16 pieces per real value
 constexpr int NSUB = 2 * NSPLIT;  // sub-tiles per operand: re h/m/l, im h/m/l
-constexpr int THREADS = 704;     // GPP: MMA, producer, 8 converter warps, 4 epilogue warps
+constexpr int THREADS = 448;     // GPP: MMA, producer, 8 converter warps, 4 epilogue warps
 constexpr int THREADS_FF = 608;  // FF: MMA, producer, 16 epilogue warps, the -B_im warp
 // FF (A operand pre-split, no converter work): the 16 warps 2..17 all drain
 // TMEM, four per lane quarter, each over one 16-column group with its own
 // weights in registers and its own partial-sum slot; GPP: warps 4..7, one per
 // quarter, all columns.
 constexpr int FF_EPI_WARPS = 4;
-constexpr int NCONV = 16;          // converter warps
+constexpr int NCONV = 8;          // converter warps
 constexpr int QK = 8;             // GPP: complex k-values per quarter of the FP64 staging ring
 constexpr int FQ = 5;             // its quarters
 constexpr uint32_t FQ_BYTES = BM * QK * 16;
@@ -809,17 +809,17 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
                     }
                 }
 #pragma unroll
-                for (int c0 = 0; c0 < BN && EPI == EPI_GPP; c0 += 8) {
+                for (int c0 = 0; c0 < BN && EPI == EPI_GPP; c0 += 16) {
                     // X = [A_re B_re | A_re B_im], Y = [A_im B_re | A_im B_im]
-                    float xr[8], xi[8], yr[8], yi[8];
-                    tc::tmem_ld8(tl + c0, xr);
-                    tc::tmem_ld8(tl + BN + c0, xi);
-                    tc::tmem_ld8(tl + 2 * BN + c0, yr);
-                    tc::tmem_ld8(tl + 3 * BN + c0, yi);
+                    float xr[16], xi[16], yr[16], yi[16];
+                    tc::tmem_ld16(tl + c0, xr);
+                    tc::tmem_ld16(tl + BN + c0, xi);
+                    tc::tmem_ld16(tl + 2 * BN + c0, yr);
+                    tc::tmem_ld16(tl + 3 * BN + c0, yi);
                     tc::tmem_ld_wait();
-                    if (c0 + 8 >= BN) release();
+                    if (c0 + 16 >= BN) release();
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
+                    for (int j = 0; j < 16; ++j) {
                         const int c = c0 + j;
                         const float2 sv = make_float2(xr[j] - yi[j], xi[j] + yr[j]);
                         // tile column c = 3*(igp offset) + iw; column 63 is padding
