@@ -1099,13 +1099,14 @@ FK_DEV double2 warp_tree(double2 v) {
 
 // Per-band sums into rows[n1][8] = {sch iw0..2, ssx iw0..2, stat, 0}.  Bands
 // n1 >= nvband add the contraction's k-slice partials P[slot][m][3]
-// (rows_band_warp, below).  Occupied bands n1 < nvband, one warp per (band,
-// component c of 7; rows_warp): for c < 6, over columns my_igp, the chunk
+// (rows_band_warp, below).  Occupied bands n1 < nvband, one block per (band,
+// component c of 7; rows_flag_block): for c < 6, over columns my_igp, the chunk
 // partials of the prep F[ch][n1][my_igp][6] times the reference's weight
 // (sch: 0.5*vcoul*conj(aqsm), BGW-Kernels/gppKer.cpp:346,421; ssx:
-// occ*vcoul*conj(aqsm), :419), the lanes taking columns and a fixed shuffle
-// tree adding them (deterministic); c == 6: the static-remainder partials
+// occ*vcoul*conj(aqsm), :419), the threads taking (chunk, column) items and a
+// fixed tree adding them (deterministic); c == 6: the static-remainder partials
 // S[slot][n1].
+constexpr int ROWS_THREADS = 128;
 struct RowsArgs {
     int nb, nv, ng, nslots;
     const double2* P;
@@ -1132,7 +1133,11 @@ struct RowsArgs {
     bool fsch = false;    // occupied bands' sch components from P (rows from m0 = 0), not from F
 };
 
-FK_DEV void rows_warp(const RowsArgs& ra, int n1, int c, int lane) {
+// Bound: the round trips to memory of a thread's items, one after another.  Over one
+// warp, column by column, 1638 columns took 51 of them and the kernel 119 us at
+// 512 x 2 x 32768 x 1638 (now 21 us); eight items are in flight at a time.
+FK_DEV void rows_flag_block(const RowsArgs& ra, int n1, int c, int tid) {
+    constexpr int T = ROWS_THREADS;
     const int nb = ra.nb, nv = ra.nv, ng = ra.ng, nslots_s = ra.nslots_s, nch = ra.nch;
     const double2 *S = ra.S, *F = ra.F, *aqsm = ra.aqsm;
     const long ldm = ra.ldm;
@@ -1141,17 +1146,17 @@ FK_DEV void rows_warp(const RowsArgs& ra, int n1, int c, int lane) {
     double2* rows = ra.rows;
     double2 v = make_double2(0.0, 0.0);
     if (c == 6) {
-        if (S && lane < nslots_s) v = ordered_sum(S + (long)lane * nb + n1, 32L * nb, (nslots_s - lane + 31) / 32);
+        if (S && tid < nslots_s) v = ordered_sum(S + (long)tid * nb + n1, (long)T * nb, (nslots_s - tid + T - 1) / T);
     } else if (ra.fsch && c < 3) {
         // the band's sch component from the contraction: its k-slice partials in slot order
         const int m0 = ra.m0 < 0 ? nv : ra.m0;
         const long M = nb - m0, m = n1 - m0;
-        if (lane < ra.nslots) v = ordered_sum(ra.P + ((long)lane * M + m) * 3 + c, 32L * M * 3, (ra.nslots - lane + 31) / 32);
+        if (tid < ra.nslots) v = ordered_sum(ra.P + ((long)tid * M + m) * 3 + c, (long)T * M * 3, (ra.nslots - tid + T - 1) / T);
     } else if (ra.P2) {
         // half sum, occupied band: weight * (cm S1 + conj(cm S2)) per column
         const int kind = c / 3, r = ((c % 3) * 2 + kind) * 2;
         const double occ = 1.0;
-        for (int h = lane; h < ng; h += 32) {
+        for (int h = tid; h < ng; h += T) {
             const int g = igp[h];
             if (g < 0) continue;
             const double2 s1 = ordered_sum(F + ((long)n1 * ng + h) * 12 + r, (long)nv * ng * 12, nch);
@@ -1160,17 +1165,26 @@ FK_DEV void rows_warp(const RowsArgs& ra, int n1, int c, int lane) {
             v = cadd(v, cscale(cadd(cmul(cm, s1), cconj(cmul(cm, s2))), kind ? occ * vcoul[g] : 0.5 * vcoul[g]));
         }
     } else if (ra.wf) {
-        // weights from the prep; the chunk sums' loads all in flight at once
+        // weights from the prep; item i = (chunk i / ng, column i % ng)
+        constexpr int U = 8;
         const int kind = c / 3, r = (c % 3) * 2 + kind;  // kind 0: sch, 1: ssx
-        for (int h = lane; h < ng; h += 32) {
-            const double2 w = ra.wf[((long)n1 * ng + h) * 2 + kind];
-            const double2 sum = ordered_sum16(F + ((long)n1 * ng + h) * 6 + r, (long)nv * ng * 6, nch);
-            v = cadd(v, cmul(w, sum));
+        const long items = (long)nch * ng;
+        for (long i0 = tid; i0 < items; i0 += U * T) {
+            double2 w[U], x[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {  // clamped indices: every load reads a valid address
+                const long i = min(i0 + u * T, items - 1), k = i / ng, h = i - k * ng;
+                w[u] = ra.wf[((long)n1 * ng + h) * 2 + kind];
+                x[u] = F[((k * nv + n1) * ng + h) * 6 + r];
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (i0 + u * T < items) v = cadd(v, cmul(w[u], x[u]));
         }
     } else {
         const int kind = c / 3, r = (c % 3) * 2 + kind;  // kind 0: sch, 1: ssx
         const double occ = 1.0;
-        for (int h = lane; h < ng; h += 32) {
+        for (int h = tid; h < ng; h += T) {
             const int g = igp[h];
             if (g < 0) continue;
             const double2 sum = ordered_sum(F + ((long)n1 * ng + h) * 6 + r, (long)nv * ng * 6, nch);
@@ -1179,10 +1193,19 @@ FK_DEV void rows_warp(const RowsArgs& ra, int n1, int c, int lane) {
         }
     }
     // a component with no terms (stat without S) skips the tree
-    const bool empty = c == 6 && !S;
-    if (!empty) v = warp_tree(v);
-    if (lane == 0) rows[(long)n1 * 8 + c] = v;
-    if (lane == 0 && c == 2 && ra.out) ra.out[7 + n1] = v;  // acht_n1_loc
+    __shared__ double2 part[T / 32];
+    if (c != 6 || S) {
+        v = warp_tree(v);
+        if ((tid & 31) == 0) part[tid >> 5] = v;
+        __syncthreads();
+        if (tid == 0)
+            for (int w = 1; w < T / 32; ++w) v = cadd(v, part[w]);
+    }
+    if (tid == 0) {
+        rows[(long)n1 * 8 + c] = v;
+        if (c == 2 && ra.out) ra.out[7 + n1] = v;  // acht_n1_loc
+    }
+    __syncthreads();  // part is reused by the block's next task
 }
 
 // Bands n1 >= nvband, one warp per band.  GB300's FP64 pipe retires one warp
@@ -1195,8 +1218,7 @@ FK_DEV void rows_warp(const RowsArgs& ra, int n1, int c, int lane) {
 // sub-partition); warp 0 then writes the block's partial totals (eight
 // parts: components 0..2 and 6), so the totals read one value per four bands.
 // The rows buffer is [nb][8] band rows, then [band blocks][8] partials.
-constexpr int ROWS_THREADS = 128;
-__host__ __device__ inline int rows_flag_blocks(int nv) { return (nv * 7 + 3) / 4; }
+__host__ __device__ inline int rows_flag_blocks(int nv) { return nv * 7; }
 __host__ __device__ inline int rows_band_blocks(int nb, int nv) { return (nb - nv + 3) / 4; }
 __host__ __device__ inline int rows_blocks(int nb, int nv) { return rows_flag_blocks(nv) + rows_band_blocks(nb, nv); }
 __host__ __device__ inline size_t rows_bytes(int nb) {
@@ -1279,14 +1301,13 @@ FK_DEV void rows_band_warp(const RowsArgs& ra, int n1, int lane, double* parts) 
     if (lane < 6) row[6 + lane] = 0.0;  // ssx (3..5): occupied bands only
 }
 
-// Block task i of a request's rows: flag blocks (four occupied-band
-// components each, rows_warp), then band blocks (four bands each).  Every
+// Block task i of a request's rows: flag blocks (one occupied-band component
+// each), then band blocks (four bands each).  Every
 // thread of the block calls it with the same i.
 FK_DEV void rows_block(const RowsArgs& ra, int i, int tid) {
     const int warp = tid >> 5, lane = tid & 31, nfb = rows_flag_blocks(ra.nv);
     if (i < nfb) {
-        const int t = i * 4 + warp;
-        if (t < ra.nv * 7) rows_warp(ra, t / 7, t % 7, lane);
+        rows_flag_block(ra, i / 7, i % 7, tid);
         return;
     }
     const int bb = i - nfb, n0 = ra.nv + bb * 4;
