@@ -47,14 +47,6 @@ constexpr int GPP_COLS = 21;    // igp columns per 64-wide tensor-core n-tile (6
 // GPU tests' inputs with a margin (est_* kernels)
 constexpr double GPP_EST_C = 64.0;
 
-__global__ void igp_map_kernel(int ng, int nc, const int* inv, const int* indinv, int compact, int* igp, int* acol) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ng) return;
-    const int g = gpp_igp_of(i, nc, inv, indinv);
-    igp[i] = g;
-    acol[i] = g < 0 ? -1 : (compact ? i : g);
-}
-
 struct PrepArgs {
     int nb, nv, nc, ng;
     const double2 *aqsn, *eps, *wt;
@@ -74,7 +66,7 @@ struct PrepArgs {
     // from inv/indinv rather than read from igp, and the first chunk of each
     // column writes igp/acol, the epilogue weights W (mixed) and, in the last
     // column of a tensor-core tile, the image's padding rows; block (0, 0)
-    // clears the reduction's completion counter.
+    // clears the reduction's completion counter and the error word.
     int setup;
     const int *inv, *indinv;
     int* igp_out;
@@ -89,6 +81,7 @@ struct PrepArgs {
     int asx_neg;          // physics mode: the ssx weight is -occ*vcoul*conj(aqsm) (asxtemp subtracted)
     float* est;           // error estimate (EST prep): [nch][ng][3][6] magnitudes of the chunk's values
     int wm0 = -1;         // first band of the weight table W (-1: nvband)
+    int* err = nullptr;   // the contraction's error word, cleared by block (0, 0), or nullptr
 };
 
 // The set-up work of block (ch, my_igp) other than the image padding.
@@ -101,6 +94,7 @@ FK_DEV int prep_setup(const PrepArgs& p, int ch, int my_igp) {
             p.igp_out[my_igp] = igp;
             p.acol_out[my_igp] = acol;
             if (my_igp == 0 && p.counter) *p.counter = 0;
+            if (my_igp == 0 && p.err) *p.err = 0;
         }
         if (p.wf)
             for (int n1 = threadIdx.x; n1 < p.nv; n1 += blockDim.x) {
@@ -485,17 +479,69 @@ __global__ void half_break_kernel(int ng, int nc, const int* igpm, const double2
     }
 }
 
-// The diagonal value sch(igp) for columns on a block edge (igp % 512 == 0), else 0.
-__global__ void half_diag_kernel(int ng, int nc, const int* igpm, const double2* eps, const double2* wt,
-                                 const double* wx, double2* schd, int* counter) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t == 0) *counter = 0;  // the band reduction's completion count
-    if (t >= ng * 3) return;
-    const int my_igp = t / 3, iw = t % 3, igp = igpm[my_igp];
-    double2 v = make_double2(0.0, 0.0);
-    if (igp > 0 && (igp & 511) == 0)
-        v = half_sch(wx[iw], wt[(long)my_igp * nc + igp], eps[(long)my_igp * nc + igp]);
-    schd[t] = v;
+// What the half and the real-valued sum need before their preps, in one launch: the
+// column map, the epilogue weights W (rows nv.. of aqsmtemp), the image's padding, the
+// cleared counter and error word; the half sum's break table and its diagonal values
+// sch(igp) of the columns on a block edge (igp % 512 == 0, else 0); the real-valued
+// sum's aqsmtemp columns as complex (value, 0), [nb][ng] (the weights' source).
+// As separate launches these were four to six kernels of 3 to 5 us, with a gap of 2 to
+// 3 us behind each.  512 x 32768 x 20: half sum 199 -> 183 us, real-valued 163 -> 146 us.
+struct SetupArgs {
+    int nb, nv, nc, ng;
+    const int *inv, *indinv;
+    int *igp, *acol;
+    const double* vcoul;
+    float2* W;                // [ng][nb - nv], or nullptr
+    int *counter, *err;       // err: or nullptr
+    uint8_t* img;             // the image to pad, or nullptr
+    int NT, kstages, K;
+    const double2* aqsm;      // half sum (complex, all columns)
+    const double2 *eps, *wt;
+    const double* wx;
+    int* brk;
+    double2* schd;
+    const double* aqsm_re;    // real-valued sum
+    double2* ac;
+};
+constexpr int SETUP_THREADS = 128;
+__host__ __device__ inline int setup_row_blocks(int nb) { return (nb + SETUP_THREADS - 1) / SETUP_THREADS; }
+__global__ void __launch_bounds__(SETUP_THREADS) setup_kernel(SetupArgs a) {
+    const int nr = setup_row_blocks(a.nb), b = blockIdx.x, tid = threadIdx.x;
+    if (b >= nr * a.ng) {
+        const int s = b - nr * a.ng;
+        tcx::img_pad_stage<64>(a.img, s / a.NT, s % a.NT, a.NT, a.kstages, a.ng, GPP_COLS, a.K);
+        return;
+    }
+    const int h = b / nr, n = (b % nr) * SETUP_THREADS + tid;
+    const int g = gpp_igp_of(h, a.nc, a.inv, a.indinv);
+    if (b % nr == 0) {
+        if (tid == 0) {
+            a.igp[h] = g;
+            a.acol[h] = g < 0 ? -1 : (a.ac ? h : g);
+            if (a.brk) a.brk[h] = 0x7f7f7f7f;  // above every igp
+            if (h == 0) {
+                *a.counter = 0;
+                if (a.err) *a.err = 0;
+            }
+        }
+        if (a.schd && tid < 3)
+            a.schd[h * 3 + tid] = g > 0 && (g & 511) == 0
+                                      ? half_sch(a.wx[tid], a.wt[(long)h * a.nc + g], a.eps[(long)h * a.nc + g])
+                                      : make_double2(0.0, 0.0);
+    }
+    if (n >= a.nb) return;
+    double2 am = make_double2(0.0, 0.0);
+    if (a.ac) {
+        if (g >= 0) am.x = a.aqsm_re[(long)n * a.nc + g];
+        a.ac[(long)n * a.ng + h] = am;
+    } else if (g >= 0) {
+        am = a.aqsm[(long)n * a.nc + g];
+    }
+    if (a.W && n >= a.nv)
+        a.W[(long)h * (a.nb - a.nv) + n - a.nv] = g >= 0 ? tcx::weight_w1(am, 0.5 * a.vcoul[g]) : make_float2(0.f, 0.f);
+}
+inline void launch_setup(const SetupArgs& a, cudaStream_t st) {
+    setup_kernel<<<setup_row_blocks(a.nb) * a.ng + (a.img ? a.kstages * a.NT : 0), SETUP_THREADS, 0, st>>>(a);
 }
 
 // The flag-band terms of one (ig, iw): sch and ssx of flagOCC_solver (gppsum == 1)
@@ -1125,6 +1171,7 @@ struct RowsArgs {
     const double2* aqsn;  // [nb][nc]
     int nc;
     bool re_only;         // real-valued sum: the contraction partials carry it in their real parts
+    double* out_re = nullptr;  // its results [achtemp 3 | asxtemp 3 | acht_n1_loc nb], in place of out
     // totals folded in: the last block to finish (counter, zero at entry) writes out
     int* counter;
     double2* out;
@@ -1204,6 +1251,7 @@ FK_DEV void rows_flag_block(const RowsArgs& ra, int n1, int c, int tid) {
     if (tid == 0) {
         rows[(long)n1 * 8 + c] = v;
         if (c == 2 && ra.out) ra.out[7 + n1] = v;  // acht_n1_loc
+        if (c == 2 && ra.out_re) ra.out_re[6 + n1] = v.x;
     }
     __syncthreads();  // part is reused by the block's next task
 }
@@ -1293,6 +1341,7 @@ FK_DEV void rows_band_warp(const RowsArgs& ra, int n1, int lane, double* parts) 
         row[2 * c + im] = v;
         parts[p] = v;
         if (c == 2 && ra.out) ((double*)(ra.out + 7 + n1))[im] = v;  // acht_n1_loc
+        if (c == 2 && ra.out_re && !im) ra.out_re[6 + n1] = v;
     }
     if (lane >= 30) {
         row[12 + lane - 30] = a;  // component 6
@@ -1329,7 +1378,7 @@ FK_DEV void rows_block(const RowsArgs& ra, int i, int tid) {
 // add the sixteen splits; the ssx parts (occupied bands only) by threads 0..5.
 // out = [achtemp 3 | asxtemp 3 | achstemp | acht_n1_loc nb] (acht_n1_loc is
 // written by the band warps).
-FK_DEV void totals_block(int nb, int nv, const double2* rows, double2* out) {
+FK_DEV void totals_block(int nb, int nv, const double2* rows, double2* out, double* out_re = nullptr) {
     constexpr int B = 12;  // items in flight per thread: one round trip up to 16*B items
     const int t = threadIdx.x, q = t >> 4, s = t & 15;
     const int c = q < 6 ? q >> 1 : 6, im = q & 1;
@@ -1356,6 +1405,11 @@ FK_DEV void totals_block(int nb, int nv, const double2* rows, double2* out) {
     }
 #pragma unroll
     for (int off = 8; off > 0; off >>= 1) v = __dadd_rn(v, __shfl_down_sync(0xffffffffu, v, off));
+    if (out_re) {
+        if (s == 0 && c < 3 && !im) out_re[c] = v;
+        if (t < 6 && !(t & 1)) out_re[3 + (t >> 1)] = w;
+        return;
+    }
     double* o = (double*)out;
     if (s == 0) o[2 * c + im] = v;
     if (t < 6) o[6 + t] = w;
@@ -1376,7 +1430,7 @@ __global__ void __launch_bounds__(ROWS_THREADS) rows_kernel(RowsArgs ra) {
     }
     __syncthreads();
     if (!last) return;
-    totals_block(ra.nb, ra.nv, ra.rows, ra.out);
+    totals_block(ra.nb, ra.nv, ra.rows, ra.out, ra.out_re);
     if (threadIdx.x == 0) *ra.counter = 0;
 }
 
@@ -1894,22 +1948,6 @@ __global__ void real_carry_kernel(RealCarryArgs a) {
         for (int iw = 0; iw < 3; ++iw) put(iw, a.nc, 0.0);
 }
 
-// aqsmtemp's igp columns as complex (value, 0), [nb][ng]: the epilogue weights' source.
-__global__ void real_columns_kernel(int nb, int nc, int ng, const double* aqsm, const int* igp, double2* ac,
-                                    int* counter) {
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t == 0) *counter = 0;  // the band reduction's completion count
-    if (t >= (long)nb * ng) return;
-    const int n1 = (int)(t / ng), h = (int)(t % ng), g = igp[h];
-    ac[t] = make_double2(g >= 0 ? aqsm[(long)n1 * nc + g] : 0.0, 0.0);
-}
-
-// [achtemp 3 | asxtemp 3 | achstemp | acht_n1_loc nb] complex -> [3 | 3 | nb] real
-__global__ void real_out_kernel(int nb, const double2* outc, double* out) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 6 + nb; i += gridDim.x * blockDim.x)
-        out[i] = outc[i < 6 ? i : i + 1].x;
-}
-
 }  // namespace
 
 size_t gpp_workspace(const Ctx& c, const GppDev& r, bool pipelined) {
@@ -1991,24 +2029,20 @@ fk_status gpp_run_half(Ctx& c, const GppDev& r) {
         return fail(c, FK_ENOMEM, "workspace too small for GPP request");
     if (r.aqsm_compact || r.ldm != r.nc) return fail(c, FK_EINVAL, "gpp: the half sum needs all of aqsmtemp");
     c.launches = 0;
-    if ((p.mixed || p.tc64) && D) {
-        if (p.mixed && tcx::img_needs_pad(64, r.ng, GPP_COLS, r.nc))
-            tcx::img_pad_kernel<64><<<dim3(p.kstages, p.NT, 1), 256, 0, st>>>((uint8_t*)D, p.NT, p.kstages, r.ng,
-                                                                            GPP_COLS, r.nc);
-        if (cudaMemsetAsync(c.errword, 0, sizeof(int), st) != cudaSuccess)
-            return cuda_fail(c, cudaGetLastError(), "gpp: error word");
-    }
     phase_mark(c, 1);
-    igp_map_kernel<<<ceil_div(r.ng, 128), 128, 0, st>>>(r.ng, r.nc, r.inv, r.indinv, 0, igp, acol);
-    if (p.mixed && M > 0)
-        tcx::weight_table_kernel<<<dim3(ceil_div(M, 128), r.ng), 128, 0, st>>>(M, r.nv, r.ng, r.aqsm, r.ldm, r.vcoul,
-                                                                            igp, acol, 0.5, W, nullptr, nullptr);
-    if (cudaMemsetAsync(brk, 0x7f, (size_t)r.ng * sizeof(int), st) != cudaSuccess)
-        return cuda_fail(c, cudaGetLastError(), "gpp: break table");
+    SetupArgs sa{};
+    sa.nb = r.nb; sa.nv = r.nv; sa.nc = r.nc; sa.ng = r.ng;
+    sa.inv = r.inv; sa.indinv = r.indinv; sa.igp = igp; sa.acol = acol; sa.vcoul = r.vcoul;
+    sa.W = p.mixed && M > 0 ? W : nullptr;
+    sa.counter = counter;
+    sa.err = (p.mixed || p.tc64) && D ? c.errword : nullptr;
+    if (p.mixed && D && tcx::img_needs_pad(64, r.ng, GPP_COLS, r.nc)) sa.img = (uint8_t*)D;
+    sa.NT = p.NT; sa.kstages = p.kstages; sa.K = r.nc;
+    sa.aqsm = r.aqsm; sa.eps = r.eps; sa.wt = r.wt; sa.wx = r.wx; sa.brk = brk; sa.schd = schd;
+    launch_setup(sa, st);
     half_break_kernel<<<dim3(std::max(1, std::min(ceil_div(r.nc, 256), 64)), r.ng), 256, 0, st>>>(r.ng, r.nc, igp,
                                                                                                  r.eps, r.wt, brk);
-    half_diag_kernel<<<ceil_div(r.ng * 3, 128), 128, 0, st>>>(r.ng, r.nc, igp, r.eps, r.wt, r.wx, schd, counter);
-    c.launches += p.mixed && M > 0 ? 4 : 3;
+    c.launches += 2;
     for (int pass = 0; pass < p.passes; ++pass) {
         PrepArgs a{r.nb, r.nv, r.nc, r.ng, r.aqsn, r.eps, r.wt, r.wx, igp, (pass == 0 && M > 0) ? D : nullptr,
                    p.kstages, F, p.nch, p.tile, pass * NVC, 0, r.aqsm, brk};
@@ -2094,7 +2128,7 @@ fk_status gpp_run(Ctx& c, const GppDev& r, const GppPipe* pipe) {
         return fail(c, FK_ENOMEM, "workspace too small for GPP request");
     tc64::Bufs zb{};
     if (!take_tc64(c, p, zb)) return fail(c, FK_ENOMEM, "workspace too small for GPP request");
-    if ((p.mixed || p.tc64) && D) {
+    if (p.tc64 && D) {  // (mixed: the prep clears it)
         cudaError_t e = cudaMemsetAsync(c.errword, 0, sizeof(int), st);  // bounded-wait status
         if (e != cudaSuccess) return cuda_fail(c, e, "gpp: error word");
     }
@@ -2116,6 +2150,7 @@ fk_status gpp_run(Ctx& c, const GppDev& r, const GppPipe* pipe) {
             a.W = (p.mixed && M > 0) ? W : nullptr;
             a.M = M;
             a.wm0 = p.m0;
+            a.err = p.mixed && D ? c.errword : nullptr;
             a.counter = counter;
             a.wf = wf;
             a.asx_neg = Q == 2;
@@ -2726,7 +2761,7 @@ struct RealPlan {
     GppDev cd;      // its shape
     long K2;
     int nch, tile;
-    size_t bytesDv, bytesMask, bytesF, bytesAC, bytesOutc, bytesD64;
+    size_t bytesDv, bytesMask, bytesF, bytesAC, bytesD64;
 };
 
 RealPlan make_real_plan(const Ctx& c, const GppRealDev& r) {
@@ -2743,7 +2778,6 @@ RealPlan make_real_plan(const Ctx& c, const GppRealDev& r) {
     q.bytesMask = (size_t)r.ng * r.nc;
     q.bytesF = (size_t)q.nch * std::max(r.nv, 1) * r.ng * 6 * sizeof(double2);
     q.bytesAC = (size_t)r.nb * r.ng * sizeof(double2);
-    q.bytesOutc = (7 + (size_t)r.nb) * sizeof(double2);
     return q;
 }
 }  // namespace
@@ -2751,7 +2785,7 @@ RealPlan make_real_plan(const Ctx& c, const GppRealDev& r) {
 size_t gpp_real_workspace(const Ctx& c, const GppRealDev& r) {
     const RealPlan q = make_real_plan(c, r);
     return q.c.bytesD + q.c.bytesW + q.c.bytesP + q.c.bytesRows + q.c.bytesIgp + q.bytesDv + q.bytesMask + q.bytesF +
-           q.bytesAC + q.bytesOutc + q.c.bytesZ() + 13 * 256;
+           q.bytesAC + q.c.bytesZ() + 12 * 256;
 }
 
 fk_status gpp_real_run(Ctx& c, const GppRealDev& r) {
@@ -2770,30 +2804,25 @@ fk_status gpp_real_run(Ctx& c, const GppRealDev& r) {
     uint8_t* mask = (uint8_t*)c.ws.take(q.bytesMask);
     double2* F = (double2*)c.ws.take(q.bytesF);
     double2* AC = (double2*)c.ws.take(q.bytesAC);
-    double2* outc = (double2*)c.ws.take(q.bytesOutc);
     int* counter = (int*)c.ws.take(sizeof(int));
-    if (!igp || !rows || !Dv || !mask || !F || !AC || !outc || !counter || (p.bytesD && !D) || (p.bytesP && !P) ||
+    if (!igp || !rows || !Dv || !mask || !F || !AC || !counter || (p.bytesD && !D) || (p.bytesP && !P) ||
         (p.bytesW && !W))
         return fail(c, FK_ENOMEM, "workspace too small for the real-valued GPP request");
     tc64::Bufs zb{};
     if (!take_tc64(c, p, zb)) return fail(c, FK_ENOMEM, "workspace too small for the real-valued GPP request");
     c.launches = 0;
-    if ((p.mixed || p.tc64) && D) {
-        if (p.mixed && tcx::img_needs_pad(64, r.ng, GPP_COLS, (int)q.K2))
-            tcx::img_pad_kernel<64><<<dim3(p.kstages, p.NT, 1), 256, 0, st>>>((uint8_t*)D, p.NT, p.kstages, r.ng,
-                                                                            GPP_COLS, (int)q.K2);
-        if (cudaMemsetAsync(c.errword, 0, sizeof(int), st) != cudaSuccess)
-            return cuda_fail(c, cudaGetLastError(), "gpp_real: error word");
-    }
     phase_mark(c, 1);
-    igp_map_kernel<<<ceil_div(r.ng, 128), 128, 0, st>>>(r.ng, r.nc, r.inv, r.indinv, 1, igp, acol);
-    real_columns_kernel<<<ceil_div(r.nb * r.ng, 256), 256, 0, st>>>(r.nb, r.nc, r.ng, r.aqsm, igp, AC, counter);
-    c.launches += 2;
-    if (p.mixed && M > 0) {
-        tcx::weight_table_kernel<<<dim3(ceil_div(M, 128), r.ng), 128, 0, st>>>(M, r.nv, r.ng, AC, r.ng, r.vcoul, igp,
-                                                                            acol, 0.5, W, nullptr, nullptr);
-        ++c.launches;
-    }
+    SetupArgs sa{};
+    sa.nb = r.nb; sa.nv = r.nv; sa.nc = r.nc; sa.ng = r.ng;
+    sa.inv = r.inv; sa.indinv = r.indinv; sa.igp = igp; sa.acol = acol; sa.vcoul = r.vcoul;
+    sa.W = p.mixed && M > 0 ? W : nullptr;
+    sa.counter = counter;
+    sa.err = (p.mixed || p.tc64) && D ? c.errword : nullptr;
+    if (p.mixed && D && tcx::img_needs_pad(64, r.ng, GPP_COLS, (int)q.K2)) sa.img = (uint8_t*)D;
+    sa.NT = p.NT; sa.kstages = p.kstages; sa.K = (int)q.K2;
+    sa.aqsm_re = r.aqsm; sa.ac = AC;
+    launch_setup(sa, st);
+    ++c.launches;
     const int passes = std::max(1, ceil_div(r.nv, NVC));
     for (int pass = 0; pass < passes; ++pass) {
         RealPrepArgs a{r.nb, r.nv, r.nc, r.ng, r.aqsn, r.eps, r.wt, r.wx, r.lda, igp,
@@ -2850,10 +2879,9 @@ fk_status gpp_real_run(Ctx& c, const GppRealDev& r) {
     RowsArgs ra{r.nb, r.nv, r.ng, P ? p.KS * p.NT : 0, P, 0, nullptr, q.nch, F, r.ng, AC, r.vcoul, igp, acol, rows};
     ra.re_only = true;
     ra.counter = counter;  // the last block also writes the totals
-    ra.out = outc;
+    ra.out_re = r.out;
     rows_kernel<<<rows_blocks(r.nb, r.nv), ROWS_THREADS, 0, st>>>(ra);
-    real_out_kernel<<<std::max(1, std::min(ceil_div(6 + r.nb, 256), 64)), 256, 0, st>>>(r.nb, outc, r.out);
-    c.launches += 2;
+    ++c.launches;
     phase_mark(c, 4);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? FK_OK : cuda_fail(c, e, "gpp_real kernels");

@@ -1294,12 +1294,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256)
 // else min(ROWS, cols - ROWS*nt).  NS sub-tiles per stage (six for the GPP
 // images and the FF B images, four for FF's A image).  Grid (kstages, NT, planes).
 template <int ROWS, int NS = NSUB>
-__global__ void img_pad_kernel(uint8_t* img, int NT, int kstages, int cols, int gpp_cols, int K) {
-    const int kst = blockIdx.x, nt = blockIdx.y, pl = blockIdx.z;
+__device__ __forceinline__ void img_pad_stage(uint8_t* img, int kst, long tile, int NT, int kstages, int cols, int gpp_cols,
+                                              int K) {
+    const int nt = (int)(tile % NT);  // tile = plane * NT + n-tile
     const int vr = gpp_cols > 0 ? 3 * min(gpp_cols, cols - gpp_cols * nt) : min(ROWS, cols - ROWS * nt);
     const int kv = min(BK, K - kst * BK);  // valid k-values of this stage
     if (vr >= ROWS && kv >= BK) return;
-    uint8_t* st = img + (((long)pl * NT + nt) * kstages + kst) * (long)(ROWS * NS * 64);
+    uint8_t* st = img + (tile * kstages + kst) * (long)(ROWS * NS * 64);
     for (int i = threadIdx.x; i < ROWS * BK; i += blockDim.x) {
         const int row = i / BK, k = i % BK;
         if (row < vr && k < kv) continue;
@@ -1307,6 +1308,10 @@ __global__ void img_pad_kernel(uint8_t* img, int NT, int kstages, int cols, int 
 #pragma unroll
         for (int q = 0; q < NS; ++q) *(uint16_t*)(st + q * ROWS * 64 + off) = 0;
     }
+}
+template <int ROWS, int NS = NSUB>
+__global__ void img_pad_kernel(uint8_t* img, int NT, int kstages, int cols, int gpp_cols, int K) {
+    img_pad_stage<ROWS, NS>(img, blockIdx.x, (long)blockIdx.z * NT + blockIdx.y, NT, kstages, cols, gpp_cols, K);
 }
 // True when some image position needs img_pad_kernel.
 inline bool img_needs_pad(int rows_per_tile, int cols, int gpp_cols, int K) {
