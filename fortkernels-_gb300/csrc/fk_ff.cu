@@ -307,10 +307,10 @@ struct FfPlan {
     int zgroup = 0;
 };
 
-// The converted planes of an FP64 request held at once: 2 GB of images (the
-// planes of 512 x 4096 x 512 x 15 in one launch), at most the 64 planes of one
-// launch's table.
-constexpr size_t FF_ZGROUP_BYTES = (size_t)2 << 30;
+// The converted planes of an FP64 request held at once: 4 GB of images (the R and A
+// planes of 512 x 4096 x 512 x 15 in one launch: over 76 CTA pairs, the units of R and
+// of A each left a last wave partly empty), at most the 64 planes of one launch's table.
+constexpr size_t FF_ZGROUP_BYTES = (size_t)4 << 30;
 
 // k-slices for the persistent tensor-core kernel (see fk_gpp.cu)
 void ff_pick_split_tc(long tiles, int K, int sms, int& KS, int& kchunk) {
@@ -416,19 +416,8 @@ FfPlan make_plan(const Ctx& c, const FfDev& r, const double* ekq_h, const double
         p.KS = std::max(1, std::min((c.sms * 2 + tiles - 1) / tiles, std::max(1, r.nc / 256)));
         p.kchunk = ((r.nc + p.KS - 1) / p.KS + 15) / 16 * 16;
         p.KS = (r.nc + p.kchunk - 1) / p.kchunk;
-        if (r.tc64) {
-            const tc64::Plan one = tc64::make_plan(r.nb, r.ng, r.nc, 1, c.sms / 2);
-            p.zgroup = (int)std::min<size_t>(std::min(nplanes, (int)tc64::MAXPL), std::max<size_t>(1, FF_ZGROUP_BYTES / one.bytesB));
-            p.zgroup = ceil_div(nplanes, ceil_div(nplanes, p.zgroup));  // even groups
-            p.z = tc64::make_plan(r.nb, r.ng, r.nc, p.zgroup, c.sms / 2);
-            p.tc64 = p.z.KS > 0;
-        }
-        if (p.tc64) {
-            p.NT = 2 * p.z.NT;  // its partial slots: the re and im half of each 64-wide n-tile
-            p.KS = p.z.KS;
-        }
     }
-    if (p.mixed || p.tc64) {
+    if (p.mixed || r.tc64) {
         // the correction term of band n1 reads the A planes ifq_c and ifq_c + 1 only
         // (achDtemp_cor_Kernel, FFKer_cori/ffKernel.cpp:212-246): sort the bands by that
         // bracket so that each A plane is contracted over the row tiles of its bands only
@@ -438,7 +427,7 @@ FfPlan make_plan(const Ctx& c, const FfDev& r, const double* ekq_h, const double
             const int ka = p.fact[a].kind ? p.fact[a].ifq_c : 1 << 30, kb = p.fact[b].kind ? p.fact[b].ifq_c : 1 << 30;
             return ka < kb;
         });
-        long tiles = 0;
+        long tiles = 0, ztiles = 0;
         for (int f : p.planesA) {
             int lo = -1, hi = -1;
             for (int i = 0; i < r.nb; ++i) {
@@ -452,9 +441,24 @@ FfPlan make_plan(const Ctx& c, const FfDev& r, const double* ekq_h, const double
             p.aLo.push_back(lo);
             p.aHi.push_back(hi);
             tiles += hi > lo ? (hi - 1) / tcx::BM - lo / tcx::BM + 1 : 0;
+            ztiles += hi > lo ? (hi - 1) / tc64::BM - lo / tc64::BM + 1 : 0;
         }
         // k-slices for the one launch over all A planes' (row tile, n-tile) pairs
         if (p.mixed) ff_pick_split_tc(std::max(1L, tiles) * p.NT, r.nc, c.sms, p.KSa, p.kchunka);
+        if (r.tc64) {
+            const int all = std::max(1, (int)(p.planesR.size() + p.planesA.size())), pairs = c.sms / 2;
+            const tc64::Plan one = tc64::make_plan(r.nb, r.ng, r.nc, 1, pairs);
+            p.zgroup = (int)std::min<size_t>(std::min(all, (int)tc64::MAXPL), std::max<size_t>(1, FF_ZGROUP_BYTES / one.bytesB));
+            const int launches = ceil_div(all, p.zgroup);
+            p.zgroup = ceil_div(all, launches);  // even groups
+            ztiles += (long)p.planesR.size() * one.MT;
+            p.z = tc64::make_plan(r.nb, r.ng, r.nc, p.zgroup, pairs, std::max(1L, ztiles / launches), 90000.0);
+            p.tc64 = p.z.KS > 0;
+        }
+        if (p.tc64) {
+            p.NT = 2 * p.z.NT;  // its partial slots: the re and im half of each 64-wide n-tile
+            p.KS = p.z.KS;
+        }
     }
     const size_t slots = (size_t)p.KS * p.NT * (p.mixed ? tcx::FF_EPI_WARPS : 1);  // partial slots per plane
     const size_t slotsA = p.mixed ? (size_t)p.KSa * p.NT * tcx::FF_EPI_WARPS : slots;
@@ -501,8 +505,10 @@ fk_status ff_run(Ctx& c, const FfDev& r, const FfHost& h, const FfPipe* pipe) {
     FactRow* fact = (FactRow*)tab;
     int* order = p.mixed || p.tc64 ? (int*)(tab + ft.order) : nullptr;
     int* planes = (int*)(tab + ft.planes);
-    double2* PR = (double2*)c.ws.take(slots * std::max(nR, 1) * r.nb * 2 * sizeof(double2));
-    double2* PA = nA ? (double2*)c.ws.take(slotsA * nA * r.nb * 2 * sizeof(double2)) : nullptr;
+    // FP64 on the tensor cores: the A planes' partials follow the R planes' (one launch covers both)
+    const size_t bytesPA = slotsA * nA * r.nb * 2 * sizeof(double2);
+    double2* PR = (double2*)c.ws.take(slots * std::max(nR, 1) * r.nb * 2 * sizeof(double2) + (p.tc64 ? bytesPA : 0));
+    double2* PA = !nA ? nullptr : p.tc64 ? PR + slots * nR * r.nb * 2 : (double2*)c.ws.take(bytesPA);
     double2* tabs = (double2*)c.ws.take(3 * (size_t)r.nb * r.nf * sizeof(double2));
     double2* SD = (double2*)c.ws.take((size_t)r.ne * r.nb * sizeof(double2));
     SchdiTab stab{};
@@ -694,31 +700,6 @@ fk_status ff_run(Ctx& c, const FfDev& r, const FfHost& h, const FfPipe* pipe) {
             k<<<grid1, tcx::THREADS_FF, smem, st>>>(t);
             kernel_end(c);
             c.launches += 2;
-        } else if (p.tc64) {
-            a.rowmap = order;
-            const size_t pslab = slots * r.nb * 2;
-            for (int g0 = 0; g0 < nb_; g0 += p.zgroup) {
-                ContractArgs ag = a;
-                ag.batches = std::min(p.zgroup, nb_ - g0);
-                ag.batch_plane = pls + g0;
-                ag.P = P + g0 * pslab;
-                // R planes: all bands; A planes: the 256-row tiles of the bands that read each one
-                tc64::PlaneTab tab{};
-                tab.n = ag.batches;
-                for (int j = 0; j < tab.n; ++j) {
-                    const int lo = a0 < 0 ? 0 : p.aLo[a0 + g0 + j], hi = a0 < 0 ? r.nb : p.aHi[a0 + g0 + j];
-                    tab.mt0[j] = hi > lo ? lo / tc64::BM : 0;
-                    tab.MT[j] = hi > lo ? (hi - 1) / tc64::BM - tab.mt0[j] + 1 : 0;
-                    tab.u0[j + 1] = tab.u0[j] + tab.MT[j] * p.z.NT * p.z.KS;
-                }
-                if (tab.u0[tab.n] == 0) continue;
-                // the timed kernel is the R planes' contraction
-                const bool prof = c.profiling;
-                if (a0 >= 0) c.profiling = false;
-                tc64::enqueue<EPI_FF>(c, ag, p.z, zb, tab, a0 < 0);
-                if (a0 >= 0) --c.nk;
-                c.profiling = prof;
-            }
         } else {
             dim3 grid(p.MT, p.NT * p.KS * nb_);
             auto k = d64::contract_kernel<EPI_FF>;
@@ -729,7 +710,45 @@ fk_status ff_run(Ctx& c, const FfDev& r, const FfHost& h, const FfPipe* pipe) {
             ++c.launches;
         }
     };
-    if (!pipe) {
+    // FP64 on the tensor cores: planes i0 .. i1-1 of the R planes followed by the A planes
+    // (their partials in the same order): R planes over all bands and with both sums, A
+    // planes over the 256-row tiles of the bands that read each one
+    auto contract64 = [&](int i0, int i1) {
+        const size_t pslab = slots * r.nb * 2;
+        // the timed kernel is the R planes' contraction, whose flops the caller counts
+        if (c.profiling && i0 < nR && nR < i1) i1 = nR;
+        for (int g0 = i0, g1; g0 < i1; g0 = g1) {
+            g1 = std::min(g0 + p.zgroup, i1);
+            ContractArgs a{};
+            a.A = r.aqsn; a.lda = r.nc; a.M = r.nb; a.rowmap = order;
+            const int n2 = std::max(0, std::min(g1, nR) - g0);
+            a.B = n2 ? r.epsR : r.epsA;
+            a.B2 = r.epsA; a.batches1 = n2;
+            a.ldb = r.nc; a.bstride = (long)r.ng * r.nc; a.N = r.ng; a.K = r.nc;
+            a.batches = g1 - g0; a.batch_plane = planes + g0;
+            a.aqsm = r.aqsm; a.ldm = r.nc; a.vcoul = r.vcoul; a.igp = igp; a.acol = igp; a.wscale = 1.0; a.G = 2;
+            a.P = PR + g0 * pslab;
+            tc64::PlaneTab tab{};
+            tab.n = a.batches;
+            tab.n2 = n2;
+            for (int j = 0; j < tab.n; ++j) {
+                const int lo = j < n2 ? 0 : p.aLo[g0 + j - nR], hi = j < n2 ? r.nb : p.aHi[g0 + j - nR];
+                tab.mt0[j] = hi > lo ? lo / tc64::BM : 0;
+                tab.MT[j] = hi > lo ? (hi - 1) / tc64::BM - tab.mt0[j] + 1 : 0;
+                tab.u0[j + 1] = tab.u0[j] + tab.MT[j] * p.z.NT * p.z.KS;
+            }
+            if (tab.u0[tab.n] == 0) continue;
+            const bool prof = c.profiling;
+            if (!n2) c.profiling = false;
+            tc64::enqueue<EPI_FF>(c, a, p.z, zb, tab);
+            if (!n2) --c.nk;
+            c.profiling = prof;
+        }
+        return i1;
+    };
+    if (p.tc64 && !pipe) {
+        for (int i = 0; i < nR + nA;) i = contract64(i, nR + nA);
+    } else if (!pipe) {
         if (nR) contract(r.epsR, planes, nR, PR, imgR, bscaleR, -1);
         if (nA) contract(r.epsA, planes + nR, nA, PA, imgA, bscaleA, 0);  // A planes: AW only
     } else {
@@ -744,6 +763,10 @@ fk_status ff_run(Ctx& c, const FfDev& r, const FfHost& h, const FfPipe* pipe) {
                 return cuda_fail(c, cudaGetLastError(), "ff: pipeline wait");
             uint8_t* img = isR ? imgR : imgA;
             float* bs = isR ? bscaleR : bscaleA;
+            if (p.tc64) {
+                contract64(p.groups[q], p.groups[q + 1]);
+                continue;
+            }
             contract(isR ? r.epsR : r.epsA, planes + (isR ? 0 : nR) + g0, n, isR ? PR + g0 * pslab : PA + g0 * pslabA,
                      img ? img + g0 * islab : nullptr, bs ? bs + (size_t)g0 * r.ng : nullptr, isR ? -1 : g0);
         }

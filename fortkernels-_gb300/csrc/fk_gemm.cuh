@@ -51,6 +51,8 @@ struct ContractArgs {
     // FP64 engine behind the tensor-core one (fk_tc64.cuh)
     int nt_tiles = 0;               // n-tiles of the slot layout (0: ceil(N / BN))
     const int* only_if = nullptr;   // the launch does nothing while this is 0
+    const void* B2 = nullptr;       // batches from batches1 on read their planes here
+    int batches1 = 0;
     const int* rowmap = nullptr;    // row m of A and aqsm (nullptr: m0 + m)
 };
 
@@ -134,7 +136,8 @@ __global__ void __launch_bounds__(THREADS) contract_kernel(ContractArgs a) {
     const int mt = blockIdx.x, nt = blockIdx.y % NT;
     const int ks = (blockIdx.y / NT) % a.KS, batch = blockIdx.y / (NT * a.KS);
     const int plane = a.batch_plane ? a.batch_plane[batch] : batch;
-    const double2* B = reinterpret_cast<const double2*>(a.B) + (long)plane * a.bstride;
+    const double2* B =
+        reinterpret_cast<const double2*>(a.B2 && batch >= a.batches1 ? a.B2 : a.B) + (long)plane * a.bstride;
     const int k0 = ks * a.kchunk;
     const int k1 = min(a.K, k0 + a.kchunk);
     const int nk = k1 > k0 ? ceil_div(k1 - k0, BK) : 0;

@@ -1632,7 +1632,7 @@ template <int EPI>
 void run_tc64(Ctx& c, const ContractArgs& a, const tc64::Plan& z, const tc64::Bufs& b, bool have_a = false) {
     tc64::enqueue_weights(c, a, EPI == EPI_GPP ? a.N / 3 : a.N, b, false);
     if (!have_a) tc64::enqueue_a(c, a, z, b);
-    tc64::enqueue<EPI>(c, a, z, b, tc64::one_plane(z), false);
+    tc64::enqueue<EPI>(c, a, z, b, tc64::one_plane(z));
 }
 
 // A side branch of the context's stream: work queued between fork and join on

@@ -72,6 +72,7 @@ constexpr int MAXPL = 64;             // planes of one launch
 // Planes (batches) of one launch, each over its own range of 256-row tiles.
 struct PlaneTab {
     int n;
+    int n2;  // the planes before n2 also get the sums weighted by W2 (FF)
     int u0[MAXPL + 1], mt0[MAXPL], MT[MAXPL];
 };
 
@@ -91,7 +92,8 @@ struct Args {
 
 // ------------------------------------------------------------- conversion
 struct SplitArgs {
-    const double2* src;
+    const double2 *src, *src2;  // batches from n1 on read their planes from src2
+    int n1;
     long ld, plane_stride;
     const int* planes;   // plane index of each batch (nullptr: identity)
     const int* rowmap;   // image row -> source row (nullptr: identity)
@@ -183,7 +185,7 @@ __global__ void __launch_bounds__(256) split_kernel(SplitArgs s) {
     }
     uint32_t ph = 0;
     for (int row = blockIdx.y; row < s.rows; row += gridDim.y, ph ^= 1) {
-        const double2* src = s.src + (long)plane * s.plane_stride + (long)(s.rowmap ? s.rowmap[row] : row) * s.ld + k0;
+        const double2* src = (batch < s.n1 ? s.src : s.src2) + (long)plane * s.plane_stride + (long)(s.rowmap ? s.rowmap[row] : row) * s.ld + k0;
         if (SMEM_ROW) {
             __syncthreads();  // the previous row was read
             if (threadIdx.x == 0) {
@@ -587,6 +589,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) contract
             const int ea = t.ea[(long)x.ks * t.M + mc];
             const int* ebp = t.eb + ((long)x.pl * t.KS + x.ks) * t.N + x.nt * BN;
             const int n0 = x.nt * BN, ncol = min(BN, t.N - n0);
+            const bool both = EPI == EPI_FF && x.pl < t.tab.n2;
             double2 g[3] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
 #pragma unroll
             for (int j0 = 0; j0 < BN; j0 += 8) {
@@ -605,7 +608,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) contract
                     for (int j = 0; j < 4; ++j) {
                         const int n = n0 + min(j0 + jb + j, ncol - 1), h = EPI == EPI_GPP ? n / 3 : n;
                         w1[j] = t.W1[(long)h * t.M + mc];
-                        if (EPI == EPI_FF) w2[j] = t.W2 ? t.W2[(long)h * t.M + mc] : make_double2(0.0, 0.0);
+                        if (EPI == EPI_FF) w2[j] = both ? t.W2[(long)h * t.M + mc] : make_double2(0.0, 0.0);
                     }
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
@@ -618,7 +621,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) contract
                         const double sr = half ? -s : s;
                         g[gi].x = fma(half ? w1[j].y : w1[j].x, sr, g[gi].x);
                         g[gi].y = fma(half ? w1[j].x : w1[j].y, s, g[gi].y);
-                        if (EPI == EPI_FF && t.W2) {
+                        if (EPI == EPI_FF && both) {
                             g[1].x = fma(half ? w2[j].y : w2[j].x, sr, g[1].x);
                             g[1].y = fma(half ? w2[j].x : w2[j].y, s, g[1].y);
                         }
@@ -655,22 +658,24 @@ struct Plan {
     size_t slots() const { return (size_t)KS * NT * 2; }  // partial slots per plane
 };
 
-// The k-split: the fewest pair-cycles over whole waves, a unit costing ~7200
-// cycles per stage and ~45000 for its weighted sums (measured on GB300: see the
-// epilogue's FP64 instructions).  KS == 0: no split fits (callers keep the DMMA kernel).
-inline Plan make_plan(int M, int N, int K, int planes, int pairs) {
+// The k-split: the fewest pair-cycles over whole waves, a unit costing ~8700
+// cycles per stage and `sums` for its weighted sums (measured on GB300: ~50000 for one
+// sum per column, ~90000 with FF's second one; see the epilogue's FP64 instructions).
+// row_tiles: the launch's row tiles over all planes (0: every plane has all of
+// them).  KS == 0: no split fits (callers keep the DMMA kernel).
+inline Plan make_plan(int M, int N, int K, int planes, int pairs, long row_tiles = 0, double sums = 50000.0) {
     Plan p{};
     p.MT = ceil_div(std::max(M, 1), BM);
     p.NT = ceil_div(std::max(N, 1), BN);
     p.kstages = ceil_div(K, BK);
-    const long tiles = (long)p.MT * p.NT * std::max(planes, 1);
+    const long tiles = (row_tiles > 0 ? row_tiles : (long)p.MT * std::max(planes, 1)) * p.NT;
     double best = 1e300;
     for (int ks = 1; ks <= std::min(p.kstages, 512); ++ks) {
         const int ku = ceil_div(p.kstages, ks);
         if (ku * BK > MAXK || ceil_div(p.kstages, ku) != ks) continue;
         if (2l * p.NT * ks * std::max(planes, 1) > 65535) continue;  // the DMMA kernel's grid
         const long waves = (tiles * ks + pairs - 1) / pairs;
-        const double cost = (double)waves * (ku * 7200.0 + 45000.0);
+        const double cost = (double)waves * (ku * 8700.0 + sums);
         if (cost < best * 0.999) {
             best = cost;
             p.KS = ks;
@@ -714,7 +719,7 @@ inline void launch_split(Ctx& c, const SplitArgs& s, int batches) {
 // The digits of a.A's rows m0 .. m0+M-1 (or rowmap[0 .. M)) and the flag's reset.
 inline void enqueue_a(Ctx& c, const ContractArgs& a, const Plan& p, const Bufs& b) {
     cudaMemsetAsync(flag_word(c), 0, sizeof(int), c.stream);
-    SplitArgs s{a.rowmap ? a.A : a.A + (long)a.m0 * a.lda, a.lda, 0, nullptr, a.rowmap, a.M, a.K, p.KS, p.kst_unit,
+    SplitArgs s{a.rowmap ? a.A : a.A + (long)a.m0 * a.lda, nullptr, 1, a.lda, 0, nullptr, a.rowmap, a.M, a.K, p.KS, p.kst_unit,
                 p.kstages, 2 * p.MT, b.A, b.ea, flag_word(c), c.errword, c.wait_limit};
     launch_split<false>(c, s, 1);
 }
@@ -722,11 +727,11 @@ inline void enqueue_a(Ctx& c, const ContractArgs& a, const Plan& p, const Bufs& 
 // The digits of a.batches planes (at most MAXPL) of a.B, the contraction over the row tiles of `tab` and the
 // DMMA kernel for rows that cannot be represented.
 template <int EPI>
-inline void enqueue(Ctx& c, ContractArgs a, const Plan& p, const Bufs& b, const PlaneTab& tab, bool second) {
-    SplitArgs s{(const double2*)a.B, a.ldb, a.bstride, a.batch_plane, nullptr, a.N, a.K, p.KS, p.kst_unit, p.kstages,
+inline void enqueue(Ctx& c, ContractArgs a, const Plan& p, const Bufs& b, const PlaneTab& tab) {
+    SplitArgs s{(const double2*)a.B, (const double2*)a.B2, a.B2 ? a.batches1 : a.batches, a.ldb, a.bstride, a.batch_plane, nullptr, a.N, a.K, p.KS, p.kst_unit, p.kstages,
                 p.NT, b.B, b.eb, flag_word(c), c.errword, c.wait_limit};
     launch_split<true>(c, s, a.batches);
-    Args t{b.A, b.B, b.ea, b.eb, b.W1, second ? b.W2 : nullptr, a.P, a.M, a.N, p.NT, p.KS, p.kst_unit, p.kstages, a.G,
+    Args t{b.A, b.B, b.ea, b.eb, b.W1, b.W2, a.P, a.M, a.N, p.NT, p.KS, p.kst_unit, p.kstages, a.G,
            flag_word(c), c.errword, c.wait_limit, tab};
     auto k = contract_kernel<EPI>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
