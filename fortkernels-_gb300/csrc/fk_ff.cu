@@ -27,47 +27,6 @@
 namespace fk {
 namespace {
 
-__global__ void ff_igp_kernel(int ng, int nc, const int* inv, const int* indinv, int* igp) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ng) return;
-    int ind = inv[i];
-    int g = (ind >= 0 && ind < nc) ? indinv[ind] : -1;
-    igp[i] = (g >= 0 && g < nc) ? g : -1;
-}
-
-// Sum the (KS x NT) partial slots of each (batch, row, group) and scatter into
-// the per-plane tables RW/RS [nb][nf]; partial row i belongs to band order[i]
-// (or i).  One warp per (row, batch); lane 4g + c takes component c (RW re, RW
-// im, RS re, RS im) of slots g, g+8, .. in order, so that the four lanes of a
-// slot read its 32-byte (RW, RS) record as one sector, then three shuffle
-// levels add the eight slot groups (fixed order: deterministic).  GB300's FP64
-// pipe retires one warp instruction per 64 cycles per sub-partition: this takes
-// slots/8 + 3 FP64 adds per warp.
-__global__ void ff_rows_kernel(int nb, int nf, int batches, int slots_per_batch, const int* planes,
-                               const double2* P, double2* RW, double2* RS, const int* order) {
-    const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), b = blockIdx.y, lane = threadIdx.x & 31;
-    if (i >= nb || b >= batches) return;  // warp-uniform
-    const int g = lane >> 2, comp = lane & 3;
-    const double* q = (const double*)(P + ((long)b * slots_per_batch * nb + i) * 2) + comp;
-    const long sstride = 4L * nb;  // doubles per slot
-    const int ns = slots_per_batch;
-    double v = 0.0;
-    for (int s0 = g; s0 < ns; s0 += 64) {
-        double a[8];  // eight loads in flight; clamped indices, +0.0 past the end (exact)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) a[j] = q[(long)min(s0 + 8 * j, ns - 1) * sstride];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v = __dadd_rn(v, s0 + 8 * j < ns ? a[j] : 0.0);
-    }
-#pragma unroll
-    for (int off = 4; off < 32; off <<= 1) v = __dadd_rn(v, __shfl_xor_sync(0xffffffffu, v, off));
-    if (lane >= 4) return;
-    const int n1 = order ? order[i] : i;
-    const int f = planes[b];
-    if (comp < 2) ((double*)(RW + (long)n1 * nf + f))[comp] = v;
-    else if (RS) ((double*)(RS + (long)n1 * nf + f))[comp - 2] = v;
-}
-
 struct FactRow {
     int ifq_a, ifq_c, kind;  // kind: 0 none, 1 schDttt_corKernel1, 2 schDttt_corKernel2
     double fa1, fa2, fc1, fc2;
@@ -102,7 +61,7 @@ FK_DEV double2 gc_div(double2 a, double2 b) {
 // (iw, n1), sum over ifreq of -((0, pref[f]) x schDt[n1][f]) / (wx - coh[f]),
 // coh[f] = (grid[f] - brd[f].re, 0 - brd[f].im), wx = freqevalmin - ekq[n1] +
 // (iw-1)*freqevalstep.  The (n1, f) numerator and the f terms do not depend on
-// iw: they are formed once here (same FP64 operations as inside the loop), and
+// iw: they are formed once (same FP64 operations as inside the loop), and
 // for the mixed path also as FP32 tables, with coh.re split into a float-float
 // pair so that the nearly cancelling difference wx - coh.re keeps its accuracy.
 struct SchdiTab {
@@ -111,46 +70,93 @@ struct SchdiTab {
     float2* cohr;        // [nf]: coh.re as (hi, lo)
 };
 
-__global__ void ff_schdi_tables_kernel(EpiArgs a, SchdiTab t) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x, n1 = blockIdx.y;
-    if (f >= a.nf) return;
-    const double2 coh = make_double2(__dsub_rn(a.grid[f], a.brd[f].x), 0.0 - a.brd[f].y);
-    const double2 num = cmul(make_double2(0.0, a.pref[f]), schdt_of(a, n1, f));
-    t.num[(long)n1 * a.nf + f] = num;
-    if (n1 == 0) t.coh[f] = coh;
-    if (t.f32) {
-        t.f32[(long)n1 * a.nf + f] =
-            make_float4(f64_to_f32_bits(num.x), f64_to_f32_bits(num.y), f64_to_f32_bits(0.0 - coh.y), 0.f);
-        if (n1 == 0) {
+// The column map, and the f terms of the schDi sum.
+__global__ void ff_setup_kernel(int ng, int nc, const int* inv, const int* indinv, int* igp, EpiArgs a, SchdiTab t) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < ng) {
+        const int ind = inv[i];
+        const int g = (ind >= 0 && ind < nc) ? indinv[ind] : -1;
+        igp[i] = (g >= 0 && g < nc) ? g : -1;
+    }
+    if (i < a.nf) {
+        const double2 coh = make_double2(__dsub_rn(a.grid[i], a.brd[i].x), 0.0 - a.brd[i].y);
+        t.coh[i] = coh;
+        if (t.f32) {
             const float hi = f64_to_f32_bits(coh.x);
-            t.cohr[f] = make_float2(hi, f64_to_f32_bits(coh.x - (double)hi));
+            t.cohr[i] = make_float2(hi, f64_to_f32_bits(coh.x - (double)hi));
         }
     }
 }
 
-// FP64: the reference's operations per term (GPUComplex_divide), block = one band,
-// threads = consecutive iw, so every f-table load is uniform across the warp.
-__global__ void ff_schdi_kernel(EpiArgs a, SchdiTab t) {
-    const int iw = blockIdx.x * blockDim.x + threadIdx.x, n1 = blockIdx.y;
-    if (iw >= a.ne) return;
-    double2 s = make_double2(0.0, 0.0);
-    const double wx = a.fmin - a.ekq[n1] + (iw - 1) * a.fstep;
-    const double2* num = t.num + (long)n1 * a.nf;
-    for (int f = 0; f < a.nf; ++f) {
-        const double2 coh = t.coh[f];
-        const double2 q = gc_div(num[f], make_double2(__dsub_rn(wx, coh.x), 0 - coh.y));
-        s = cadd(s, make_double2(0.0 - q.x, 0.0 - q.y));
+// The contraction's partial sums P[plane][slot][row][2] of the R planes (both sums:
+// RW, RS) and of the A planes (the first: AW); partial row i belongs to band order[i]
+// (or i).
+struct FfPartials {
+    int nR, nA, slotsR, slotsA;
+    const int* planes;  // the R planes' frequencies, then the A planes'
+    const double2 *PR, *PA;
+    double2 *RW, *RS, *AW;
+    const int* order;
+};
+// One plane of row i into the tables [nb][nf], by one warp: lane 4g + c takes component c
+// (RW re, RW im, RS re, RS im) of slots g, g+8, .. in order, so that the four lanes of a
+// slot read its 32-byte (RW, RS) record as one sector, then three shuffle levels add the
+// eight slot groups (fixed order: deterministic).  GB300's FP64 pipe retires one warp
+// instruction per 64 cycles per sub-partition: this takes slots/8 + 3 FP64 adds per warp.
+FK_DEV void ff_row_plane(const FfPartials& q, int nb, int nf, int i, int n1, int b, int lane) {
+    const bool isR = b < q.nR;
+    const int g = lane >> 2, comp = lane & 3, ns = isR ? q.slotsR : q.slotsA;
+    const double2* P = isR ? q.PR + (long)b * ns * nb * 2 : q.PA + (long)(b - q.nR) * ns * nb * 2;
+    const double* p = (const double*)(P + (long)i * 2) + comp;
+    const long sstride = 4L * nb;  // doubles per slot
+    double v = 0.0;
+    for (int s0 = g; s0 < ns; s0 += 64) {
+        double a[8];  // eight loads in flight; clamped indices, +0.0 past the end (exact)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a[j] = p[(long)min(s0 + 8 * j, ns - 1) * sstride];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v = __dadd_rn(v, s0 + 8 * j < ns ? a[j] : 0.0);
     }
-    a.SD[(long)iw * a.nb + n1] = s;
+#pragma unroll
+    for (int off = 4; off < 32; off <<= 1) v = __dadd_rn(v, __shfl_xor_sync(0xffffffffu, v, off));
+    if (lane >= 4) return;
+    const long at = (long)n1 * nf + q.planes[b];
+    if (comp < 2) ((double*)((isR ? q.RW : q.AW) + at))[comp] = v;
+    else if (isR) ((double*)(q.RS + at))[comp - 2] = v;
+}
+
+// FP64: the reference's operations per term (GPUComplex_divide).  The frequencies of one
+// iw go to the lanes of a group (the least power of two that holds them, at most a
+// warp), so that a warp's FP64 instructions serve 32 terms.
+FK_DEV void ff_schdi64(const EpiArgs& a, const SchdiTab& t, int n1, int tid, int threads) {
+    int gl = 1;
+    while (gl < 32 && gl < a.nf) gl <<= 1;
+    const int l = tid & (gl - 1), groups = threads / gl;
+    const double2* num = t.num + (long)n1 * a.nf;
+    for (int w0 = 0; w0 < a.ne; w0 += groups) {  // whole warps stay in the loop
+        const int iw = w0 + tid / gl;
+        double2 s = make_double2(0.0, 0.0);
+        if (iw < a.ne) {
+            const double wx = a.fmin - a.ekq[n1] + (iw - 1) * a.fstep;
+            for (int f = l; f < a.nf; f += gl) {
+                const double2 coh = t.coh[f];
+                const double2 q = gc_div(num[f], make_double2(__dsub_rn(wx, coh.x), 0 - coh.y));
+                s = cadd(s, make_double2(0.0 - q.x, 0.0 - q.y));
+            }
+        }
+        for (int off = gl >> 1; off > 0; off >>= 1) {
+            s.x = __dadd_rn(s.x, __shfl_xor_sync(0xffffffffu, s.x, off));
+            s.y = __dadd_rn(s.y, __shfl_xor_sync(0xffffffffu, s.y, off));
+        }
+        if (iw < a.ne && l == 0) a.SD[(long)iw * a.nb + n1] = s;
+    }
 }
 
 // Mixed: the same sum in FP32.  wx - coh.re = (wx_hi - coh_hi) + (wx_lo - coh_lo):
 // the first difference is exact when the two are close (Sterbenz), so the
 // denominator keeps full relative accuracy where it is small; terms are added
 // in FP32 over 32 frequencies, then into a float-float (TwoSum) accumulator.
-__global__ void ff_schdi32_kernel(EpiArgs a, SchdiTab t) {
-    const int iw = blockIdx.x * blockDim.x + threadIdx.x, n1 = blockIdx.y;
-    if (iw >= a.ne) return;
+FK_DEV void ff_schdi32(const EpiArgs& a, const SchdiTab& t, int n1, int iw) {
     const double wx = a.fmin - a.ekq[n1] + (iw - 1) * a.fstep;
     const float wh = f64_to_f32_bits(wx), wl = f64_to_f32_bits(wx - (double)wh);
     const float4* tab = t.f32 + (long)n1 * a.nf;
@@ -173,30 +179,43 @@ __global__ void ff_schdi32_kernel(EpiArgs a, SchdiTab t) {
     a.SD[(long)iw * a.nb + n1] = make_double2((double)ar.hi + (double)ar.lo, (double)ai.hi + (double)ai.lo);
 }
 
-FK_DEV void bsum(double2& v, double2* sm) {
-    for (int off = 16; off > 0; off >>= 1) {
-        v.x += __shfl_down_sync(0xffffffffu, v.x, off);
-        v.y += __shfl_down_sync(0xffffffffu, v.y, off);
+// One band per block: the rows of every plane (a warp per plane), the numerators of its
+// schDi sums, the sums.  Bound: FP64 instructions and the round trips between the steps;
+// as four launches (rows of R, rows of A, numerators, sums) these took 43 us at
+// 512 x 4096 x 512 x 15 mixed with a gap behind each, now 35 us.
+constexpr int BANDS_THREADS = 256;
+__global__ void __launch_bounds__(BANDS_THREADS) ff_bands_kernel(EpiArgs a, SchdiTab t, FfPartials q) {
+    const int i = blockIdx.x, tid = threadIdx.x, n1 = q.order ? q.order[i] : i;
+    for (int b = tid >> 5; b < q.nR + q.nA; b += BANDS_THREADS / 32) ff_row_plane(q, a.nb, a.nf, i, n1, b, tid & 31);
+    __syncthreads();
+    for (int f = tid; f < a.nf; f += BANDS_THREADS) {
+        const double2 num = cmul(make_double2(0.0, a.pref[f]), schdt_of(a, n1, f));
+        t.num[(long)n1 * a.nf + f] = num;
+        if (t.f32)
+            t.f32[(long)n1 * a.nf + f] =
+                make_float4(f64_to_f32_bits(num.x), f64_to_f32_bits(num.y), f64_to_f32_bits(0.0 - t.coh[f].y), 0.f);
     }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     __syncthreads();
-    if (lane == 0) sm[warp] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double2 s = make_double2(0.0, 0.0);
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s = cadd(s, sm[w]);
-        v = s;
+    if (t.f32) {
+        for (int iw = tid; iw < a.ne; iw += BANDS_THREADS) ff_schdi32(a, t, n1, iw);
+    } else {
+        ff_schdi64(a, t, n1, tid, BANDS_THREADS);
     }
 }
 
-// One block per output iw (blockIdx.x < ne) plus one block for the
-// iw-independent scalars (blockIdx.x == ne).
-__global__ void ff_epilogue_kernel(EpiArgs a) {
-    __shared__ double2 sm[32];
-    const int tid = threadIdx.x, iw = blockIdx.x;
+// One block per output iw (blockIdx.x < ne) plus one block for the iw-independent
+// scalars (blockIdx.x == ne); the schDt_matrix output is copied by all of them.  The
+// four complex sums over the bands are added together: every thread's eight parts go to
+// shared memory, and warp w adds part w, 13 FP64 instructions (one block-wide shuffle
+// sum after another took 28 us for 11 blocks, now 11 us).
+constexpr int EPI_THREADS = 256;
+__global__ void __launch_bounds__(EPI_THREADS) ff_epilogue_kernel(EpiArgs a) {
+    __shared__ double sm[8][EPI_THREADS], tot[8], lastv[2];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, iw = blockIdx.x;
     // iw-independent sums, computed redundantly per block (tiny)
-    double2 achs = make_double2(0, 0), asx = achs, cor = achs;
-    for (int n1 = tid; n1 < a.nb; n1 += blockDim.x) {
+    double2 achs = make_double2(0, 0), asx = achs, cor = achs, achd = achs;
+    for (int n1 = tid; n1 < a.nb; n1 += EPI_THREADS) {
+        if (iw < a.ne) achd = cadd(achd, a.SD[(long)iw * a.nb + n1]);
         achs = cadd(achs, a.RW[(long)n1 * a.nf + 1]);
         const FactRow fr = a.fact[n1];
         if (n1 < a.nv) {
@@ -212,20 +231,13 @@ __global__ void ff_epilogue_kernel(EpiArgs a) {
             cor = cadd(cor, v);
         }
     }
-    bsum(achs, sm);
-    bsum(asx, sm);
-    bsum(cor, sm);
-    if (iw == a.ne) {
-        if (tid == 0) a.out[0] = cscale(achs, -0.5);
-        // schDt_matrix output
-        for (long i = tid; i < (long)a.nb * a.nf; i += blockDim.x)
-            a.out[1 + 4L * a.ne + i] = (a.flags & FK_FF_SCHDT_GEMM) ? a.RS[i] : make_double2(0.0, 0.0);
-        return;
-    }
-    double2 achd = make_double2(0, 0);
-    for (int n1 = tid; n1 < a.nb; n1 += blockDim.x) achd = cadd(achd, a.SD[(long)iw * a.nb + n1]);
-    bsum(achd, sm);
-    if (tid == 0) {
+    const double part[8] = {achs.x, achs.y, asx.x, asx.y, cor.x, cor.y, achd.x, achd.y};
+#pragma unroll
+    for (int w = 0; w < 8; ++w) sm[w][tid] = part[w];
+    // schDt_matrix output
+    for (long i = (long)iw * EPI_THREADS + tid; i < (long)a.nb * a.nf; i += (long)(a.ne + 1) * EPI_THREADS)
+        a.out[1 + 4L * a.ne + i] = (a.flags & FK_FF_SCHDT_GEMM) ? a.RS[i] : make_double2(0.0, 0.0);
+    if (tid == EPI_THREADS - 1 && iw < a.ne) {
         // sch2Di after achDtemp_Kernel holds the value of its last (n1, ifreq)
         // iteration, which achDtemp_cor_Kernel adds once per band (:191-192, :241).
         double2 last = make_double2(0.0, 0.0);
@@ -241,14 +253,33 @@ __global__ void ff_epilogue_kernel(EpiArgs a) {
             intfact = -log(intfact);
             last = csub(make_double2(0.0, 0.0), cscale(cmul(make_double2(0.0, a.pref_zb), avg), intfact));
         }
-        const int ne = a.ne;
-        double2 asx_iw = asx;
-        if (!(a.flags & FK_FF_SPLIT_ACHD)) asx_iw = cadd(asx_iw, achd);  // ffKernel.cpp:495
-        a.out[1 + iw] = asx_iw;
-        a.out[1 + ne + iw] = (a.flags & FK_FF_SPLIT_ACHD) ? achd : make_double2(0.0, 0.0);
-        a.out[1 + 2 * ne + iw] = cor;
-        a.out[1 + 3 * ne + iw] = cscale(last, (double)a.nb);
+        lastv[0] = last.x;
+        lastv[1] = last.y;
     }
+    __syncthreads();
+    double v = sm[warp][lane];
+#pragma unroll
+    for (int j = 1; j < EPI_THREADS / 32; ++j) v = __dadd_rn(v, sm[warp][lane + 32 * j]);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v = __dadd_rn(v, __shfl_down_sync(0xffffffffu, v, off));
+    if (lane == 0) tot[warp] = v;
+    __syncthreads();
+    if (tid != 0) return;
+    achs = make_double2(tot[0], tot[1]);
+    asx = make_double2(tot[2], tot[3]);
+    cor = make_double2(tot[4], tot[5]);
+    achd = make_double2(tot[6], tot[7]);
+    if (iw == a.ne) {
+        a.out[0] = cscale(achs, -0.5);
+        return;
+    }
+    const int ne = a.ne;
+    double2 asx_iw = asx;
+    if (!(a.flags & FK_FF_SPLIT_ACHD)) asx_iw = cadd(asx_iw, achd);  // ffKernel.cpp:495
+    a.out[1 + iw] = asx_iw;
+    a.out[1 + ne + iw] = (a.flags & FK_FF_SPLIT_ACHD) ? achd : make_double2(0.0, 0.0);
+    a.out[1 + 2 * ne + iw] = cor;
+    a.out[1 + 3 * ne + iw] = cscale(make_double2(lastv[0], lastv[1]), (double)a.nb);
 }
 
 // compute_fact, FFKer_cori/ffKernel.cpp:30-78 (host copy; the oracle holds
@@ -583,7 +614,16 @@ fk_status ff_run(Ctx& c, const FfDev& r, const FfHost& h, const FfPipe* pipe) {
     }
 
     phase_mark(c, 1);
-    ff_igp_kernel<<<ceil_div(r.ng, 128), 128, 0, st>>>(r.ng, r.nc, r.inv, r.indinv, igp);
+    EpiArgs ea{};
+    ea.nb = r.nb; ea.nv = r.nv; ea.nf = r.nf; ea.ne = r.ne;
+    ea.RW = RW; ea.RS = RS; ea.AW = AW; ea.fact = fact;
+    ea.ekq = r.ekq; ea.grid = r.grid; ea.pref = r.pref; ea.brd = r.brd;
+    ea.pref_zb = r.pref_zb; ea.fmin = r.fmin; ea.fstep = r.fstep; ea.occ = r.occ; ea.flags = r.flags;
+    const bool phys = (r.flags & FK_FF_PHYSICS) != 0;
+    ea.fminI = phys ? r.fmin : (double)(int)r.fmin;
+    ea.fstepI = phys ? r.fstep : (double)(int)r.fstep;
+    ea.SD = SD; ea.out = r.out;
+    ff_setup_kernel<<<ceil_div(std::max(r.ng, r.nf), 128), 128, 0, st>>>(r.ng, r.nc, r.inv, r.indinv, igp, ea, stab);
     ++c.launches;
     phase_mark(c, 2);
     if (p.mixed) {
@@ -772,31 +812,10 @@ fk_status ff_run(Ctx& c, const FfDev& r, const FfHost& h, const FfPipe* pipe) {
         }
     }
     phase_mark(c, 3);
-    if (nR) {
-        ff_rows_kernel<<<dim3(ceil_div(r.nb, 4), nR), 128, 0, st>>>(r.nb, r.nf, nR, (int)slots, planes, PR, RW, RS,
-                                                                     order);
-        ++c.launches;
-    }
-    if (nA) {
-        // (rows outside a plane's tiles give values no band reads)
-        ff_rows_kernel<<<dim3(ceil_div(r.nb, 4), nA), 128, 0, st>>>(r.nb, r.nf, nA, (int)slotsA, planes + nR, PA, AW,
-                                                                     nullptr, order);
-        ++c.launches;
-    }
-    EpiArgs ea{};
-    ea.nb = r.nb; ea.nv = r.nv; ea.nf = r.nf; ea.ne = r.ne;
-    ea.RW = RW; ea.RS = RS; ea.AW = AW; ea.fact = fact;
-    ea.ekq = r.ekq; ea.grid = r.grid; ea.pref = r.pref; ea.brd = r.brd;
-    ea.pref_zb = r.pref_zb; ea.fmin = r.fmin; ea.fstep = r.fstep; ea.occ = r.occ; ea.flags = r.flags;
-    const bool phys = (r.flags & FK_FF_PHYSICS) != 0;
-    ea.fminI = phys ? r.fmin : (double)(int)r.fmin;
-    ea.fstepI = phys ? r.fstep : (double)(int)r.fstep;
-    ea.SD = SD; ea.out = r.out;
-    ff_schdi_tables_kernel<<<dim3(ceil_div(r.nf, 128), r.nb), 128, 0, st>>>(ea, stab);
-    if (p.mixed) ff_schdi32_kernel<<<dim3(ceil_div(r.ne, 128), r.nb), 128, 0, st>>>(ea, stab);
-    else ff_schdi_kernel<<<dim3(ceil_div(r.ne, 128), r.nb), 128, 0, st>>>(ea, stab);
-    c.launches += 1;
-    ff_epilogue_kernel<<<r.ne + 1, 256, 0, st>>>(ea);
+    // (A planes: rows outside a plane's tiles give values no band reads)
+    const FfPartials fp{nR, nA, (int)slots, (int)slotsA, planes, PR, PA, RW, RS, AW, order};
+    ff_bands_kernel<<<r.nb, BANDS_THREADS, 0, st>>>(ea, stab, fp);
+    ff_epilogue_kernel<<<r.ne + 1, EPI_THREADS, 0, st>>>(ea);
     c.launches += 2;
     phase_mark(c, 4);
     e = cudaGetLastError();
