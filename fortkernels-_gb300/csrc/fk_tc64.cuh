@@ -591,42 +591,66 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) contract
             const int n0 = x.nt * BN, ncol = min(BN, t.N - n0);
             const bool both = EPI == EPI_FF && x.pl < t.tab.n2;
             double2 g[3] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+            // GPP: eight columns per turn of a rolled loop, H moving down by eight, and g[k] the sum
+            // of class (t0 + k) % 3 of the columns.  Unrolled over the 64 columns the code runs once
+            // per unit and its bound was fetching it: 64 x 777 x 7 220 -> 217 us, 512 x 32768 x 20
+            // 409 -> 400 us.  FF (twice the arithmetic per column) stays unrolled: rolled, 40 x 640 x
+            // 48 x 6 took 130 us instead of 127.
+            constexpr int TURN = EPI == EPI_FF ? BN : 8;
+#pragma unroll 1
+            for (int t0 = 0; t0 < BN; t0 += TURN) {
 #pragma unroll
-            for (int j0 = 0; j0 < BN; j0 += 8) {
-                float c5[8], c6[8];
-                tc::tmem_ld8(tl + 256u + j0, c5);
-                tc::tmem_ld8(tl + 384u + j0, c6);
-                tc::tmem_ld_wait();
-                if (j0 + 8 >= BN) {
-                    release(2);
-                    release(3);
-                }
-#pragma unroll
-                for (int jb = 0; jb < 8; jb += 4) {
-                    double2 w1[4], w2[4];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int n = n0 + min(j0 + jb + j, ncol - 1), h = EPI == EPI_GPP ? n / 3 : n;
-                        w1[j] = t.W1[(long)h * t.M + mc];
-                        if (EPI == EPI_FF) w2[j] = both ? t.W2[(long)h * t.M + mc] : make_double2(0.0, 0.0);
+                for (int q = 0; q < TURN; q += 8) {
+                    const int j0 = t0 + q;
+                    float c5[8], c6[8];
+                    tc::tmem_ld8(tl + 256u + j0, c5);
+                    tc::tmem_ld8(tl + 384u + j0, c6);
+                    tc::tmem_ld_wait();
+                    if (j0 + 8 >= BN) {
+                        release(2);
+                        release(3);
                     }
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int col = j0 + jb + j;
-                        if (col >= ncol) continue;  // warp-uniform
-                        const double s = fixed_to_double(H[col], fmaf(c6[jb + j], 0x1p-18f, c5[jb + j] * 0x1p-9f),
-                                                         ea + ebp[col] - 46);
-                        // half 0: w * s, half 1: w * (i s)
-                        const int gi = EPI == EPI_GPP ? col % 3 : 0;
-                        const double sr = half ? -s : s;
-                        g[gi].x = fma(half ? w1[j].y : w1[j].x, sr, g[gi].x);
-                        g[gi].y = fma(half ? w1[j].x : w1[j].y, s, g[gi].y);
-                        if (EPI == EPI_FF && both) {
-                            g[1].x = fma(half ? w2[j].y : w2[j].x, sr, g[1].x);
-                            g[1].y = fma(half ? w2[j].x : w2[j].y, s, g[1].y);
+                    for (int jb = 0; jb < 8; jb += 4) {
+                        if (EPI != EPI_FF && j0 + jb >= ncol) continue;  // warp-uniform
+                        double2 w1[4], w2[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const int col = min(j0 + jb + j, ncol - 1), n = n0 + col, h = EPI == EPI_GPP ? n / 3 : n;
+                            w1[j] = t.W1[(long)h * t.M + mc];
+                            if (EPI == EPI_FF) w2[j] = both ? t.W2[(long)h * t.M + mc] : make_double2(0.0, 0.0);
+                        }
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            if (j0 + jb + j >= ncol) continue;  // warp-uniform
+                            const double s = fixed_to_double(
+                                H[q + jb + j], fmaf(c6[jb + j], 0x1p-18f, c5[jb + j] * 0x1p-9f), ea + ebp[j0 + jb + j] - 46);
+                            // half 0: w * s, half 1: w * (i s)
+                            const int gi = EPI == EPI_GPP ? (jb + j) % 3 : 0;
+                            const double sr = half ? -s : s;
+                            g[gi].x = fma(half ? w1[j].y : w1[j].x, sr, g[gi].x);
+                            g[gi].y = fma(half ? w1[j].x : w1[j].y, s, g[gi].y);
+                            if (EPI == EPI_FF && both) {
+                                g[1].x = fma(half ? w2[j].y : w2[j].x, sr, g[1].x);
+                                g[1].y = fma(half ? w2[j].x : w2[j].y, s, g[1].y);
+                            }
                         }
                     }
                 }
+#pragma unroll
+                for (int j = 0; j + TURN < BN; ++j) H[j] = H[j + TURN];
+                if (EPI == EPI_GPP) {  // (t0 + 8) % 3 = (t0 + 2) % 3
+                    const double2 g0 = g[0], g1 = g[1];
+                    g[0] = g[2];
+                    g[1] = g0;
+                    g[2] = g1;
+                }
+            }
+            if (EPI == EPI_GPP) {  // back to class k % 3 (64 % 3 = 1)
+                const double2 g2 = g[2];
+                g[2] = g[1];
+                g[1] = g[0];
+                g[0] = g2;
             }
             if (m < t.M) {
                 double2* out = t.P + ((((long)x.pl * t.KS + x.ks) * t.NT + x.nt) * 2 + half) * (long)t.M * t.G + (long)m * t.G;
