@@ -1892,19 +1892,22 @@ struct RealCarryArgs {
 // later block at the same offset.  E of an element thus depends on its own
 // mask and values and on that first later set time only: one thread per
 // element, looking ahead through the masks of the later blocks (usually one).
+// Bound: FP64 instructions (64 cycles each).  The usual element has one source per iw
+// that lasts one time, and needs none; signs and counts are formed in FP32.
+// 512 x 32768 x 20 mixed: 30 -> 13 us.
 template <int IMG>
 __global__ void real_carry_kernel(RealCarryArgs a) {
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long)a.ng * a.nc) return;
     const int my_igp = (int)(t / a.nc), g = (int)(t % a.nc);
     auto put = [&](int iw, int gg, double v) {
-        const double s = (gg & 1) ? 0.0 - v : v;
         if (IMG) {
             const int nt = my_igp / GPP_COLS, row = (my_igp % GPP_COLS) * 3 + iw;
+            const float f = f64_to_f32_bits(v);
             tcx::bimg_store_part<64>(a.img + (long)nt * a.kstages * tcx::Cfg<64>::B_BYTES, row, gg >> 1, gg & 1,
-                                     f64_to_f32_bits(s));
+                                     (gg & 1) ? 0.f - f : f);
         } else {
-            a.D64[((long)my_igp * 3 + iw) * 2 * a.K2 + gg] = s;
+            a.D64[((long)my_igp * 3 + iw) * 2 * a.K2 + gg] = (gg & 1) ? 0.0 - v : v;
         }
     };
     const uint8_t* mrow = a.mask + (long)my_igp * a.nc;
@@ -1928,6 +1931,7 @@ __global__ void real_carry_kernel(RealCarryArgs a) {
                 }
             }
             auto upto = [](int T, int iw) { return (T - iw + 2) / 3; };  // #{t < T : t = iw mod 3}
+            int touched = 0;
 #pragma unroll
             for (int ws = 0; ws < 3; ++ws) {
                 if (!((m >> ws) & 1)) continue;
@@ -1936,7 +1940,10 @@ __global__ void real_carry_kernel(RealCarryArgs a) {
 #pragma unroll
                 for (int iw = 0; iw < 3; ++iw) {
                     const int n = upto(t1, iw) - upto(t0, iw);
-                    if (n) e[iw] = __fma_rn((double)n, dv[ws], e[iw]);
+                    // e[iw] still 0: 1 * D + 0 is D, and the first term needs no addition
+                    if (n == 1 && !(touched >> iw & 1)) e[iw] = dv[ws];
+                    else if (n) e[iw] = __fma_rn(f32_to_f64_bits((float)n), dv[ws], e[iw]);
+                    touched |= (n ? 1 : 0) << iw;
                 }
             }
         }
