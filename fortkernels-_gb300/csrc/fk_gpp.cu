@@ -1785,7 +1785,9 @@ __device__ __noinline__ RealTerm real_term_rare(double wxt, double w, double ep)
     return t;
 }
 
-__global__ void __launch_bounds__(PREP_THREADS) real_prep_mixed_kernel(RealPrepArgs p) {
+// The chunks make one wave of four blocks per SM (make_real_plan): 64 registers.  At 78,
+// three blocks, the wave was not one: 44 us at 512 x 32768 x 20, now 32 (the call 129 -> 117).
+__global__ void __launch_bounds__(PREP_THREADS, 4) real_prep_mixed_kernel(RealPrepArgs p) {
     __shared__ double2 sm[8 * NVC * 6];
     const int my_igp = blockIdx.y, ch = blockIdx.x, tid = threadIdx.x;
     const int igp = p.igp[my_igp];
