@@ -88,8 +88,6 @@ FK_DEV double2 ordered_sum_g(const double2* x, long stride, int n) {
     return s;
 }
 FK_DEV double2 ordered_sum(const double2* x, long stride, int n) { return ordered_sum_g<8>(x, stride, n); }
-// The same with the loads of up to 16 terms in flight.
-FK_DEV double2 ordered_sum16(const double2* x, long stride, int n) { return ordered_sum_g<16>(x, stride, n); }
 
 // --------------------------------------------- compensated FP32 accumulation
 // float-float (hi, lo) accumulator updated with Knuth's TwoSum: exact sum of

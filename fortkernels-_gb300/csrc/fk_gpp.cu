@@ -61,7 +61,7 @@ struct PrepArgs {
     int ch0;     // first chunk of this launch (blockIdx.x counts from it)
     // half-sum mode (FK_GPP_HALF_SUM)
     const double2* aqsm;  // full [nb][nc] (half sum); the weights' source (set-up, below)
-    const int* brk;       // [ng]: first ig whose |Omega2| < 1e-6 (the flag bands stop there)
+    const int* brk;       // [ng][HALF_CHUNKS]: first ig whose |Omega2| < 1e-6 in each chunk (half_brk: the flag bands stop there)
     // Set-up folded into the first pass (setup != 0): the column map is computed
     // from inv/indinv rather than read from igp, and the first chunk of each
     // column writes igp/acol, the epilogue weights W (mixed) and, in the last
@@ -449,34 +449,42 @@ FK_DEV double2 half_sch(double wxt, double2 wt, double2 eps) {
 // ig takes part in column igp's noflag sum (the reference program's 512-wide blocks)
 FK_DEV bool half_member(int ig, int igp) { return ig < igp - 1 && (ig & 511) != 511; }
 
-// brk[my_igp] = the first ig < igp with |wtilde^2 * I_eps| < to1 (brk starts above
-// every igp).  The test runs in FP32 on |Omega2|^2 against to1^2; inside a relative
-// guard band of 1e-5 around it (the FP32 error is ~1e-7) the FP64 test decides, so
-// every decision is the FP64 one.
+// The first ig < igp with |wtilde^2 * I_eps| < to1 is found chunk by chunk (half_break: the
+// smallest hit of one chunk of the column, or a value above every igp).  The test runs in FP32
+// on |Omega2|^2 against to1^2; inside a relative guard band of 1e-5 around it (the FP32 error
+// is ~1e-7) the FP64 test decides, so every decision is the FP64 one.
+constexpr int HALF_CHUNKS = 64;
 __device__ __noinline__ bool half_break64(double2 w, double2 ep) {
     const double2 o = cmul(cmul(w, w), ep);
     return hypot(o.x, o.y) < 1e-6;
 }
-__global__ void half_break_kernel(int ng, int nc, const int* igpm, const double2* eps, const double2* wt, int* brk) {
-    const int my_igp = blockIdx.y;
-    const int igp = igpm[my_igp];
-    if (igp <= 0) return;  // block-uniform
-    // warps walk [0, igp) together; the first hit of each warp goes to one atomicMin
-    const int stride = gridDim.x * blockDim.x;
-    for (int base = blockIdx.x * blockDim.x; base < igp; base += stride) {
-        const int ig = base + threadIdx.x;
-        int first = 0x7fffffff;
-        if (ig < igp) {
-            const double2 w64 = wt[(long)my_igp * nc + ig], e64 = eps[(long)my_igp * nc + ig];
-            const float2 w = c64_to_f32(w64), o = cmulf(cmulf(w, w), c64_to_f32(e64));
-            const float o2 = o.x * o.x + o.y * o.y;
-            bool hit = o2 < 1e-12f;
-            if (!(o2 < 1e30f) || fabsf(o2 - 1e-12f) <= 1e-12f * GUARD || !(o2 > 1e-36f)) hit = half_break64(w64, e64);
-            if (hit) first = ig;
-        }
-        first = __reduce_min_sync(0xffffffffu, first);
-        if ((threadIdx.x & 31) == 0 && first != 0x7fffffff) atomicMin(&brk[my_igp], first);
+// One block; every thread calls it.
+FK_DEV void half_break(int nc, int igp, int chunk, const double2* wt, const double2* eps, int* out) {
+    const int span = ceil_div(nc, HALF_CHUNKS), g1 = min(igp, (chunk + 1) * span);
+    int first = 0x7fffffff;
+    for (int ig = chunk * span + threadIdx.x; ig < g1; ig += blockDim.x) {
+        const double2 w64 = wt[ig], e64 = eps[ig];
+        const float2 w = c64_to_f32(w64), o = cmulf(cmulf(w, w), c64_to_f32(e64));
+        const float o2 = o.x * o.x + o.y * o.y;
+        bool hit = o2 < 1e-12f;
+        if (!(o2 < 1e30f) || fabsf(o2 - 1e-12f) <= 1e-12f * GUARD || !(o2 > 1e-36f)) hit = half_break64(w64, e64);
+        if (hit) first = min(first, ig);
     }
+    __shared__ int sm[8];
+    first = __reduce_min_sync(0xffffffffu, first);
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = first;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) first = min(first, sm[w]);
+        *out = first;
+    }
+}
+// The first hit of column my_igp (whole warps call it).
+FK_DEV int half_brk(const int* brk, int my_igp) {
+    const int* b = brk + (long)my_igp * HALF_CHUNKS;
+    int v = 0x7fffffff;
+    for (int i = threadIdx.x & 31; i < HALF_CHUNKS; i += 32) v = min(v, b[i]);
+    return __reduce_min_sync(0xffffffffu, v);
 }
 
 // What the half and the real-valued sum need before their preps, in one launch: the
@@ -485,7 +493,7 @@ __global__ void half_break_kernel(int ng, int nc, const int* igpm, const double2
 // sch(igp) of the columns on a block edge (igp % 512 == 0, else 0); the real-valued
 // sum's aqsmtemp columns as complex (value, 0), [nb][ng] (the weights' source).
 // As separate launches these were four to six kernels of 3 to 5 us, with a gap of 2 to
-// 3 us behind each.  512 x 32768 x 20: half sum 199 -> 183 us, real-valued 163 -> 146 us.
+// 3 us behind each.  512 x 32768 x 20: half sum 199 -> 175 us, real-valued 163 -> 146 us.
 struct SetupArgs {
     int nb, nv, nc, ng;
     const int *inv, *indinv;
@@ -508,7 +516,15 @@ __host__ __device__ inline int setup_row_blocks(int nb) { return (nb + SETUP_THR
 __global__ void __launch_bounds__(SETUP_THREADS) setup_kernel(SetupArgs a) {
     const int nr = setup_row_blocks(a.nb), b = blockIdx.x, tid = threadIdx.x;
     if (b >= nr * a.ng) {
-        const int s = b - nr * a.ng;
+        int s = b - nr * a.ng;
+        if (a.brk) {
+            if (s < HALF_CHUNKS * a.ng) {
+                const int h = s / HALF_CHUNKS, c = s % HALF_CHUNKS;
+                half_break(a.nc, gpp_igp_of(h, a.nc, a.inv, a.indinv), c, a.wt + (long)h * a.nc, a.eps + (long)h * a.nc, a.brk + s);
+                return;
+            }
+            s -= HALF_CHUNKS * a.ng;
+        }
         tcx::img_pad_stage<64>(a.img, s / a.NT, s % a.NT, a.NT, a.kstages, a.ng, GPP_COLS, a.K);
         return;
     }
@@ -518,7 +534,6 @@ __global__ void __launch_bounds__(SETUP_THREADS) setup_kernel(SetupArgs a) {
         if (tid == 0) {
             a.igp[h] = g;
             a.acol[h] = g < 0 ? -1 : (a.ac ? h : g);
-            if (a.brk) a.brk[h] = 0x7f7f7f7f;  // above every igp
             if (h == 0) {
                 *a.counter = 0;
                 if (a.err) *a.err = 0;
@@ -541,7 +556,8 @@ __global__ void __launch_bounds__(SETUP_THREADS) setup_kernel(SetupArgs a) {
         a.W[(long)h * (a.nb - a.nv) + n - a.nv] = g >= 0 ? tcx::weight_w1(am, 0.5 * a.vcoul[g]) : make_float2(0.f, 0.f);
 }
 inline void launch_setup(const SetupArgs& a, cudaStream_t st) {
-    setup_kernel<<<setup_row_blocks(a.nb) * a.ng + (a.img ? a.kstages * a.NT : 0), SETUP_THREADS, 0, st>>>(a);
+    const int blocks = setup_row_blocks(a.nb) * a.ng + (a.brk ? HALF_CHUNKS * a.ng : 0) + (a.img ? a.kstages * a.NT : 0);
+    setup_kernel<<<blocks, SETUP_THREADS, 0, st>>>(a);
 }
 
 // The flag-band terms of one (ig, iw): sch and ssx of flagOCC_solver (gppsum == 1)
@@ -573,7 +589,7 @@ __global__ void __launch_bounds__(PREP_THREADS) prep_half_kernel(PrepArgs p) {
     const int my_igp = blockIdx.y, ch = p.ch0 + blockIdx.x, tid = threadIdx.x;
     const int igp = p.igp[my_igp];
     const int nflag = min(NVC, p.nv - p.n1base);
-    const int stop = igp < 0 ? 0 : min(igp, p.brk[my_igp]);
+    const int stop = igp < 0 ? 0 : min(igp, half_brk(p.brk, my_igp));
     double2 acc[NVC * 12];
 #pragma unroll
     for (int i = 0; i < NVC * 12; ++i) acc[i] = make_double2(0.0, 0.0);
@@ -637,7 +653,7 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) prep_half_mixed_kernel(PrepAr
     const int my_igp = blockIdx.y, ch = p.ch0 + blockIdx.x, tid = threadIdx.x;
     const int igp = p.igp[my_igp];
     const int nflag = min(NVC, p.nv - p.n1base);
-    const int stop = igp < 0 ? 0 : min(igp, p.brk[my_igp]);
+    const int stop = igp < 0 ? 0 : min(igp, half_brk(p.brk, my_igp));
     const float limitone = 250000.0f, limittwo = 0.25f, to1 = 1e-6f, to1sq = 1e-12f;
     float2 acc[NVC * 12];
 #pragma unroll
@@ -1203,12 +1219,12 @@ FK_DEV void rows_flag_block(const RowsArgs& ra, int n1, int c, int tid) {
         // half sum, occupied band: weight * (cm S1 + conj(cm S2)) per column
         const int kind = c / 3, r = ((c % 3) * 2 + kind) * 2;
         const double occ = 1.0;
-        for (int h = tid; h < ng; h += T) {
+        for (long i = tid; i < (long)nch * ng; i += T) {  // item i = (chunk i / ng, column i % ng)
+            const long k = i / ng, h = i - k * ng;
             const int g = igp[h];
             if (g < 0) continue;
-            const double2 s1 = ordered_sum(F + ((long)n1 * ng + h) * 12 + r, (long)nv * ng * 12, nch);
-            const double2 s2 = ordered_sum(F + ((long)n1 * ng + h) * 12 + r + 1, (long)nv * ng * 12, nch);
-            const double2 cm = cconj(aqsm[(long)n1 * ldm + acol[h]]);
+            const double2* x = F + ((k * nv + n1) * ng + h) * 12 + r;
+            const double2 s1 = x[0], s2 = x[1], cm = cconj(aqsm[(long)n1 * ldm + acol[h]]);
             v = cadd(v, cscale(cadd(cmul(cm, s1), cconj(cmul(cm, s2))), kind ? occ * vcoul[g] : 0.5 * vcoul[g]));
         }
     } else if (ra.wf) {
@@ -1231,10 +1247,11 @@ FK_DEV void rows_flag_block(const RowsArgs& ra, int n1, int c, int tid) {
     } else {
         const int kind = c / 3, r = (c % 3) * 2 + kind;  // kind 0: sch, 1: ssx
         const double occ = 1.0;
-        for (int h = tid; h < ng; h += T) {
+        for (long i = tid; i < (long)nch * ng; i += T) {
+            const long k = i / ng, h = i - k * ng;
             const int g = igp[h];
             if (g < 0) continue;
-            const double2 sum = ordered_sum(F + ((long)n1 * ng + h) * 6 + r, (long)nv * ng * 6, nch);
+            const double2 sum = F[((k * nv + n1) * ng + h) * 6 + r];
             const double2 cm = cconj(aqsm[(long)n1 * ldm + acol[h]]);
             v = cadd(v, cscale(cmul(cm, sum), kind ? occ * vcoul[g] : 0.5 * vcoul[g]));
         }
@@ -1961,7 +1978,7 @@ __global__ void real_carry_kernel(RealCarryArgs a) {
 
 size_t gpp_workspace(const Ctx& c, const GppDev& r, bool pipelined) {
     Plan p = make_plan(c, r, 0, pipelined, gpp_pair(r, pipelined), gpp_fsch(r));
-    const size_t half = (r.flags & FK_GPP_HALF_SUM) ? p.bytesP + (size_t)r.ng * (4 + 3 * sizeof(double2)) + 768 : 0;
+    const size_t half = (r.flags & FK_GPP_HALF_SUM) ? p.bytesP + (size_t)r.ng * (4 * HALF_CHUNKS + 3 * sizeof(double2)) + 768 : 0;
     const size_t wf = (size_t)r.nv * r.ng * 2 * sizeof(double2);
     // the error estimate's column magnitudes, row norms and band bounds (when on)
     const size_t est = (c.est_on && p.mixed)
@@ -2029,7 +2046,7 @@ fk_status gpp_run_half(Ctx& c, const GppDev& r) {
     double2* P2 = p.bytesP ? (double2*)c.ws.take(p.bytesP) : nullptr;
     double2* rows = (double2*)c.ws.take(p.bytesRows);
     float2* W = p.bytesW ? (float2*)c.ws.take(p.bytesW) : nullptr;
-    int* brk = (int*)c.ws.take((size_t)r.ng * sizeof(int));
+    int* brk = (int*)c.ws.take((size_t)r.ng * HALF_CHUNKS * sizeof(int));
     double2* schd = (double2*)c.ws.take((size_t)r.ng * 3 * sizeof(double2));
     int* counter = (int*)c.ws.take(sizeof(int));
     tc64::Bufs zb{};
@@ -2049,9 +2066,7 @@ fk_status gpp_run_half(Ctx& c, const GppDev& r) {
     sa.NT = p.NT; sa.kstages = p.kstages; sa.K = r.nc;
     sa.aqsm = r.aqsm; sa.eps = r.eps; sa.wt = r.wt; sa.wx = r.wx; sa.brk = brk; sa.schd = schd;
     launch_setup(sa, st);
-    half_break_kernel<<<dim3(std::max(1, std::min(ceil_div(r.nc, 256), 64)), r.ng), 256, 0, st>>>(r.ng, r.nc, igp,
-                                                                                                 r.eps, r.wt, brk);
-    c.launches += 2;
+    ++c.launches;
     for (int pass = 0; pass < p.passes; ++pass) {
         PrepArgs a{r.nb, r.nv, r.nc, r.ng, r.aqsn, r.eps, r.wt, r.wx, igp, (pass == 0 && M > 0) ? D : nullptr,
                    p.kstages, F, p.nch, p.tile, pass * NVC, 0, r.aqsm, brk};
