@@ -344,19 +344,20 @@ struct FfPlan {
 constexpr size_t FF_ZGROUP_BYTES = (size_t)4 << 30;
 
 // k-slices for the persistent tensor-core kernel (see fk_gpp.cu)
-void ff_pick_split_tc(long tiles, int K, int workers, double unit, int& KS, int& kchunk) {
-    const int kst = ceil_div(K, tcx::BK), kmax = std::max(1, K / 256);
+void ff_pick_split_tc(long tiles, int K, int sms, int& KS, int& kchunk) {
+    const int kmax = std::max(1, K / 256);
+    int best = 1;
     double best_cost = 1e30;
     for (int ks = 1; ks <= std::min(kmax, 64); ++ks) {
-        const int ku = ceil_div(kst, ks);
-        const long waves = (tiles * ks + workers - 1) / workers;
-        const double cost = (double)waves * (ku + unit);
-        if (cost < best_cost * 0.999) {
-            best_cost = cost;
-            kchunk = ku * tcx::BK;
-        }
+        const long units = tiles * ks;
+        const long waves = (units + sms - 1) / sms;
+        const double eff = (double)units / (double)(waves * sms);
+        const double cost = (1.0 / eff) * (1.0 + 0.002 * ks);
+        if (cost < best_cost - 1e-9) { best_cost = cost; best = ks; }
+        if (eff > 0.92 && units >= sms) break;
     }
-    KS = ceil_div(K, kchunk);
+    kchunk = ((K + best - 1) / best + tcx::BK - 1) / tcx::BK * tcx::BK;
+    KS = (K + kchunk - 1) / kchunk;
 }
 
 constexpr int FF_PIPE_GROUPS = 8;  // copy groups of a pipelined request at most (events 0..7 of Ctx::pipe_ev)
@@ -430,7 +431,7 @@ FfPlan make_plan(const Ctx& c, const FfDev& r, const double* ekq_h, const double
         p.kstages = ceil_div(r.nc, tcx::BK);
         p.MT = ceil_div(r.nb, 2 * tcx::BM);
         p.NT = ceil_div(r.ng, p.BN);
-        ff_pick_split_tc((long)p.MT * p.NT * nplanes, r.nc, c.sms / 2, 4.0, p.KS, p.kchunk);
+        ff_pick_split_tc((long)p.MT * p.NT * nplanes, r.nc, c.sms / 2, p.KS, p.kchunk);
         const size_t bb = tcx::Cfg<64, true>::B_BYTES;
         p.bytesImgR = p.planesR.size() * (size_t)p.NT * p.kstages * bb;
         p.bytesImgA = p.planesA.size() * (size_t)p.NT * p.kstages * bb;
@@ -474,7 +475,7 @@ FfPlan make_plan(const Ctx& c, const FfDev& r, const double* ekq_h, const double
             ztiles += hi > lo ? (hi - 1) / tc64::BM - lo / tc64::BM + 1 : 0;
         }
         // k-slices for the one launch over all A planes' (row tile, n-tile) pairs
-        if (p.mixed) ff_pick_split_tc(std::max(1L, tiles) * p.NT, r.nc, c.sms, 14.0, p.KSa, p.kchunka);
+        if (p.mixed) ff_pick_split_tc(std::max(1L, tiles) * p.NT, r.nc, c.sms, p.KSa, p.kchunka);
         if (r.tc64) {
             const int all = std::max(1, (int)(p.planesR.size() + p.planesA.size())), pairs = c.sms / 2;
             const tc64::Plan one = tc64::make_plan(r.nb, r.ng, r.nc, 1, pairs);
