@@ -182,7 +182,8 @@ FK_DEV void ff_schdi32(const EpiArgs& a, const SchdiTab& t, int n1, int iw) {
 // One band per block: the rows of every plane (a warp per plane), the numerators of its
 // schDi sums, the sums.  Bound: FP64 instructions and the round trips between the steps;
 // as four launches (rows of R, rows of A, numerators, sums) these took 43 us at
-// 512 x 4096 x 512 x 15 mixed with a gap behind each, now 35 us.
+// 512 x 4096 x 512 x 15 mixed with a gap behind each, now 35 us (23 with the A planes'
+// partials of whole rows, make_plan).
 constexpr int BANDS_THREADS = 256;
 __global__ void __launch_bounds__(BANDS_THREADS) ff_bands_kernel(EpiArgs a, SchdiTab t, FfPartials q) {
     const int i = blockIdx.x, tid = threadIdx.x, n1 = q.order ? q.order[i] : i;
@@ -329,6 +330,7 @@ struct FfPlan {
     // it, contracted with KSa k-slices of kchunka.
     std::vector<int> order, aLo, aHi;
     int KSa = 0, kchunka = 0;
+    int slicea = 0;              // A planes: stages drained together at most (several such slices in a unit)
     bool mixed;
     size_t bytes, bytesImgR, bytesImgA, bytesW, bytesAimg;
     size_t bytesScale;  // mixed: 2^-k of every A image row and of every row of the converted planes
@@ -475,7 +477,26 @@ FfPlan make_plan(const Ctx& c, const FfDev& r, const double* ekq_h, const double
             ztiles += hi > lo ? (hi - 1) / tc64::BM - lo / tc64::BM + 1 : 0;
         }
         // k-slices for the one launch over all A planes' (row tile, n-tile) pairs
-        if (p.mixed) ff_pick_split_tc(std::max(1L, tiles) * p.NT, r.nc, c.sms, p.KSa, p.kchunka);
+        if (p.mixed) {
+            // A unit costs as much as 14 stages there (its weights, sums and stores): units of
+            // several slices where that gives the shorter waves, the slices still drained each
+            // by itself (group_stages; every FP32 sum is the same).  512 x 4096 x 512 x 15: seven
+            // slices in one unit, 129 -> 119 us; the bands kernel reads a seventh of the partials.
+            const long t = std::max(1L, tiles) * p.NT;
+            ff_pick_split_tc(t, r.nc, c.sms, p.KSa, p.kchunka);
+            const int slice = p.kchunka / tcx::BK, n = p.KSa;
+            double best = 1e30;
+            for (int m = 1; m <= n; ++m) {
+                const long waves = (t * ceil_div(n, m) + c.sms - 1) / c.sms;
+                const double cost = (double)waves * (std::min(m * slice, p.kstages) + 14);
+                if (cost < best * 0.999) {
+                    best = cost;
+                    p.kchunka = m * slice * tcx::BK;
+                }
+            }
+            p.KSa = ceil_div(r.nc, p.kchunka);
+            p.slicea = slice;
+        }
         if (r.tc64) {
             const int all = std::max(1, (int)(p.planesR.size() + p.planesA.size())), pairs = c.sms / 2;
             const tc64::Plan one = tc64::make_plan(r.nb, r.ng, r.nc, 1, pairs);
@@ -707,6 +728,7 @@ fk_status ff_run(Ctx& c, const FfDev& r, const FfHost& h, const FfPipe* pipe) {
                 t.c.batches = 1;
                 t.c.KS = p.KSa;
                 t.c.kchunk = p.kchunka;
+                t.group_stages = p.slicea;
                 auto k = tcx::tc_contract_planes_kernel<EPI_FF, 64, true>;
                 constexpr size_t smem = tcx::Cfg<64, true>::SMEM;
                 cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -140,6 +140,7 @@ struct TcArgs {
     long long wait_limit; // bound of the waits between roles, cycles (0 is allowed: any wait that
                           // is not satisfied on its first test gives up)
     int chunk_stages;     // k-stages accumulated in TMEM between drains (0: 1)
+    int group_stages;     // FF on single CTAs: drained groups do not cross multiples of this many stages of the unit (0: no bound)
     int ff_no_rs;         // FF: the unweighted sum (partial 1) is not needed; only the vcoul-weighted one
 };
 
@@ -384,6 +385,12 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
         k0 = ks * t.c.kchunk;
         k1 = min(t.c.K, k0 + t.c.kchunk);
     };
+    // the stage behind the group that starts at stage sg0
+    auto group_end = [&](const TcArgs& t, int sg0, int nst, int CH) {
+        int e = min(nst, sg0 + C::GRP * CH);
+        if (C::SL && !PAIR && t.group_stages) e = min(e, (sg0 / t.group_stages + 1) * t.group_stages);
+        return e;
+    };
     auto fail = [&](int code) {
         atomicOr(err, code);
         s_abort = 1;
@@ -434,7 +441,7 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
                 const int CH = t.chunk_stages > 0 ? t.chunk_stages : 1;
                 // a served request may carry a pre-split A image (its stages' A lands on fullB)
                 const bool ua = APRE || (Src::kTable && t.Aimg != nullptr);
-                for (int sg0 = 0; sg0 < nst && ok; sg0 += C::GRP * CH, ++grp) {
+                for (int sg0 = 0, sg1; sg0 < nst && ok; sg0 = sg1, ++grp) {
                     // a group: up to GRP chunks of CH stages, each into its own buffer of the slot
                     const int slot = grp % C::NSLOT;
                     const uint32_t bpar = ((grp / C::NSLOT) & 1) ^ 1;
@@ -442,7 +449,7 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
                                             : tc::mbar_wait(&accEmpty[slot], bpar, wait_limit);
                     if (!tc::warp_all(freed)) { fail(1); ok = false; break; }
                     tc::tc_fence_after();
-                    const int sg1 = min(nst, sg0 + C::GRP * CH);
+                    sg1 = group_end(t, sg0, nst, CH);
                     for (int st0 = sg0, b = slot * C::GRP; st0 < sg1 && ok; st0 += CH, ++b) {
                         // X, Y (two accumulators) or, SL, the one accumulator D = dX
                         const uint32_t dX = tmem + (uint32_t)(b * C::ACC_COLS), dY = dX + 2 * BN;
@@ -742,7 +749,8 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
             // added in registers with one round-to-nearest FP32 addition before the
             // weighted sums: half the arithmetic, waits and returns per chunk)
             for (int st0 = 0; st0 < nst; ++grp) {
-                const int npass = min(C::GRP, (nst - st0 + CH - 1) / CH);  // chunks in the group
+                // chunks in the group
+                const int npass = PAIR ? min(C::GRP, (nst - st0 + CH - 1) / CH) : (group_end(t, st0, nst, CH) - st0 + CH - 1) / CH;
                 const int slot = grp % C::NSLOT;
                 const int b = slot * C::GRP, b2 = b + 1;
                 if (!tc::warp_all(tc::mbar_wait(&accFull[slot], (grp / C::NSLOT) & 1, wait_limit) && !s_abort)) {
@@ -750,7 +758,7 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
                     ok = false;
                     break;
                 }
-                st0 += npass * CH;
+                st0 = PAIR ? st0 + npass * CH : group_end(t, st0, nst, CH);
                 tc::tc_fence_after();
                 const uint32_t tl = tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(b * C::ACC_COLS);
                 const uint32_t tl2 = tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(b2 * C::ACC_COLS);
