@@ -482,9 +482,10 @@ FfPlan make_plan(const Ctx& c, const FfDev& r, const double* ekq_h, const double
             // several slices where that gives the shorter waves, the slices still drained each
             // by itself (group_stages; every FP32 sum is the same).  512 x 4096 x 512 x 15: seven
             // slices in one unit, 129 -> 119 us; the bands kernel reads a seventh of the partials.
-            const long t = std::max(1L, tiles) * p.NT;
+            long t = std::max(1L, tiles) * p.NT;
             ff_pick_split_tc(t, r.nc, c.sms, p.KSa, p.kchunka);
             const int slice = p.kchunka / tcx::BK, n = p.KSa;
+            if (pipelined) t = std::max(1L, t / std::max(1, (int)p.groups.size() - 1 - p.ngR));  // a copy group's launch
             double best = 1e30;
             for (int m = 1; m <= n; ++m) {
                 const long waves = (t * ceil_div(n, m) + c.sms - 1) / c.sms;
@@ -599,8 +600,12 @@ fk_status ff_run(Ctx& c, const FfDev& r, const FfHost& h, const FfPipe* pipe) {
     if (order) std::memcpy(h.tab + ft.order, p.order.data(), r.nb * sizeof(int));
     std::memcpy(h.tab + ft.planes, p.planesR.data(), nR * sizeof(int));
     std::memcpy(h.tab + ft.planes + nR * sizeof(int), p.planesA.data(), nA * sizeof(int));
-    e = cudaMemcpyAsync(tab, h.tab, ft.bytes, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && !pipe) e = cudaEventRecord(c.pinned_ev, st);
+    // (pipelined: on the copy stream, ahead of the planes -- from a second stream the copy
+    // waited for the copies in flight, 0.9 ms of 5)
+    cudaStream_t ts = pipe ? c.copy_stream : st;
+    e = cudaMemcpyAsync(tab, h.tab, ft.bytes, cudaMemcpyHostToDevice, ts);
+    if (e == cudaSuccess) e = cudaEventRecord(c.pinned_ev, ts);
+    if (e == cudaSuccess && pipe) e = cudaEventRecord(c.pipe_ev[PIPE_READY], ts);
     if (e == cudaSuccess) e = cudaMemsetAsync(tabs, 0, 3 * (size_t)r.nb * r.nf * sizeof(double2), st);
     if (e != cudaSuccess) return cuda_fail(c, e, "ff: tables");
     c.launches = 0;
@@ -630,7 +635,6 @@ fk_status ff_run(Ctx& c, const FfDev& r, const FfHost& h, const FfPipe* pipe) {
                            isR ? pipe->epsR : pipe->epsA, isR ? pipe->epsR_d : pipe->epsA_d, q);
         }
         if (e == cudaSuccess) e = cudaStreamWaitEvent(st, c.pipe_ev[PIPE_READY], 0);
-        if (e == cudaSuccess) e = cudaEventRecord(c.pinned_ev, st);  // behind both copies out of the pinned buffer
         if (e != cudaSuccess) return cuda_fail(c, e, "ff: plane copies");
     }
 
