@@ -18,7 +18,8 @@
 // FP64 path: every branch quantity follows the reference's expression
 // sequence with round-to-nearest FP64 operations (no contraction), so each
 // branch is taken exactly as in the reference's C++; the contraction runs on
-// FP64 DMMA.  Mixed path: the branch quantities are evaluated in FP32 from an
+// the tensor cores by exact digit products (fk_tc64.cuh), or on FP64 DMMA where
+// there is no room for their images.  Mixed path: the branch quantities are evaluated in FP32 from an
 // FP64 wdiff and re-evaluated with the exact FP64 sequence whenever a test
 // value lies within a relative guard band of its threshold, so branch
 // decisions remain those of the FP64 sequence; the bulk products run in FP32

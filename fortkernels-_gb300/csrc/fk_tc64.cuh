@@ -81,7 +81,7 @@ struct Args {
     const uint8_t* B;    // [plane][nt][kstage][digit][im, re, -im][64][64 B]
     const int* ea;       // [slice][M] exponent of each A row's slice
     const int* eb;       // [plane][slice][N]
-    const double2 *W1, *W2;  // epilogue weights [column or igp][M]; W2: FF's second sum (nullptr: not needed)
+    const double2 *W1, *W2;  // epilogue weights [column or igp][M]; W2: FF's second sum (planes before tab.n2)
     double2* P;          // [plane][slice][nt][re/im half][M][G]
     int M, N, NT, KS, kst_unit, kstages, G;
     const int* skip;     // nonzero: a row cannot be represented, do nothing
