@@ -180,13 +180,21 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // Arrive on the barrier at the same shared-memory offset in CTA `rank` of the
-// cluster, with the default semantics (release at CTA scope): it orders only
-// this thread's own earlier operations.  Enough where the arrive reports work
-// that is already complete where it will be used: a TMEM buffer whose loads were
-// waited for, or operand tiles whose bulk copies have landed (their barrier has
-// completed) in the shared memory that the pair's MMAs read.  A cluster-wide
-// release costs 1000-2000 cycles per arrive; in the relay of the odd CTA's
-// operands it set the period of the FF contraction's stages (~1790 cycles).
+// cluster, releasing at cluster scope what this thread has observed: needed where
+// the arrive reports stores of other threads of this CTA (operand tiles written by
+// converter warps) to the CTA that issues the MMAs on them.
+__device__ __forceinline__ void mbar_arrive_remote(uint64_t* bar, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(bar)), "r"(rank));
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(a) : "memory");
+}
+// The same with release at CTA scope: nothing but the arrive itself reaches the other CTA
+// in order.  For what no store of this CTA takes part in: a TMEM buffer whose loads were
+// waited for, or operand tiles that bulk copies wrote.  Those copies have completed
+// (their barrier's phase has) in the shared memory that the pair's MMAs read, and copies and
+// MMAs both belong to the async proxy; this relies on completion alone.  A cluster-wide
+// release costs 1000-2000 cycles per arrive: in the relay of FF's operands it set the
+// period of the contraction's stages (~1790 cycles).
 __device__ __forceinline__ void mbar_arrive_peer(uint64_t* bar, uint32_t rank) {
     uint32_t a;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(bar)), "r"(rank));

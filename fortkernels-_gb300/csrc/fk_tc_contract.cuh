@@ -27,8 +27,8 @@
 // Work units are (m-tile, n-tile, k-slice, batch); CTA i takes units
 // i, i + gridDim.x, ...  What set the pace before: MMAs issued from a lane == 0
 // branch (92-102 cycles each beside busy warps instead of 64; now a converged
-// warp with one elected lane) and, on CTA pairs, the odd CTA's relay, whose
-// cluster-scope release took 1000-2000 cycles per stage.  The GPP contraction over
+// warp with one elected lane) and, on CTA pairs with pre-split operands, the odd CTA's
+// relay, whose cluster-scope release took 1000-2000 cycles per stage.  The GPP contraction over
 // 26 n-tiles went from 3.09 to 2.10 ms (1610 cycles per stage of 24 MMAs = 1536),
 // FF's R planes from 0.448 to 0.326 ms.  Every wait is bounded; on timeout the CTA records
 // an error code and unwinds without further waits of unbounded length.
@@ -420,7 +420,10 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
                         ok = false;
                         break;
                     }
-                    tc::mbar_arrive_peer(&peerFull[s], 0);
+                    // the converter warps' stores need a release that the other CTA can
+                    // acquire; tiles that came by bulk copy do not (fk_tc.cuh)
+                    if (ua) tc::mbar_arrive_peer(&peerFull[s], 0);
+                    else tc::mbar_arrive_remote(&peerFull[s], 0);
                 }
             }
         } else if (!PAIR || rank == 0) {
