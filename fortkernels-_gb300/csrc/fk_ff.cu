@@ -523,7 +523,8 @@ FfPlan make_plan(const Ctx& c, const FfDev& r, const double* ekq_h, const double
               p.bytesImgR + p.bytesImgA + p.bytesW + p.bytesAimg + p.bytesScale + 20 * 256;
     if (p.tc64)
         p.bytes += p.z.bytesA + p.z.bytesEa + p.zgroup * (p.z.bytesB + p.z.bytesEb) +
-                   2 * (size_t)r.nb * r.ng * sizeof(double2) + 6 * 256;
+                   2 * (size_t)r.nb * r.ng * sizeof(double2) +
+                   p.z.guard_bytes(r.nb, 2, (int)(p.planesR.size() + p.planesA.size())) + 7 * 256;
     return p;
 }
 
@@ -587,7 +588,10 @@ fk_status ff_run(Ctx& c, const FfDev& r, const FfHost& h, const FfPipe* pipe) {
         zb.eb = (int*)c.ws.take(p.zgroup * p.z.bytesEb);
         zb.W1 = (double2*)c.ws.take((size_t)r.nb * r.ng * sizeof(double2));
         zb.W2 = (double2*)c.ws.take((size_t)r.nb * r.ng * sizeof(double2));
-        if (!zb.A || !zb.B || !zb.ea || !zb.eb || !zb.W1 || !zb.W2)
+        zb.planes = nR + nA;
+        zb.guard_bytes = p.z.guard_bytes(r.nb, 2, zb.planes);
+        zb.guard = (uint8_t*)c.ws.take(zb.guard_bytes);
+        if (!zb.A || !zb.B || !zb.ea || !zb.eb || !zb.W1 || !zb.W2 || !zb.guard)
             return fail(c, FK_ENOMEM, "workspace too small for FF request");
     }
     if (!igp || !tab || !PR || (nA && !PA) || !tabs || !SD || (p.bytesImgR && !imgR) ||
@@ -771,7 +775,7 @@ fk_status ff_run(Ctx& c, const FfDev& r, const FfHost& h, const FfPipe* pipe) {
             auto k = d64::contract_kernel<EPI_FF>;
             cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d64::SMEM);
             kernel_begin(c);
-            k<<<grid, d64::THREADS, d64::SMEM, st>>>(a);
+            k<<<grid, d64::THREADS, d64::SMEM, st>>>(a, d64::Redo{});
             kernel_end(c);
             ++c.launches;
         }
@@ -806,7 +810,7 @@ fk_status ff_run(Ctx& c, const FfDev& r, const FfHost& h, const FfPipe* pipe) {
             if (tab.u0[tab.n] == 0) continue;
             const bool prof = c.profiling;
             if (!n2) c.profiling = false;
-            tc64::enqueue<EPI_FF>(c, a, p.z, zb, tab);
+            tc64::enqueue<EPI_FF>(c, a, p.z, zb, tab, g0);
             if (!n2) --c.nk;
             c.profiling = prof;
         }

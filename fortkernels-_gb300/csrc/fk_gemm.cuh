@@ -50,7 +50,6 @@ struct ContractArgs {
     double2* P;             // [slots][M][G]
     // FP64 engine behind the tensor-core one (fk_tc64.cuh)
     int nt_tiles = 0;               // n-tiles of the slot layout (0: ceil(N / BN))
-    const int* only_if = nullptr;   // the launch does nothing while this is 0
     const void* B2 = nullptr;       // batches from batches1 on read their planes here
     int batches1 = 0;
     const int* rowmap = nullptr;    // row m of A and aqsm (nullptr: m0 + m)
@@ -126,15 +125,64 @@ FK_DEV void cp_async16(void* smem, const void* gmem, bool pred) {
 FK_DEV void cp_commit() { asm volatile("cp.async.commit_group;\n"); }
 template <int N> FK_DEV void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
+// Which tiles a launch behind the tensor-core engine does: all where *flag is set, else those
+// with bound > rowmax + excess in some row.  rowmax: powers of two per sum and row,
+// [batch][G][M]; bound: the same of two n-tiles, [batch][slice][n-tile pair][G][M] (0: none).
+struct Redo {
+    const int* flag = nullptr;  // nullptr: every tile
+    const unsigned *rowmax = nullptr, *bound = nullptr;
+    int excess = 0;
+};
+// Tile t of a launch: row tile, n-tile, k-slice, batch.
+struct Tile {
+    int mt, nt, ks, batch;
+};
+FK_DEV Tile tile_at(const ContractArgs& a, int t) {
+    const int MT = ceil_div(a.M, BM), NT = a.nt_tiles ? a.nt_tiles : ceil_div(a.N, BN), y = t / MT;
+    return {t % MT, y % NT, (y / NT) % a.KS, y / (NT * a.KS)};
+}
+// Bit j: tile t0 + j * step (below n) is to be redone; block-uniform, and the same for both
+// n-tiles of a pair, which hold the real and imaginary halves of its sums.
+FK_DEV unsigned redo_mask(const ContractArgs& a, const Redo& r, int t0, int step, int n) {
+    __shared__ unsigned sm[THREADS / 32];
+    unsigned mask = *r.flag ? 0xffffffffu : 0u;
+    constexpr int U = 4, I = (BM * GMAX + THREADS - 1) / THREADS;
+    for (int j = 0; j < 32 && t0 + j * step < n; j += U) {
+        unsigned b[U][I], top[U][I];  // the loads of U tiles in flight
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int t = t0 + (j + u) * step;
+            const Tile x = tile_at(a, t);
+            const long unit = ((long)x.batch * a.KS + x.ks) * (a.nt_tiles / 2) + x.nt / 2;
+#pragma unroll
+            for (int q = 0; q < I; ++q) {
+                const int i = threadIdx.x + q * THREADS, m = x.mt * BM + i % BM, c = i / BM;
+                const bool ok = t < n && c < a.G && m < a.M;
+                b[u][q] = ok ? r.bound[(unit * a.G + c) * a.M + m] : 0u;
+                top[u][q] = ok ? r.rowmax[((long)x.batch * a.G + c) * a.M + m] : 0u;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int q = 0; q < I; ++q)
+                if (b[u][q] && (int)b[u][q] > (int)top[u][q] + r.excess) mask |= 1u << (j + u);
+    }
+    mask = __reduce_or_sync(0xffffffffu, mask);
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = mask;
+    __syncthreads();
+    for (int w = 0; w < THREADS / 32; ++w) mask |= sm[w];
+    __syncthreads();  // sm is written again for the next 32 tiles
+    return mask;
+}
+
 template <int EPI>
-__global__ void __launch_bounds__(THREADS) contract_kernel(ContractArgs a) {
+FK_DEV void contract_tile(const ContractArgs& a, Tile x) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2* As = reinterpret_cast<double2*>(smem_raw);
     double2* Bs = As + STAGES * BM * LDS;
-    if (a.only_if && !*a.only_if) return;
     const int NT = a.nt_tiles ? a.nt_tiles : ceil_div(a.N, BN);
-    const int mt = blockIdx.x, nt = blockIdx.y % NT;
-    const int ks = (blockIdx.y / NT) % a.KS, batch = blockIdx.y / (NT * a.KS);
+    const int mt = x.mt, nt = x.nt, ks = x.ks, batch = x.batch;
     const int plane = a.batch_plane ? a.batch_plane[batch] : batch;
     const double2* B =
         reinterpret_cast<const double2*>(a.B2 && batch >= a.batches1 ? a.B2 : a.B) + (long)plane * a.bstride;
@@ -231,6 +279,25 @@ __global__ void __launch_bounds__(THREADS) contract_kernel(ContractArgs a) {
     }
     __syncthreads();
     epi_reduce_store<BM, 8>(a, part, mt, (batch * a.KS + ks) * NT + nt);
+}
+
+// A block per tile, or (r.flag) blocks that walk the tiles and do those to be redone: one
+// wave, each block's checks in flight together.  (A block per tile behind the tensor-core engine
+// waited for its own loads in every wave of two blocks per SM: 2-3 us of a 220 us call.)
+template <int EPI>
+__global__ void __launch_bounds__(THREADS) contract_kernel(ContractArgs a, Redo r) {
+    const int n = ceil_div(a.M, BM) * (a.nt_tiles ? a.nt_tiles : ceil_div(a.N, BN)) * a.KS * a.batches;
+    const int b = blockIdx.y * gridDim.x + blockIdx.x, step = gridDim.x * gridDim.y;
+    for (int t0 = b; t0 < n; t0 += 32 * step) {
+        unsigned mask = r.flag ? redo_mask(a, r, t0, step, n) : 1u;
+        for (int j = 0; mask; ++j, mask >>= 1) {
+            const int t = t0 + j * step;
+            if (t >= n) break;
+            if (!(mask & 1)) continue;
+            contract_tile<EPI>(a, tile_at(a, t));
+            __syncthreads();  // its shared memory is reused
+        }
+    }
 }
 }  // namespace d64
 

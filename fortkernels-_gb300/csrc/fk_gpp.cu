@@ -1480,8 +1480,8 @@ struct Plan {
     // FP64 on the tensor cores (fk_tc64.cuh): the main and the static remainder contraction, and their workspace
     bool tc64;
     tc64::Plan z, zs;
-    size_t zA, zB, zEa, zEb, zW;
-    size_t bytesZ() const { return tc64 ? zA + zB + zEa + zEb + zW + 5 * 256 : 0; }
+    size_t zA, zB, zEa, zEb, zW, zG;
+    size_t bytesZ() const { return tc64 ? zA + zB + zEa + zEb + zW + zG + 6 * 256 : 0; }
 };
 
 // fk_gpp's mixed path and its FP64 path on the tensor cores (not the half sum, not
@@ -1601,6 +1601,7 @@ Plan make_plan(const Ctx& c, const GppDev& r, int ks_override = 0, bool pipeline
             p.zEa = p.z.bytesEa;
             p.zEb = p.z.bytesEb;
             p.zW = (size_t)r.ng * M * sizeof(double2);
+            p.zG = p.z.guard_bytes(M, 3, 1);
         }
     }
     const int BM = p.mixed ? f32::BM : d64::BM, BN = p.mixed ? f32::BN : d64::BN;
@@ -1623,6 +1624,7 @@ Plan make_plan(const Ctx& c, const GppDev& r, int ks_override = 0, bool pipeline
         p.zEa = std::max(p.zEa, p.zs.bytesEa);
         p.zEb = std::max(p.zEb, p.zs.bytesEb);
         p.zW = (size_t)r.ng * r.nb * sizeof(double2);
+        p.zG = std::max(p.zG, p.zs.guard_bytes(r.nb, 1, 1));
     }
     p.bytesD = M <= 0 ? 0
                : p.mixed ? (size_t)p.NT * p.kstages * tcx::Cfg<64>::B_BYTES
@@ -1645,13 +1647,17 @@ bool take_tc64(Ctx& c, const Plan& p, tc64::Bufs& b) {
     b.eb = (int*)c.ws.take(p.zEb);
     b.W1 = (double2*)c.ws.take(p.zW);
     b.W2 = nullptr;
-    return b.A && b.B && b.ea && b.eb && b.W1;
+    b.planes = 1;
+    b.guard_bytes = p.zG;
+    b.guard = (uint8_t*)c.ws.take(p.zG);
+    return b.A && b.B && b.ea && b.eb && b.W1 && b.guard;
 }
 template <int EPI>
-void run_tc64(Ctx& c, const ContractArgs& a, const tc64::Plan& z, const tc64::Bufs& b, bool have_a = false) {
+void run_tc64(Ctx& c, const ContractArgs& a, const tc64::Plan& z, const tc64::Bufs& b, bool have_a = false,
+              bool re_only = false) {
     tc64::enqueue_weights(c, a, EPI == EPI_GPP ? a.N / 3 : a.N, b, false);
     if (!have_a) tc64::enqueue_a(c, a, z, b);
-    tc64::enqueue<EPI>(c, a, z, b, tc64::one_plane(z));
+    tc64::enqueue<EPI>(c, a, z, b, tc64::one_plane(z), 0, re_only);
 }
 
 // A side branch of the context's stream: work queued between fork and join on
@@ -2108,7 +2114,7 @@ fk_status gpp_run_half(Ctx& c, const GppDev& r) {
             auto k = d64::contract_kernel<EPI_GPP>;
             set_smem(k, d64::SMEM);
             kernel_begin(c);
-            k<<<dim3(p.MT, p.NT * p.KS), d64::THREADS, d64::SMEM, st>>>(a);
+            k<<<dim3(p.MT, p.NT * p.KS), d64::THREADS, d64::SMEM, st>>>(a, d64::Redo{});
             kernel_end(c);
         }
         ++c.launches;
@@ -2327,7 +2333,7 @@ fk_status gpp_run(Ctx& c, const GppDev& r, const GppPipe* pipe) {
             auto k = d64::contract_kernel<EPI_GPP>;
             set_smem(k, d64::SMEM);
             kernel_begin(c);
-            k<<<grid, d64::THREADS, d64::SMEM, st>>>(a);
+            k<<<grid, d64::THREADS, d64::SMEM, st>>>(a, d64::Redo{});
             kernel_end(c);
         }
         ++c.launches;
@@ -2361,7 +2367,7 @@ fk_status gpp_run(Ctx& c, const GppDev& r, const GppPipe* pipe) {
         } else {
             auto k = d64::contract_kernel<EPI_STAT>;
             set_smem(k, d64::SMEM);
-            k<<<grid, d64::THREADS, d64::SMEM, st>>>(a);
+            k<<<grid, d64::THREADS, d64::SMEM, st>>>(a, d64::Redo{});
         }
         ++c.launches;
     }
@@ -2900,13 +2906,13 @@ fk_status gpp_real_run(Ctx& c, const GppRealDev& r) {
             k<<<std::min(p.units, c.sms), tcx::THREADS, tcx::Cfg<64>::SMEM, st>>>(t);
             kernel_end(c);
         } else if (p.tc64) {
-            run_tc64<EPI_GPP>(c, a, p.z, zb);
+            run_tc64<EPI_GPP>(c, a, p.z, zb, false, true);
             --c.launches;
         } else {
             auto k = d64::contract_kernel<EPI_GPP>;
             set_smem(k, d64::SMEM);
             kernel_begin(c);
-            k<<<dim3(p.MT, p.NT * p.KS), d64::THREADS, d64::SMEM, st>>>(a);
+            k<<<dim3(p.MT, p.NT * p.KS), d64::THREADS, d64::SMEM, st>>>(a, d64::Redo{});
             kernel_end(c);
         }
         ++c.launches;

@@ -19,12 +19,24 @@
 // where |C_c| <= 64 * (2 * 2^14 + 3 * 2^16) < 2^24: every one of these sums is
 // exact, and they are added exactly as 64-bit integers.  Classes 5 and 6 weigh
 // 2^-45 and 2^-54 and accumulate over the whole k-slice in FP32; classes 7 and
-// above (2^-59 of the rows' largest product, per term) are left out.  What is
-// left of rounding is below that of an FP64 dot product, whose accumulated
-// rounding is ~2^-53 of the running sum per term.  A row with an infinity, a
+// above are left out.
+//
+// Error.  Unlike an FP64 dot product's it is relative to the rows' largest
+// magnitudes, not to the terms: the classes left out amount to 2^-57.2 sqrt(2 K)
+// 2^(Ea + Eb) (rms over a slice of K k-values, measured against exact sums for
+// uniform, normal, graded and outlying values; at most 2^-55.7).  On rows of one
+// scale that is 2^-55 of |S|, below the rounding of an FP64 sum; on a row with an
+// outlier over a zero of the other operand, or on rows graded in opposite
+// directions, it can be more than all of S.  So the epilogue keeps, per row and
+// weighted sum, the largest term |w| |S| of all columns and slices (rowmax) and
+// per unit the largest |w| 2^(Ea + Eb) (bound), both as powers of two, and the
+// DMMA kernel of fk_gemm.cuh, launched behind, redoes the tiles (64 rows of a unit)
+// where the error exceeds 2^-48 of rowmax in some row (Plan::excess, d64::redo_mask): at
+// most 3e-15 of the row's largest term, per column and slice, stays.  The guard costs
+// 0.3-1% of a call (512 x 32768 x 20 402 -> 404 us, FF 512 x 4096 x 512 x 15 3.70 -> 3.73 ms,
+// the half sum's two contractions at 678 x 1792 x 7 280 -> 286 us).  A row with an infinity, a
 // NaN or magnitudes beyond 2^+-400 sets a flag: the contraction then does
-// nothing and the DMMA kernel of fk_gemm.cuh, launched behind it and idle
-// otherwise, fills the same partial sums.
+// nothing and the DMMA kernel fills all of the partial sums.
 //
 // One unit is a 256-row x 64-column tile over one k-slice, on a CTA pair
 // (tcgen05 cta_group::2, M = 256, N = 128: D = [S_re | S_im]); per 32 k-values
@@ -38,10 +50,14 @@
 // (PAIRS, below).
 // Measured (GB300): the contraction of GPP 512 x 2 x 32768 x 20 takes 0.17 ms
 // (DMMA 7.85 ms), FF's planes at 512 x 4096 x 512 x 15 take 3.28 ms (DMMA 222 ms;
-// the A planes over the bands that read them only); errors against 64-bit
-// references are those of the DMMA path or lower (FF 1.9e-15 against 4.8e-15).
+// the A planes over the bands that read them only).  A call's errors against 64-bit
+// references are of the DMMA path's size, on some shapes lower and on some higher (FF
+// 512 x 4096 x 512 x 15 1.9e-15 against 4.8e-15, 40 x 640 x 48 x 6 2.6e-15 against
+// 8.4e-16, GPP 512 x 32768 x 20 3.0e-15 against 2.6e-15): what is left there is the
+// order of the weighted sums, not the digits.
 #pragma once
 #include <algorithm>
+#include <cmath>
 
 #include <cuda_fp16.h>
 
@@ -85,6 +101,9 @@ struct Args {
     double2* P;          // [plane][slice][nt][re/im half][M][G]
     int M, N, NT, KS, kst_unit, kstages, G;
     const int* skip;     // nonzero: a row cannot be represented, do nothing
+    unsigned* rowmax;    // [plane][G][M] largest term of each sum (guard_term; zero at entry)
+    unsigned* bound;     // [plane][slice][nt][G][M] largest |w| 2^(Ea + Eb) of a unit (zero at entry)
+    int re_only;         // only the real parts of the sums are used (real-valued GPP)
     int* err;
     long long wait_limit;
     PlaneTab tab;
@@ -107,6 +126,27 @@ struct SplitArgs {
 
 __device__ __forceinline__ unsigned long long abs_bits(double v) {
     return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+}
+// The guard's powers of two, in few integer instructions and registers: the biased exponent of
+// a double (0 .. 2046), of the larger part of a weight, and one word per sum that holds two
+// maxima, |w| |S| in its low half and |w| 2^Eb in its high half.  Zeros need no case of
+// their own: a zero weight or sum counts as 2^-1023 on both sides of the comparison, a row of
+// zeros has the exponent ZERO_ROW, far below that.
+constexpr int ZERO_ROW = -2600, GUARD_EB = 3000;
+__device__ __forceinline__ unsigned exponent_of(double s) { return ((unsigned)__double2hiint(s) << 1) >> 21; }
+__device__ __forceinline__ unsigned exponent_of(double2 w) {
+    return max((unsigned)__double2hiint(w.x) << 1, (unsigned)__double2hiint(w.y) << 1) >> 21;
+}
+__device__ __forceinline__ unsigned guard_pair(double s, int eb) {
+    return ((unsigned)(eb + GUARD_EB) << 16) + exponent_of(s);
+}
+__device__ __forceinline__ unsigned guard_max(unsigned g, unsigned pair, double2 w) {
+    return __vmaxu2(g, pair + exponent_of(w) * 0x10001u);
+}
+// Both maxima on one scale (the second times 2^Ea), as words that are positive for every sum (0: none).
+__device__ __forceinline__ unsigned guard_term(unsigned g) { return (g & 0xffffu) + 4096u; }
+__device__ __forceinline__ unsigned guard_bound(unsigned g, int ea) {
+    return g >> 16 ? (unsigned)max(1, (int)(g >> 16) - GUARD_EB + 1023 + ea + 4096) : 0u;
 }
 // x as an integer multiple of 2^(E - 59), E = emax - 1023 (|result| <= 2^60),
 // plus 256 in every digit position: digit d (0 the leading one) is then the
@@ -217,7 +257,7 @@ __global__ void __launch_bounds__(256) split_kernel(SplitArgs s) {
         const int emax = (int)(mx >> 52);
         const bool bad = mx != 0 && (emax < 1023 - 400 || emax > 1023 + 400);  // infinities and NaN too
         if (threadIdx.x == 0) {
-            s.exps[((long)batch * s.KS + ks) * s.rows + row] = mx ? emax - 1023 : 0;
+            s.exps[((long)batch * s.KS + ks) * s.rows + row] = mx ? emax - 1023 : ZERO_ROW;
             if (bad) atomicOr(s.flag, 1);
         }
         uint8_t* tile = s.img + ((long)batch * s.tiles + row / (BSIDE ? BN : 128)) * s.kstages *
@@ -236,10 +276,12 @@ __global__ void __launch_bounds__(256) split_kernel(SplitArgs s) {
 }
 
 // Epilogue weights in FP64, [h][M]: W1 = wscale * vcoul[igp] * conj(aqsm[row][acol]), W2 = conj(aqsm) (or null);
-// row = rowmap[m] or m0 + m.
+// row = rowmap[m] or m0 + m.  Also clears the guard's nzero words (a memset of its own took 2 us).
 static __global__ void weights_kernel(int M, int m0, int ncols, const double2* aqsm, long ldm, const double* vcoul,
                                       const int* igp, const int* acol, double wscale, double2* W1, double2* W2,
-                                      const int* rowmap) {
+                                      const int* rowmap, unsigned* zero, long nzero) {
+    const long stride = (long)gridDim.x * gridDim.y * blockDim.x;
+    for (long i = ((long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; i < nzero; i += stride) zero[i] = 0;
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= M) return;
     for (int h = blockIdx.y; h < ncols; h += gridDim.y) {
@@ -339,6 +381,13 @@ __device__ __forceinline__ double fixed_to_double(long long h, float f, int ex) 
     // exponent of bit 63 is 63 - lz + ex; a carry out of the 53 bits adds one to the exponent field
     const unsigned long long bits = ((unsigned long long)(1023 + 63 - lz + ex - 1) << 52) + q;
     return __longlong_as_double((long long)(bits | (h < 0 ? 0x8000000000000000ull : 0ull)));
+}
+
+// A unit's part of the guard for sum c of row m: its largest term (the maximum over units and
+// halves does not depend on their order) and its bound (the same in both halves).
+__device__ __forceinline__ void guard(const Args& t, int pl, int ks, int nt, int c, int m, int half, unsigned g, int ea) {
+    if (half == 0 || !t.re_only) atomicMax(&t.rowmax[((long)pl * t.G + c) * t.M + m], guard_term(g));
+    if (half == 0) t.bound[((((long)pl * t.KS + ks) * t.NT + nt) * t.G + c) * t.M + m] = guard_bound(g, ea);
 }
 
 template <int EPI>
@@ -591,6 +640,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) contract
             const int n0 = x.nt * BN, ncol = min(BN, t.N - n0);
             const bool both = EPI == EPI_FF && x.pl < t.tab.n2;
             double2 g[3] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+            unsigned gm[3] = {0u, 0u, 0u};  // the guard's maxima of each sum
             // GPP: eight columns per turn of a rolled loop, H moving down by eight, and g[k] the sum
             // of class (t0 + k) % 3 of the columns.  Unrolled over the 64 columns the code runs once
             // per unit and its bound was fetching it: 64 x 777 x 7 220 -> 217 us, 512 x 32768 x 20
@@ -628,9 +678,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) contract
                             // half 0: w * s, half 1: w * (i s)
                             const int gi = EPI == EPI_GPP ? (jb + j) % 3 : 0;
                             const double sr = half ? -s : s;
+                            const unsigned pair = guard_pair(s, ebp[j0 + jb + j]);
+                            gm[gi] = guard_max(gm[gi], pair, w1[j]);
                             g[gi].x = fma(half ? w1[j].y : w1[j].x, sr, g[gi].x);
                             g[gi].y = fma(half ? w1[j].x : w1[j].y, s, g[gi].y);
                             if (EPI == EPI_FF && both) {
+                                gm[1] = guard_max(gm[1], pair, w2[j]);
                                 g[1].x = fma(half ? w2[j].y : w2[j].x, sr, g[1].x);
                                 g[1].y = fma(half ? w2[j].x : w2[j].y, s, g[1].y);
                             }
@@ -640,17 +693,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) contract
 #pragma unroll
                 for (int j = 0; j + TURN < BN; ++j) H[j] = H[j + TURN];
                 if (EPI == EPI_GPP) {  // (t0 + 8) % 3 = (t0 + 2) % 3
-                    const double2 g0 = g[0], g1 = g[1];
-                    g[0] = g[2];
-                    g[1] = g0;
-                    g[2] = g1;
+                    auto turn = [](auto(&v)[3]) {
+                        const auto v0 = v[0], v1 = v[1];
+                        v[0] = v[2];
+                        v[1] = v0;
+                        v[2] = v1;
+                    };
+                    turn(g);
+                    turn(gm);
                 }
             }
             if (EPI == EPI_GPP) {  // back to class k % 3 (64 % 3 = 1)
-                const double2 g2 = g[2];
-                g[2] = g[1];
-                g[1] = g[0];
-                g[0] = g2;
+                auto back = [](auto(&v)[3]) {
+                    const auto v2 = v[2];
+                    v[2] = v[1];
+                    v[1] = v[0];
+                    v[0] = v2;
+                };
+                back(g);
+                back(gm);
             }
             if (m < t.M) {
                 double2* out = t.P + ((((long)x.pl * t.KS + x.ks) * t.NT + x.nt) * 2 + half) * (long)t.M * t.G + (long)m * t.G;
@@ -658,9 +719,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) contract
                     // column n0 + j is of frequency (n0 + j) % 3
                     const int r = n0 % 3;
 #pragma unroll
-                    for (int q = 0; q < 3; ++q) out[(q + r) % 3] = g[q];
+                    for (int q = 0; q < 3; ++q) {
+                        out[(q + r) % 3] = g[q];
+                        guard(t, x.pl, x.ks, x.nt, (q + r) % 3, m, half, gm[q], ea);
+                    }
                 } else {
-                    for (int q = 0; q < t.G; ++q) out[q] = q == 0 ? g[0] : g[1];
+                    for (int q = 0; q < t.G; ++q) {
+                        out[q] = q == 0 ? g[0] : g[1];
+                        guard(t, x.pl, x.ks, x.nt, q, m, half, q == 0 ? gm[0] : gm[1], ea);
+                    }
                 }
             }
         }
@@ -676,10 +743,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) contract
 }
 
 // ------------------------------------------------------------------- plan
+constexpr size_t GUARD_HEAD = 256;  // the flag of rows that cannot be represented, in front of the guard's words
 struct Plan {
     int MT, NT, KS, kst_unit, kstages;
     size_t bytesA, bytesB, bytesEa, bytesEb;  // images and exponents (B: of one plane)
     size_t slots() const { return (size_t)KS * NT * 2; }  // partial slots per plane
+    // the guard's words (Bufs::guard) of `planes` planes of G sums over M rows
+    size_t guard_bytes(int M, int G, int planes) const {
+        return GUARD_HEAD + (size_t)planes * G * M * (1 + (size_t)KS * NT) * sizeof(unsigned);
+    }
+    // A tile is redone where bound exceeds rowmax by more than this power of two: the error
+    // 2^-57.2 sqrt(2 K) 2^bound then exceeds 2^-48 2^rowmax.  (The synthetic inputs of this
+    // package, all branches: at most 2^3 sqrt(2 K), 2^5 for a single column of 32 k-values;
+    // the limit is 2^9.)
+    int excess() const { return (int)std::floor(9.0 - 0.5 * std::log2(2.0 * kst_unit * BK)); }
 };
 
 // The k-split: the fewest pair-cycles over whole waves, a unit costing ~8700
@@ -718,10 +795,12 @@ struct Bufs {
     uint8_t *A, *B;
     int *ea, *eb;
     double2 *W1, *W2;
+    uint8_t* guard;       // [flag][rowmax of `planes` planes][bound]
+    size_t guard_bytes;
+    int planes;           // planes the guard covers
+    int* flag() const { return (int*)guard; }
+    unsigned* rowmax() const { return (unsigned*)(guard + GUARD_HEAD); }
 };
-
-// Set when a row cannot be represented (a word beside the error word).
-inline int* flag_word(const Ctx& c) { return c.errword + 16; }
 
 template <bool BSIDE>
 inline void launch_split(Ctx& c, const SplitArgs& s, int batches) {
@@ -742,39 +821,46 @@ inline void launch_split(Ctx& c, const SplitArgs& s, int batches) {
 
 // The digits of a.A's rows m0 .. m0+M-1 (or rowmap[0 .. M)) and the flag's reset.
 inline void enqueue_a(Ctx& c, const ContractArgs& a, const Plan& p, const Bufs& b) {
-    cudaMemsetAsync(flag_word(c), 0, sizeof(int), c.stream);
+    cudaMemsetAsync(b.flag(), 0, sizeof(int), c.stream);
     SplitArgs s{a.rowmap ? a.A : a.A + (long)a.m0 * a.lda, nullptr, 1, a.lda, 0, nullptr, a.rowmap, a.M, a.K, p.KS, p.kst_unit,
-                p.kstages, 2 * p.MT, b.A, b.ea, flag_word(c), c.errword, c.wait_limit};
+                p.kstages, 2 * p.MT, b.A, b.ea, b.flag(), c.errword, c.wait_limit};
     launch_split<false>(c, s, 1);
 }
 
 // The digits of a.batches planes (at most MAXPL) of a.B, the contraction over the row tiles of `tab` and the
-// DMMA kernel for rows that cannot be represented.
+// DMMA kernel for rows that cannot be represented and tiles the digits are too coarse for.  The
+// launch's first plane is plane0 of the guard's; re_only as in Args.
 template <int EPI>
-inline void enqueue(Ctx& c, ContractArgs a, const Plan& p, const Bufs& b, const PlaneTab& tab) {
+inline void enqueue(Ctx& c, ContractArgs a, const Plan& p, const Bufs& b, const PlaneTab& tab, int plane0 = 0,
+                    bool re_only = false) {
     SplitArgs s{(const double2*)a.B, (const double2*)a.B2, a.B2 ? a.batches1 : a.batches, a.ldb, a.bstride, a.batch_plane, nullptr, a.N, a.K, p.KS, p.kst_unit, p.kstages,
-                p.NT, b.B, b.eb, flag_word(c), c.errword, c.wait_limit};
+                p.NT, b.B, b.eb, b.flag(), c.errword, c.wait_limit};
     launch_split<true>(c, s, a.batches);
+    const long rows = (long)a.G * a.M;  // guard words per plane: rowmax, and bound of one unit column
+    unsigned* rowmax = b.rowmax() + plane0 * rows;
+    unsigned* bound = b.rowmax() + b.planes * rows + plane0 * rows * p.KS * p.NT;
     Args t{b.A, b.B, b.ea, b.eb, b.W1, b.W2, a.P, a.M, a.N, p.NT, p.KS, p.kst_unit, p.kstages, a.G,
-           flag_word(c), c.errword, c.wait_limit, tab};
+           b.flag(), rowmax, bound, re_only ? 1 : 0, c.errword, c.wait_limit, tab};
     auto k = contract_kernel<EPI>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
     kernel_begin(c);
     k<<<2 * std::min(tab.u0[tab.n], c.sms / 2), THREADS, SMEM, c.stream>>>(t);
     kernel_end(c);
-    a.only_if = flag_word(c);
     a.nt_tiles = 2 * p.NT;
     a.KS = p.KS;
     a.kchunk = p.kst_unit * BK;
     auto f = d64::contract_kernel<EPI>;
     cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d64::SMEM);
-    f<<<dim3(ceil_div(a.M, d64::BM), a.nt_tiles * a.KS * a.batches), d64::THREADS, d64::SMEM, c.stream>>>(a);
+    const int tiles = ceil_div(a.M, d64::BM) * a.nt_tiles * a.KS * a.batches;
+    f<<<std::min(tiles, 2 * c.sms), d64::THREADS, d64::SMEM, c.stream>>>(a, d64::Redo{b.flag(), rowmax, bound, p.excess()});
     c.launches += 2;
 }
 
+// The weights, and the guard's reset: ahead of each contraction, or of a call's launches over its planes.
 inline void enqueue_weights(Ctx& c, const ContractArgs& a, int ncols, const Bufs& b, bool second) {
     weights_kernel<<<dim3(ceil_div(a.M, 128), std::min(ncols, 65535)), 128, 0, c.stream>>>(
-        a.M, a.m0, ncols, a.aqsm, a.ldm, a.vcoul, a.igp, a.acol, a.wscale, b.W1, second ? b.W2 : nullptr, a.rowmap);
+        a.M, a.m0, ncols, a.aqsm, a.ldm, a.vcoul, a.igp, a.acol, a.wscale, b.W1, second ? b.W2 : nullptr, a.rowmap,
+        b.rowmax(), (long)((b.guard_bytes - GUARD_HEAD) / sizeof(unsigned)));
     ++c.launches;
 }
 
