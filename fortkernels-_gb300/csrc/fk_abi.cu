@@ -12,6 +12,7 @@
 
 #include "fk_internal.h"
 #include "fk_tc.cuh"
+#include "fk_workspace.h"
 
 namespace fk {
 
@@ -114,7 +115,7 @@ bool workspace_can_hold(Ctx& c, size_t need) {
         cudaGetLastError();
         return false;
     }
-    return avail + c.ws.cap >= need + need / 4 + (2u << 20);
+    return avail + c.ws.cap >= grown_size(need) + (1u << 20);
 }
 
 fk_status ensure_workspace(Ctx& c, size_t need) {
@@ -124,17 +125,27 @@ fk_status ensure_workspace(Ctx& c, size_t need) {
     drop_graphs(c);  // captured graphs refer to the old workspace
     cudaError_t e = cudaStreamSynchronize(c.stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "workspace: synchronize");
-    if (c.ws.base) cudaFree(c.ws.base);
-    c.ws.base = nullptr;
-    c.ws.cap = 0;
-    size_t cap = need + need / 4 + (1u << 20);
-    e = cudaMalloc(&c.ws.base, cap);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return cuda_fail(c, e, "workspace: cudaMalloc");
-    }
-    c.ws.cap = cap;
-    return FK_OK;
+    const bool ok = grow_block(
+        c.ws.base, c.ws.cap, need,
+        [&](size_t bytes) {
+            void* p = nullptr;
+            e = cudaMalloc(&p, bytes);
+            if (e == cudaSuccess) return p;
+            cudaGetLastError();
+            return (void*)nullptr;
+        },
+        [](void* p) { cudaFree(p); });
+    return ok ? FK_OK : cuda_fail(c, cudaErrorMemoryAllocation, "workspace: cudaMalloc");
+}
+
+// The workspace of a request: FP64 contracts on the tensor cores when the workspace can hold
+// its operand images (28 bytes per aqsntemp element, 42 per D or epsilon element of the planes
+// converted at once), else on DMMA.
+template <class Need>
+fk_status request_workspace(Ctx& c, fk_precision precision, bool& tc64, Need need) {
+    return choose_workspace(
+        precision == FK_FP64, tc64, FK_ENOMEM, need, [&](size_t n) { return workspace_can_hold(c, n); },
+        [&](size_t n) { return ensure_workspace(c, n); });
 }
 
 // An input array: used in place when it is device memory, staged otherwise.
@@ -677,15 +688,10 @@ fk_status gpp_call(fk_ctx_t c, int nb, int nv, int nc, int ng, const fk_c128* aq
         }
     }
     const size_t outn = 7 + (size_t)nb;
-    // FP64 contracts on the tensor cores when the workspace can hold its operand
-    // images (28 bytes per aqsntemp element, 42 per D element), else on DMMA
-    size_t need = 0;
-    for (int tc = precision == FK_FP64 ? 1 : 0; tc >= 0; --tc) {
-        r.tc64 = tc != 0;
-        need = fk::staged_bytes(ins) + fk::gpp_workspace(x, r) + outn * sizeof(double2) + 4096;
-        if (!tc || fk::workspace_can_hold(x, need)) break;
-    }
-    fk_status s = fk::ensure_workspace(x, need);
+    fk_status s = fk::request_workspace(x, precision, r.tc64, [&](bool tc) {
+        r.tc64 = tc;
+        return fk::staged_bytes(ins) + fk::gpp_workspace(x, r) + outn * sizeof(double2) + 4096;
+    });
     if (s != FK_OK) return s;
 
     // Repeated calls whose arrays are all device memory replay a captured
@@ -850,13 +856,10 @@ fk_status fk_gpp_real(fk_ctx_t c, int nb, int nv, int nc, int ng, const double* 
     r.nb = nb; r.nv = nv; r.nc = nc; r.ng = ng; r.prec = precision; r.flags = flags;
     r.lda = aqn_in_place ? nc : lda;
     const size_t outn = 6 + (size_t)nb;
-    size_t need = 0;
-    for (int tc = precision == FK_FP64 ? 1 : 0; tc >= 0; --tc) {  // as in fk_gpp
-        r.tc64 = tc != 0;
-        need = fk::staged_bytes(ins) + aqn_bytes + fk::gpp_real_workspace(x, r) + outn * sizeof(double) + 4096;
-        if (!tc || fk::workspace_can_hold(x, need)) break;
-    }
-    fk_status s = fk::ensure_workspace(x, need);
+    fk_status s = fk::request_workspace(x, precision, r.tc64, [&](bool tc) {
+        r.tc64 = tc;
+        return fk::staged_bytes(ins) + aqn_bytes + fk::gpp_real_workspace(x, r) + outn * sizeof(double) + 4096;
+    });
     if (s != FK_OK) return s;
     x.ws.reset();
     double* out = (double*)x.ws.take(outn * sizeof(double));
@@ -960,14 +963,11 @@ fk_status fk_ff(fk_ctx_t c, int nb, int nv, int nc, int ng, int nf, int ne, cons
     size_t packed = 0, packed_host = 0;
     for (auto* i : small)
         if (!fk::in_place(i)) packed += r256(i->bytes);
-    size_t need = 0;
-    for (int tc = precision == FK_FP64 ? 1 : 0; tc >= 0; --tc) {  // as in fk_gpp
-        r.tc64 = tc != 0;
-        need = fk::staged_bytes(pipelined ? bands : large) + (pipelined ? 2 * r256(planes) : 0) + r256(packed) +
+    fk_status s = fk::request_workspace(x, precision, r.tc64, [&](bool tc) {
+        r.tc64 = tc;
+        return fk::staged_bytes(pipelined ? bands : large) + (pipelined ? 2 * r256(planes) : 0) + r256(packed) +
                fk::ff_workspace(x, r, hf, pipelined) + outn * sizeof(double2) + 4096;
-        if (!tc || fk::workspace_can_hold(x, need)) break;
-    }
-    fk_status s = fk::ensure_workspace(x, need);
+    });
     if (s != FK_OK) return s;
     x.ws.reset();
     double2* out = (double2*)x.ws.take(outn * sizeof(double2));

@@ -58,7 +58,11 @@ typedef enum {
 } fk_status;
 
 typedef enum {
-    FK_FP64 = 0,   /* plain path: FP64 everywhere; matches the reference C++ to 1e-12 */
+    FK_FP64 = 0,   /* plain path: FP64 results, matching the reference C++ to 1e-12.  The
+                      contraction runs on the tensor cores as exact products of 9-bit
+                      digits where the workspace can hold their images (see
+                      fk_reserve) and the rows' magnitudes allow it to FP64's accuracy,
+                      else on FP64 DMMA: the last bits of a result depend on which */
     FK_MIXED = 1   /* branch tests and near-pole divisions in FP64, bulk
                       contractions in reduced precision with FP32 accumulation
                       and FP64 block reductions; <= 1e-6 relative to FP64 */
@@ -77,7 +81,18 @@ fk_status fk_set_stream(fk_ctx_t ctx, void* stream);
 /* Wait for all work enqueued by the context. */
 fk_status fk_synchronize(fk_ctx_t ctx);
 /* Grow the device workspace to at least `bytes` now (e.g. before capturing
- * a CUDA graph, during which the library must not allocate). */
+ * a CUDA graph, during which the library must not allocate).  The workspace
+ * keeps its largest size until fk_destroy.  An FP64 call takes the tensor-core
+ * engine when its workspace fits what is there or can be allocated, and the
+ * DMMA engine (smaller, 20 to 60 times slower on large shapes) otherwise: also
+ * during a capture, where nothing can grow.  To have the tensor-core engine
+ * captured make one call of that shape before, or reserve about
+ *   fk_gpp:  28*M*ncouls + (48*ngpown + 42*N)*ncouls bytes, M = number_bands
+ *            rounded up to a multiple of 256 and N = 3*ngpown to one of 64,
+ *   fk_ff:   28*M*ncouls + 42*N*ncouls for each plane converted at once (up to 64
+ *            planes or 4 GB), N = ngpown rounded up to a multiple of 64,
+ * and the staged inputs, weights (16 to 32 bytes per band and column) and
+ * partial sums. */
 fk_status fk_reserve(fk_ctx_t ctx, size_t bytes);
 /* Static description of a status code, and the last detailed message. */
 const char* fk_strerror(fk_status s);
