@@ -327,7 +327,9 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) prep64_kernel(PrepArgs p) {
         wx[iw] = p.wx[iw];
         const double w2 = wx[iw] * wx[iw];
         iw2[iw] = 1.0 / w2;
-        wok[iw] = w2 > 1e-200 && w2 < 1e200;
+        // |wdiff|^2 stays a number of FP32 (wtilde below 2^60), and (wx^2)^2, by which the sequence
+        // divides, a normal number
+        wok[iw] = w2 > 1e-140 && w2 < 1e36;
     }
     const double2* wrow = p.wt + (long)my_igp * p.nc;
     const double2* erow = p.eps + (long)my_igp * p.nc;
