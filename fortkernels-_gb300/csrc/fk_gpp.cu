@@ -299,8 +299,8 @@ __device__ __noinline__ Element64 element64(double wxt, double2 wt, double2 ep, 
 // Bound by the FP64 pipe (64 cycles per warp instruction on each sub-partition),
 // so the common path spends few FP64 instructions: the branch tests run in FP32
 // on |wdiff|^2 (from its FP64 value) and |wt|^2/|wdiff|^2, any element within a
-// relative 1e-5 of a threshold, out of FP32's comfortable range or not finite
-// takes the reference's sequence (element64), as do the rare branches of ssx; the
+// relative 1e-5 of a threshold, out of FP32's comfortable range or with a value
+// that is not finite takes the reference's sequence (element64), as do the rare branches of ssx; the
 // value wt*I_eps*conj(wdiff)/|wdiff|^2 needs ten (the reciprocal: an FP32 one and
 // two Newton steps, r += r(1 - n r), relative error 2^-23 -> 2^-46 -> 2^-53), and
 // ssx = Omega2/wx^2 six per element and band plus two per frequency.  512 x 2 x
@@ -336,9 +336,11 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) prep64_kernel(PrepArgs p) {
     double2* D = reinterpret_cast<double2*>(p.D);
     const int ig_end = min(p.nc, (ch + 1) * p.tile);
     auto large = [](double v) { return (((unsigned)__double2hiint(v) >> 20) & 0x7ffu) >= 1023u + 60u; };
+    auto infinite = [](double v) { return ((unsigned)__double2hiint(v) & 0x7ff00000u) == 0x7ff00000u; };  // or NaN
     for (int ig = ch * p.tile + tid; ig < ig_end; ig += PREP_THREADS) {
         const double2 wt = wrow[ig], ep = erow[ig];
         double2 eq = ep, an[NVC], pn[NVC];
+        bool bad = false;  // an occupied band's value is not finite: the sequence adds it times a zero ssx, too
         if (Q == 1 && flags) eq = p.eps[(long)my_igp * p.ng + ig];  // gppKer.cpp:139
         if (flags) {
             // aqsntemp*Omega2 of the pass's bands
@@ -347,10 +349,11 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) prep64_kernel(PrepArgs p) {
 #pragma unroll
             for (int j = 0; j < NVC; ++j) {
                 an[j] = j < nflag ? p.aqsn[(long)(p.n1base + j) * p.nc + ig] : make_double2(0.0, 0.0);
+                bad = bad || infinite(an[j].x) || infinite(an[j].y);
                 pn[j] = make_double2(fma(an[j].x, om.x, -(an[j].y * om.y)), fma(an[j].x, om.y, an[j].y * om.x));
             }
         }
-        const bool weird = all_exact || large(wt.x) || large(wt.y) || large(ep.x) || large(ep.y);
+        const bool weird = all_exact || bad || large(wt.x) || large(wt.y) || large(ep.x) || large(ep.y);
         const float2 wf = c64_to_f32(wt);
         const float wsq = wf.x * wf.x + wf.y * wf.y;
         const double y2 = wt.y * wt.y;

@@ -36,3 +36,21 @@ def test_tiny_frequencies(ctx, fk, orc):
     assert not np.isfinite(ref["asxtemp"][0]) and np.isfinite(ref["asxtemp"][2])
     assert rel(res["achtemp"], ref["achtemp"]) <= TOL
     assert rel(res["asxtemp"][2:], ref["asxtemp"][2:]) <= TOL
+
+
+@pytest.mark.parametrize("bad", [complex(np.inf, 0.0), complex(0.0, -np.inf), complex(np.nan, 1.0)], ids=str)
+@pytest.mark.parametrize("band", [0, 2])
+@pytest.mark.parametrize("flags", [0, 8])
+def test_not_finite_over_a_zero_term(ctx, fk, orc, band, bad, flags):
+    """A value of an occupied band's aqsntemp that is not finite where wtilde is 0: at wx = 0.4
+    neither sch nor ssx is taken there, and 0 times the value is NaN as in the reference."""
+    p = fk.inputs.gpp_synthetic(12, 3, 600, 7, seed=3, wx="stress")
+    p["wtilde_array"][:, 77] = 0.0
+    p["aqsntemp"][band, 77] = bad
+    res, ref = ctx.gpp(p, "fp64", flags), orc.gpp(p, flags=flags)
+    for k in KEYS:
+        np.testing.assert_array_equal(np.isnan(res[k]), np.isnan(ref[k]), err_msg=k)
+        ok = np.isfinite(ref[k])
+        if ok.any():
+            assert rel(res[k][ok], ref[k][ok]) <= TOL, k
+    assert np.isnan(ref["asxtemp"]).all()
