@@ -244,6 +244,9 @@ FK_DEV void block_sum_ff(float2 (&v)[NV], double2* sm /* [8][NV] */, double2 (&o
     }
 }
 
+// |v| >= 2^60, an infinity or NaN: squares and products of two such no longer fit FP32
+FK_DEV bool large(double v) { return (((unsigned)__double2hiint(v) >> 20) & 0x7ffu) >= 1023u + 60u; }
+
 // Sums of N <= 16 values over a block of 256 threads, in a fixed order: in each
 // step a lane hands half of its values to its partner and adds the partner's
 // half of the others (8 + 4 + 2 + 1 + 1 additions instead of a five-level tree
@@ -335,7 +338,6 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) prep64_kernel(PrepArgs p) {
     const double2* erow = p.eps + (long)my_igp * p.nc;
     double2* D = reinterpret_cast<double2*>(p.D);
     const int ig_end = min(p.nc, (ch + 1) * p.tile);
-    auto large = [](double v) { return (((unsigned)__double2hiint(v) >> 20) & 0x7ffu) >= 1023u + 60u; };
     auto infinite = [](double v) { return ((unsigned)__double2hiint(v) & 0x7ff00000u) == 0x7ff00000u; };  // or NaN
     for (int ig = ch * p.tile + tid; ig < ig_end; ig += PREP_THREADS) {
         const double2 wt = wrow[ig], ep = erow[ig];
@@ -459,7 +461,8 @@ FK_DEV bool half_member(int ig, int igp) { return ig < igp - 1 && (ig & 511) != 
 // The first ig < igp with |wtilde^2 * I_eps| < to1 is found chunk by chunk (half_break: the
 // smallest hit of one chunk of the column, or a value above every igp).  The test runs in FP32
 // on |Omega2|^2 against to1^2; inside a relative guard band of 1e-5 around it (the FP32 error
-// is ~1e-7) the FP64 test decides, so every decision is the FP64 one.
+// is ~1e-7) and for values out of FP32's range the FP64 test decides, so every decision is
+// the FP64 one.
 constexpr int HALF_CHUNKS = 64;
 __device__ __noinline__ bool half_break64(double2 w, double2 ep) {
     const double2 o = cmul(cmul(w, w), ep);
@@ -474,7 +477,9 @@ FK_DEV void half_break(int nc, int igp, int chunk, const double2* wt, const doub
         const float2 w = c64_to_f32(w64), o = cmulf(cmulf(w, w), c64_to_f32(e64));
         const float o2 = o.x * o.x + o.y * o.y;
         bool hit = o2 < 1e-12f;
-        if (!(o2 < 1e30f) || fabsf(o2 - 1e-12f) <= 1e-12f * GUARD || !(o2 > 1e-36f)) hit = half_break64(w64, e64);
+        if (large(w64.x) || large(w64.y) || large(e64.x) || large(e64.y) || !(o2 < 1e30f) || !(o2 > 1e-36f) ||
+            fabsf(o2 - 1e-12f) <= 1e-12f * GUARD)
+            hit = half_break64(w64, e64);
         if (hit) first = min(first, ig);
     }
     __shared__ int sm[8];

@@ -54,3 +54,14 @@ def test_not_finite_over_a_zero_term(ctx, fk, orc, band, bad, flags):
         if ok.any():
             assert rel(res[k][ok], ref[k][ok]) <= TOL, k
     assert np.isnan(ref["asxtemp"]).all()
+
+
+@pytest.mark.parametrize("log2", [59, 61, 130, 260, 450])
+def test_half_sum_break_beyond_fp32(ctx, fk, orc, log2):
+    """Epsilon beyond FP32's range in one column: the half sum's search for the first
+    |Omega2| < 1e-6 of a column must not stop there."""
+    p = fk.inputs.gpp_synthetic(40, 3, 700, 9, seed=4, dist="branch", wx="stress")
+    p["I_eps_array"][3] *= 2.0 ** log2
+    res, ref = ctx.gpp(p, "fp64", fk.FK_GPP_HALF_SUM), orc.gpp(p, flags=orc.ORC_GPP_HALF_SUM)
+    for k in KEYS:
+        assert rel(res[k], ref[k]) <= TOL, k

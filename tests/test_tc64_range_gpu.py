@@ -130,7 +130,7 @@ def test_ff_planes_out_of_range_go_to_dmma(ctx, fk, orc, which, planes):
     check(ctx.ff(p, "fp64", 5), want, FFKEYS)
 
 
-@pytest.mark.parametrize("flags", [0, 2])
+@pytest.mark.parametrize("flags", [0, 2, 4])
 def test_d_rows_out_of_range_go_to_dmma(ctx, fk, orc, flags):
     p = fk.inputs.gpp_synthetic(70, 2, 700, 9, seed=4, dist="branch", wx="stress")
     p["I_eps_array"][3] *= 2.0 ** 450
