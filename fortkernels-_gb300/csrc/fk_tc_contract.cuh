@@ -40,6 +40,7 @@
 #include <cuda_fp16.h>
 
 #include "fk_gemm.cuh"
+#include "fk_groups.h"
 #include "fk_tc.cuh"
 
 namespace fk {
@@ -390,9 +391,7 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
     };
     // the stage behind the group that starts at stage sg0
     auto group_end = [&](const TcArgs& t, int sg0, int nst, int CH) {
-        int e = min(nst, sg0 + C::GRP * CH);
-        if (C::SL && !PAIR && t.group_stages) e = min(e, (sg0 / t.group_stages + 1) * t.group_stages);
-        return e;
+        return fk::group_end(sg0, nst, C::GRP * CH, C::SL && !PAIR ? t.group_stages : 0);
     };
     auto fail = [&](int code) {
         atomicOr(err, code);
@@ -459,7 +458,7 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
                     for (int st0 = sg0, b = slot * C::GRP; st0 < sg1 && ok; st0 += CH, ++b) {
                         // X, Y (two accumulators) or, SL, the one accumulator D = dX
                         const uint32_t dX = tmem + (uint32_t)(b * C::ACC_COLS), dY = dX + 2 * BN;
-                        const int st1 = min(nst, st0 + CH);
+                        const int st1 = chunk_end(st0, CH, sg1);
                         for (int st = st0; st < st1; ++st, ++g) {
                             const int s = g % C::STAGES;
                             const uint32_t par = (g / C::STAGES) & 1;
@@ -756,7 +755,7 @@ __device__ __forceinline__ void tc_contract_body(Src src0, int* err, const long 
             // weighted sums: half the arithmetic, waits and returns per chunk)
             for (int st0 = 0; st0 < nst; ++grp) {
                 // chunks in the group
-                const int npass = PAIR ? min(C::GRP, (nst - st0 + CH - 1) / CH) : (group_end(t, st0, nst, CH) - st0 + CH - 1) / CH;
+                const int npass = PAIR ? min(C::GRP, (nst - st0 + CH - 1) / CH) : group_chunks(st0, group_end(t, st0, nst, CH), CH);
                 const int slot = grp % C::NSLOT;
                 const int b = slot * C::GRP, b2 = b + 1;
                 if (!tc::warp_all(tc::mbar_wait(&accFull[slot], (grp / C::NSLOT) & 1, wait_limit) && !s_abort)) {
