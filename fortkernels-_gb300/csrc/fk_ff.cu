@@ -671,12 +671,13 @@ fk_status ff_run(Ctx& c, const FfDev& r, const FfHost& h, const FfPipe* pipe) {
         cudaMemsetAsync(c.errword, 0, sizeof(int), st);
     }
     if (p.tc64) {
-        cudaMemsetAsync(c.errword, 0, sizeof(int), st);
+        e = cudaMemsetAsync(c.errword, 0, sizeof(int), st);
         ContractArgs a{};
         a.A = r.aqsn; a.lda = r.nc; a.M = r.nb; a.K = r.nc; a.rowmap = order;
         a.aqsm = r.aqsm; a.ldm = r.nc; a.vcoul = r.vcoul; a.igp = igp; a.acol = igp; a.wscale = 1.0;
         tc64::enqueue_weights(c, a, r.ng, zb, true);
-        tc64::enqueue_a(c, a, p.z, zb);
+        if (e == cudaSuccess) e = tc64::enqueue_a(c, a, p.z, zb);
+        if (e != cudaSuccess) return cuda_fail(c, e, "ff: digits");
     }
     // a0 < 0: R planes, all bands on CTA pairs; a0 >= 0: the A planes a0 .. a0+nb_-1
     // of planesA, each over the row tiles of the bands that read it

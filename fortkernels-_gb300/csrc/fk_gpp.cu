@@ -30,6 +30,7 @@
 #include <memory>
 #include <new>
 
+#include "fk_branch.h"
 #include "fk_gemm.cuh"
 #include "fk_internal.h"
 #include "fk_tc64.cuh"
@@ -1663,35 +1664,31 @@ bool take_tc64(Ctx& c, const Plan& p, tc64::Bufs& b) {
     return b.A && b.B && b.ea && b.eb && b.W1 && b.guard;
 }
 template <int EPI>
-void run_tc64(Ctx& c, const ContractArgs& a, const tc64::Plan& z, const tc64::Bufs& b, bool have_a = false,
-              bool re_only = false) {
+cudaError_t run_tc64(Ctx& c, const ContractArgs& a, const tc64::Plan& z, const tc64::Bufs& b, bool have_a = false,
+                     bool re_only = false) {
     tc64::enqueue_weights(c, a, EPI == EPI_GPP ? a.N / 3 : a.N, b, false);
-    if (!have_a) tc64::enqueue_a(c, a, z, b);
-    tc64::enqueue<EPI>(c, a, z, b, tc64::one_plane(z), 0, re_only);
+    const cudaError_t e = have_a ? cudaSuccess : tc64::enqueue_a(c, a, z, b);
+    if (e == cudaSuccess) tc64::enqueue<EPI>(c, a, z, b, tc64::one_plane(z), 0, re_only);
+    return e;
 }
 
-// A side branch of the context's stream: work queued between fork and join on
-// `side` runs beside the stream's own; join makes the stream wait for it.
-struct Branch {
-    Ctx& c;
-    cudaStream_t main, side = nullptr;
-    explicit Branch(Ctx& c_) : c(c_), main(c_.stream) {
-        if (side_ready(c) != FK_OK) return;  // no side stream (none yet, and the caller captures): the work stays in line
-        if (cudaEventRecord(c.pipe_ev[0], main) == cudaSuccess && cudaStreamWaitEvent(c.copy_stream, c.pipe_ev[0], 0) == cudaSuccess)
-            side = c.copy_stream;
-        else cudaGetLastError();
+struct CudaApi {
+    using Stream = cudaStream_t;
+    using Event = cudaEvent_t;
+    using Error = cudaError_t;
+    Error record(Event e, Stream s) { return cudaEventRecord(e, s); }
+    Error wait(Stream s, Event e) { return cudaStreamWaitEvent(s, e, 0); }
+    Error synchronize(Stream s) { return cudaStreamSynchronize(s); }
+    bool capturing(Stream s) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        return cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
     }
-    // queues f's launches (which go to c.stream) on the side stream
-    template <class F>
-    void run(F f) {
-        if (side) c.stream = side;
-        f();
-        c.stream = main;
-        if (side && cudaEventRecord(c.pipe_ev[1], side) != cudaSuccess) cudaStreamSynchronize(side);
-    }
-    void join() {
-        if (side) cudaStreamWaitEvent(main, c.pipe_ev[1], 0);
-    }
+    void clear() { cudaGetLastError(); }
+};
+// (no side stream: none yet, and the caller captures)
+struct SideBranch : Branch<CudaApi> {
+    explicit SideBranch(Ctx& c)
+        : Branch(CudaApi{}, c.stream, side_ready(c) == FK_OK ? c.copy_stream : nullptr, c.pipe_ev[0], c.pipe_ev[1]) {}
 };
 
 template <class K>
@@ -2118,7 +2115,8 @@ fk_status gpp_run_half(Ctx& c, const GppDev& r) {
             k<<<std::min(p.units, c.sms), tcx::THREADS, tcx::Cfg<64>::SMEM, st>>>(t);
             kernel_end(c);
         } else if (p.tc64) {
-            run_tc64<EPI_GPP>(c, a, p.z, zb);
+            const cudaError_t e = run_tc64<EPI_GPP>(c, a, p.z, zb);
+            if (e != cudaSuccess) return cuda_fail(c, e, "gpp: digits");
             continue;
         } else {
             auto k = d64::contract_kernel<EPI_GPP>;
@@ -2275,19 +2273,21 @@ fk_status gpp_run(Ctx& c, const GppDev& r, const GppPipe* pipe) {
     // 512 x 32768 x 20: the prep takes 103 us at one block per SM instead of 98 at two, the
     // digits hide behind it, the call goes from 435 to 406 us.
     if (p.tc64) {
-        Branch br(c);
+        SideBranch br(c);
+        cudaError_t ea = cudaSuccess;
         ContractArgs a{};
         a.A = r.aqsn; a.lda = r.nc; a.m0 = p.m0; a.M = M; a.K = r.nc;
         for (int pass = 0; pass < p.passes; ++pass) launch_prep(prep_args(pass), dim3(p.nch, r.ng));
-        br.run([&] { tc64::enqueue_a(c, a, p.z, zb); });
-        br.join();
+        br.run([&] { ea = tc64::enqueue_a(c, a, p.z, zb); });
+        const cudaError_t ej = br.join();
+        if (ea != cudaSuccess || ej != cudaSuccess) return cuda_fail(c, ea != cudaSuccess ? ea : ej, "gpp: digits");
     }
     for (int pass = 0; pass < p.passes && !pipe && !p.tc64; ++pass) launch_prep(prep_args(pass), dim3(p.nch, r.ng));
     phase_mark(c, 2);
     // mixed: the static remainder beside the main contraction (both need the prep's set-up
     // only): 130 x 4099 x 70 98 -> 95 us
-    std::unique_ptr<Branch> stat;
-    if (S && p.mixed && M > 0 && !pipe && !c.profiling) stat.reset(new (std::nothrow) Branch(c));
+    std::unique_ptr<SideBranch> stat;
+    if (S && p.mixed && M > 0 && !pipe && !c.profiling) stat.reset(new (std::nothrow) SideBranch(c));
     if (M > 0 && !pipe) {
         ContractArgs a{};
         a.A = r.aqsn; a.lda = r.nc; a.m0 = p.m0; a.M = M;
@@ -2337,7 +2337,7 @@ fk_status gpp_run(Ctx& c, const GppDev& r, const GppPipe* pipe) {
                 kernel_end(c);
             }
         } else if (p.tc64) {
-            run_tc64<EPI_GPP>(c, a, p.z, zb, true);
+            run_tc64<EPI_GPP>(c, a, p.z, zb, true);  // (the digits were queued above)
             --c.launches;
         } else {
             auto k = d64::contract_kernel<EPI_GPP>;
@@ -2361,7 +2361,8 @@ fk_status gpp_run(Ctx& c, const GppDev& r, const GppPipe* pipe) {
             auto launch = [&] { k<<<grid, f32::THREADS, f32::SMEM, c.stream>>>(a); };
             if (stat) {
                 stat->run(launch);
-                stat->join();
+                const cudaError_t ej = stat->join();
+                if (ej != cudaSuccess) return cuda_fail(c, ej, "gpp: static remainder");
             } else {
                 launch();
             }
@@ -2370,9 +2371,10 @@ fk_status gpp_run(Ctx& c, const GppDev& r, const GppPipe* pipe) {
             const bool prof = c.profiling;
             const int nk = c.nk;
             c.profiling = false;
-            run_tc64<EPI_STAT>(c, a, p.zs, zb);
+            const cudaError_t e = run_tc64<EPI_STAT>(c, a, p.zs, zb);
             c.profiling = prof;
             c.nk = nk;
+            if (e != cudaSuccess) return cuda_fail(c, e, "gpp: digits");
             --c.launches;
         } else {
             auto k = d64::contract_kernel<EPI_STAT>;
@@ -2916,7 +2918,8 @@ fk_status gpp_real_run(Ctx& c, const GppRealDev& r) {
             k<<<std::min(p.units, c.sms), tcx::THREADS, tcx::Cfg<64>::SMEM, st>>>(t);
             kernel_end(c);
         } else if (p.tc64) {
-            run_tc64<EPI_GPP>(c, a, p.z, zb, false, true);
+            const cudaError_t e = run_tc64<EPI_GPP>(c, a, p.z, zb, false, true);
+            if (e != cudaSuccess) return cuda_fail(c, e, "gpp_real: digits");
             --c.launches;
         } else {
             auto k = d64::contract_kernel<EPI_GPP>;

@@ -820,11 +820,13 @@ inline void launch_split(Ctx& c, const SplitArgs& s, int batches) {
 }
 
 // The digits of a.A's rows m0 .. m0+M-1 (or rowmap[0 .. M)) and the flag's reset.
-inline void enqueue_a(Ctx& c, const ContractArgs& a, const Plan& p, const Bufs& b) {
-    cudaMemsetAsync(b.flag(), 0, sizeof(int), c.stream);
+inline cudaError_t enqueue_a(Ctx& c, const ContractArgs& a, const Plan& p, const Bufs& b) {
+    const cudaError_t e = cudaMemsetAsync(b.flag(), 0, sizeof(int), c.stream);
+    if (e != cudaSuccess) return e;
     SplitArgs s{a.rowmap ? a.A : a.A + (long)a.m0 * a.lda, nullptr, 1, a.lda, 0, nullptr, a.rowmap, a.M, a.K, p.KS, p.kst_unit,
                 p.kstages, 2 * p.MT, b.A, b.ea, b.flag(), c.errword, c.wait_limit};
     launch_split<false>(c, s, 1);
+    return cudaSuccess;  // (launch errors: the caller's check behind its last launch)
 }
 
 // The digits of a.batches planes (at most MAXPL) of a.B, the contraction over the row tiles of `tab` and the
