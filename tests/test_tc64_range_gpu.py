@@ -179,3 +179,16 @@ def test_wait_timeout_is_reported(ctx, fk, orc, path):
         ctx.set_wait_limit(-1)
     ctx.synchronize()
     check(call(), ref, keys)
+
+
+def test_half_sum_weights_out_of_range(ctx, fk, orc):
+    """A band of aqsmtemp beyond 2^400: the half sum's second contraction (rows of aqsmtemp)
+    goes to DMMA, the other bands keep their values."""
+    p = fk.inputs.gpp_synthetic(70, 2, 700, 9, seed=6, dist="branch", wx="stress")
+    want = orc.gpp(p, flags=orc.ORC_GPP_HALF_SUM)["acht_n1_loc"]
+    q = dict(p, aqsmtemp=p["aqsmtemp"].copy())
+    q["aqsmtemp"][10] *= 2.0 ** 450
+    got, ref = ctx.gpp(q, "fp64", fk.FK_GPP_HALF_SUM)["acht_n1_loc"], orc.gpp(q, flags=orc.ORC_GPP_HALF_SUM)["acht_n1_loc"]
+    keep = np.arange(70) != 10
+    assert rel(got[keep], want[keep]) <= TOL
+    assert rel(got[10:11], ref[10:11]) <= TOL
