@@ -278,10 +278,10 @@ fk_status fk_wait_error_status(int word, char* msg, size_t msg_len) {
                  {0x8, "copy warp waiting for a free operand stage"},
                  {0x10, "epilogue waiting for an accumulator"},
                  {0x20, "converter warps waiting for operand rows"},
-                 {0x40, "copy warp waiting for a free staging half"},
+                 {0x40, "copy warp waiting for a free staging quarter"},
                  {0x80, "copy warp waiting for its last copies"},
                  {0x100, "self-test wait"},
-                 {0x200, "plane conversion waiting for its row copy"},
+                 {0x200, "plane conversion or digit split waiting for its row copy"},
                  {0x400, "-B_im warp waiting for an operand stage"}};
     std::string m;
     if (word == 0) {
@@ -974,8 +974,8 @@ fk_status fk_ff(fk_ctx_t c, int nb, int nv, int nc, int ng, int nf, int ne, cons
     fk::phase_mark(x, 0);
     fk::FfPipe pipe{};
     // small inputs (and the planner's tables) through the pinned buffer: one copy
-    // each, and the call does not wait for the stream; it holds the previous call's
-    // until their copies are done
+    // each.  It holds the previous call's until their copies are done, and those lie on
+    // the stream behind the call before: the host queues one call ahead at most
     uint8_t* small_d = packed ? (uint8_t*)x.ws.take(packed) : nullptr;
     uint8_t* pb = (uint8_t*)fk::pinned_buffer(x, packed + fk::ff_table_bytes(r));
     if (!out || (packed && !small_d)) return fk::fail(x, FK_ENOMEM, "workspace: staging");

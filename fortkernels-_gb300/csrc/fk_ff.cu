@@ -598,8 +598,8 @@ fk_status ff_run(Ctx& c, const FfDev& r, const FfHost& h, const FfPipe* pipe) {
         (p.bytesImgA && !imgA) || (p.bytesW && !W) || (p.bytesAimg && !Aimg) || (p.bytesScale && !scales))
         return fail(c, FK_ENOMEM, "workspace too small for FF request");
     double2 *RW = tabs, *RS = tabs + (size_t)r.nb * r.nf, *AW = tabs + 2 * (size_t)r.nb * r.nf;
-    // the tables -> device, through pinned memory: the call neither waits for the
-    // stream nor issues a copy per table
+    // the tables -> device, through pinned memory: one copy, not one per table, and no
+    // wait for it here (the next call's use of the pinned buffer waits, fk_abi.cu)
     std::memcpy(h.tab, p.fact.data(), r.nb * sizeof(FactRow));
     if (order) std::memcpy(h.tab + ft.order, p.order.data(), r.nb * sizeof(int));
     std::memcpy(h.tab + ft.planes, p.planesR.data(), nR * sizeof(int));

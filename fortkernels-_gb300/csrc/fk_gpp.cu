@@ -15,11 +15,13 @@
 //      epilogue applies 0.5*vcoul[igp]*conj(aqsmtemp[n1][igp]) and reduces
 //      each row to its three iw sums (fk_gemm.cuh);
 //   3. add all partials in a fixed order (finalize kernels).
-// FP64 path: every branch quantity follows the reference's expression
-// sequence with round-to-nearest FP64 operations (no contraction), so each
-// branch is taken exactly as in the reference's C++; the contraction runs on
-// the tensor cores by exact digit products (fk_tc64.cuh), or on FP64 DMMA where
-// there is no room for their images.  Mixed path: the branch quantities are evaluated in FP32 from an
+// FP64 path: each branch is taken exactly as in the reference's C++: an element near
+// a threshold follows the reference's expression sequence with round-to-nearest FP64
+// operations (no contraction), as every element of the half and real-valued sums does;
+// clear of the thresholds the full sum's prep decides in FP32 and forms its values with
+// FMAs and a reciprocal refined to FP64 (prep64_kernel).  The contraction runs on
+// the tensor cores by digit products (fk_tc64.cuh), or on FP64 DMMA where
+// there is no room for their images or the digits are too coarse.  Mixed path: the branch quantities are evaluated in FP32 from an
 // FP64 wdiff and re-evaluated with the exact FP64 sequence whenever a test
 // value lies within a relative guard band of its threshold, so branch
 // decisions remain those of the FP64 sequence; the bulk products run in FP32
@@ -2271,7 +2273,7 @@ fk_status gpp_run(Ctx& c, const GppDev& r, const GppPipe* pipe) {
     }
     // FP64: aqsntemp's digits (bound by memory) beside the prep (by the FP64 pipe).
     // 512 x 32768 x 20: the prep takes 103 us at one block per SM instead of 98 at two, the
-    // digits hide behind it, the call goes from 435 to 406 us.
+    // digits hide behind it, the call goes from 435 to 409 us.
     if (p.tc64) {
         SideBranch br(c);
         cudaError_t ea = cudaSuccess;

@@ -191,8 +191,9 @@ fk_status fk_gpp_real(fk_ctx_t ctx, int number_bands, int nvband, int ncouls, in
 #define FK_GPP_STATIC_SCRATCH_BYTES (64u << 20)
 
 /*
- * fk_gpp_static: the FP64 GPP sum of fk_gpp (same arguments and results as
- * fk_gpp with precision FK_FP64) for callers that must not allocate device
+ * fk_gpp_static: the FP64 GPP sum of fk_gpp (same arguments as fk_gpp with
+ * precision FK_FP64, same results to FP64 rounding: it always contracts on
+ * DMMA) for callers that must not allocate device
  * memory: a process whose GPU memory is already owned by another allocator
  * (a framework's caching pool that has reserved the device), or a loop that
  * cannot take the device-wide synchronisation of cudaMalloc/cudaFree.  No
